@@ -315,7 +315,8 @@ LB_API int lb_deltanet_step(lb_ctx* c, uint64_t state, uint64_t q, uint64_t k, u
     p.z = (const float*)z; p.g = (const float*)g; p.beta = (const float*)beta; p.out = (float*)out;
     p.HV = HV; p.HK = HK;
     void* params[] = {&p, &n_steps};
-    return lb_launch(c, in_is_f32 ? LBK_deltanet_step_f32 : LBK_deltanet_step_bf16, (unsigned)HV, 4, 1, 128, 0, params, 1);
+    const int kernel = n_steps == 1 ? (in_is_f32 ? LBK_deltanet_one_f32 : LBK_deltanet_one_bf16) : in_is_f32 ? LBK_deltanet_step_f32 : LBK_deltanet_step_bf16;
+    return lb_launch(c, kernel, (unsigned)HV, 4, 1, 128, 0, params, 1);
 }
 
 LB_API int lb_decay_gate(lb_ctx* c, uint64_t a, uint64_t a_log, uint64_t dt_bias, uint64_t b, uint64_t g_out,
