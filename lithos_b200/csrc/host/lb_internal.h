@@ -45,6 +45,7 @@
     X(LaunchKernel, cuLaunchKernel,                                                                             \
       (CUfunction, unsigned, unsigned, unsigned, unsigned, unsigned, unsigned, unsigned, CUstream, void**, void**)) \
     X(LaunchKernelEx, cuLaunchKernelEx, (const CUlaunchConfig*, CUfunction, void**, void**))                    \
+    X(OccupancyMaxActiveClusters, cuOccupancyMaxActiveClusters, (int*, CUfunction, const CUlaunchConfig*))      \
     X(StreamCreate, cuStreamCreate, (CUstream*, unsigned int))                                                  \
     X(StreamDestroy, cuStreamDestroy, (CUstream))                                                               \
     X(StreamSynchronize, cuStreamSynchronize, (CUstream))                                                       \
@@ -90,9 +91,8 @@ int lb_driver_load(char* err, size_t errlen); /* LB_OK or LB_ERR_NO_DRIVER */
     X(gemm_int4_mma_b32)              \
     X(gemm_int4_mma_b64)              \
     X(gemm_int4_tc)                   \
-    X(gemm_int4_tc_g1)                \
-    X(gemm_int4_tc_ta)                \
-    X(gemm_int4_tc_ta_g1)             \
+    X(gemm_int4_tc_256)               \
+    X(gemm_int4_tc_exact)             \
     X(gptq_dequant_f32)               \
     X(gptq_unpack_u8)                 \
     X(dense_bf16_gemv)                \
@@ -223,6 +223,7 @@ struct lb_ctx {
     /* strip-packed copies made by lb_gemv_pack and still alive: lb_gemv_int4 runs the strip-packed kernel for these matrices */
     struct { uint64_t qweight, packed; int K, N, swiglu; } packed_reg[LB_PACKED_REG_MAX];
     int n_packed_reg;
+    int tc_clusters[9];     /* [k]: clusters of k CTAs of one per SM that run at once (0: not asked yet) */
     int chain_mailbox;      /* hand vectors from a GEMV to the next one through the mailbox (1, default) or a grid barrier (0) */
     int capturing;     /* stream capture in progress */
     uint64_t capture_launches0;

@@ -205,11 +205,33 @@ LB_API int lb_gemv_int4_host(lb_ctx* c, const uint32_t* qweight, const uint16_t*
 }
 
 /* ---- batched int4 projection ---------------------------------------------------------
- * 33..64 tokens (9..64 with LB_GEMM_TCGEN05): gemm_int4_tc (tcgen05, one CTA per SM: 128 columns x a K slice);
- * otherwise, or with LB_GEMM_MMA_SYNC, the mma.sync kernels (two CTAs per SM): the faster one at each size
- * as measured (bench.py --workload batched).  The K slices of a column block are the CTAs
+ * 33..256 tokens (from 9 with LB_GEMM_TCGEN05): gemm_int4_tc (tcgen05, one CTA per SM: 128 columns x a K slice); up to 32 tokens
+ * gemm_int4_tc_exact or, as always with LB_GEMM_MMA_SYNC, the mma.sync kernels (two CTAs per SM).  The K slices of a column block are the CTAs
  * of one cluster (<= 8); the slice count fills the SMs without starting a second wave and leaves
  * every slice at least four K-groups. */
+
+/* clusters of k CTAs of the tcgen05 kernels (one CTA per SM) that run at once: the SMs of a GPC do not all divide by k, and one
+ * cluster too many doubles the time (4096 -> 2048 at 48 tokens: 14.2 us as 16 clusters of 8, 8.0 as clusters of what fits) */
+static int tc_clusters(lb_ctx* c, int k) {
+    if (k <= 1) return c->sm_count;
+    if (!c->tc_clusters[k]) {
+        CUlaunchConfig cfg;
+        memset(&cfg, 0, sizeof cfg);
+        CUlaunchAttribute attr;
+        memset(&attr, 0, sizeof attr);
+        attr.id = CU_LAUNCH_ATTRIBUTE_CLUSTER_DIMENSION;
+        attr.value.clusterDim.x = 1; attr.value.clusterDim.y = (unsigned)k; attr.value.clusterDim.z = 1;
+        cfg.gridDimX = (unsigned)c->sm_count; cfg.gridDimY = (unsigned)k; cfg.gridDimZ = 1;
+        cfg.blockDimX = LB_TC_THREADS; cfg.blockDimY = cfg.blockDimZ = 1;
+        cfg.sharedMemBytes = LB_TC_X_HALVES * 256 * 128;
+        cfg.attrs = &attr; cfg.numAttrs = 1;
+        int n = 0;
+        if (!c->fn[LBK_gemm_int4_tc_256] || lb_drv.OccupancyMaxActiveClusters(&n, c->fn[LBK_gemm_int4_tc_256], &cfg) != CUDA_SUCCESS || n < 1) n = c->sm_count / k;
+        c->tc_clusters[k] = n;
+    }
+    return c->tc_clusters[k];
+}
+
 LB_API int lb_gemm_int4(lb_ctx* c, uint64_t qweight, uint64_t scales, uint64_t qzeros, uint64_t x, uint64_t y, int K, int N,
                         int B, int flags) {
     if (!c || !qweight || !scales || !x || !y || K <= 0 || N <= 0 || K % 128 || N % 16 || B < 1 || B > LB_GEMM_MAX_BATCH ||
@@ -229,12 +251,14 @@ LB_API int lb_gemm_int4(lb_ctx* c, uint64_t qweight, uint64_t scales, uint64_t q
         if (lb_gemv_int4(c, qweight, scales, qzeros, x, y, K, N, flags & LB_GEMV_Y_F32) == LB_OK) return LB_OK; /* else: the batched kernel */
     const int blocks = (N + 127) / 128, groups = K / 128;
     void* params[] = {&p};
-    if ((B > 32 && !(flags & LB_GEMM_MMA_SYNC)) || (flags & LB_GEMM_TCGEN05)) {
+    /* up to 32 tokens no weight is rounded: gemm_int4_tc_exact or the mma.sync kernels, the faster one.  us, mma.sync / tcgen05, at 12 tokens: 17408 -> 5120
+     * 34.4 / 31.0, 6144 -> 5120 17.8 / 13.0, 1024 -> 1024 6.8 / 6.3 (matrices that are split along K), 5120 -> 17408 23.9 / 24.5, 5120 -> 34816 39.1 / 49.0
+     * (whole columns: two CTAs per SM against one); at 32 tokens 47.7 / 32.8, 24.5 / 13.9, 11.3 / 6.9, 34.7 / 28.6, 54.7 / 57.8; at 8 tokens 28.8 / 27.8,
+     * 14.4 / 13.0, 5.6 / 5.4, 20.0 / 24.4, 32.6 / 48.6 */
+    const int exact = B > 8 && B <= 32 && !(flags & (LB_GEMM_MMA_SYNC | LB_GEMM_TCGEN05)) && (B > 16 ? blocks : 2 * blocks) <= c->sm_count;
+    if (exact || (B > 32 && !(flags & LB_GEMM_MMA_SYNC)) || (flags & LB_GEMM_TCGEN05)) {
         const int nt = B > 128 ? 256 : B > 64 ? 128 : B > 32 ? 64 : B > 16 ? 32 : 16;
-        const int ta = nt > 128 || getenv("LB_GEMM_SMEM_A") == NULL; /* weights through tensor memory (default), or the shared-memory operand tiles for comparison (up to 128 tokens) */
-        unsigned smem = ta ? (unsigned)((nt > 128 ? 3 : nt > 64 ? 6 : nt > 32 ? 12 : 16) * nt * 256) /* 3..16 activation stages */
-                           : (unsigned)(4 * 32768 + (nt > 64 ? 3 : nt > 32 ? 5 : nt > 16 ? 10 : 16) * nt * 256); /* four weight stages + 3..16 activation stages */
-        if (smem < (unsigned)nt * 132u * 4u) smem = (unsigned)nt * 132u * 4u; /* the epilogue's partial tile [nt][132] fp32 lies over the stages */
+        const unsigned smem = nt > 128 ? (unsigned)(LB_TC_X_HALVES * nt * 128) : (unsigned)((nt > 64 ? 6 : 7) * nt * 256); /* activation stages; the partial tile [nt][132] fp32 fits over them */
         if (x & 15) return lb_fail(c, LB_ERR_INVALID, "lb_gemm_int4: x must be 16-byte aligned");
         CUtensorMap tm; /* X [B, K] fp16, box = 64 k (128 bytes) x NT tokens, laid down with the 128-byte swizzle */
         cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)B};
@@ -247,9 +271,10 @@ LB_API int lb_gemm_int4(lb_ctx* c, uint64_t qweight, uint64_t scales, uint64_t q
         memcpy(p.tmap_x, &tm, sizeof tm);
         int ksplit = c->sm_count / blocks;
         if (ksplit > 8) ksplit = 8;
-        while (ksplit > 1 && groups / ksplit < 4) ksplit--;
+        while (ksplit > 1 && (groups / ksplit < 4 || tc_clusters(c, ksplit) < blocks)) ksplit--;
         if (ksplit < 1) ksplit = 1;
-        return lb_launch_cluster(c, ta ? (nt > 128 ? LBK_gemm_int4_tc_ta_g1 : LBK_gemm_int4_tc_ta) : nt > 64 ? LBK_gemm_int4_tc_g1 : LBK_gemm_int4_tc, (unsigned)blocks, (unsigned)ksplit, 1, 576, smem, params, 1, (unsigned)ksplit);
+        return lb_launch_cluster(c, exact ? LBK_gemm_int4_tc_exact : nt > 128 ? LBK_gemm_int4_tc_256 : LBK_gemm_int4_tc, (unsigned)blocks, (unsigned)ksplit, 1,
+                                 exact ? LB_TC_EXACT_THREADS : LB_TC_THREADS, smem, params, 1, (unsigned)ksplit);
     }
     const int rows = B > 32 ? 64 : B > 16 ? 32 : B > 8 ? 16 : 8; /* token rows the CTA stages */
     const int kernel = B > 32 ? LBK_gemm_int4_mma_b64 : B > 16 ? LBK_gemm_int4_mma_b32 : B > 8 ? LBK_gemm_int4_mma_b16 : LBK_gemm_int4_mma_b8;
