@@ -206,7 +206,7 @@ LB_API int lb_gemv_int4_host(lb_ctx* c, const uint32_t* qweight, const uint16_t*
 
 /* ---- batched int4 projection ---------------------------------------------------------
  * 33..256 tokens (from 9 with LB_GEMM_TCGEN05): gemm_int4_tc (tcgen05, one CTA per SM: 128 columns x a K slice); up to 32 tokens
- * gemm_int4_tc_exact or, as always with LB_GEMM_MMA_SYNC, the mma.sync kernels (two CTAs per SM).  The K slices of a column block are the CTAs
+ * gemm_int4_tc_exact16 / 32 or, as always with LB_GEMM_MMA_SYNC, the mma.sync kernels (two CTAs per SM).  The K slices of a column block are the CTAs
  * of one cluster (<= 8); the slice count fills the SMs without starting a second wave and leaves
  * every slice at least four K-groups. */
 
@@ -251,10 +251,10 @@ LB_API int lb_gemm_int4(lb_ctx* c, uint64_t qweight, uint64_t scales, uint64_t q
         if (lb_gemv_int4(c, qweight, scales, qzeros, x, y, K, N, flags & LB_GEMV_Y_F32) == LB_OK) return LB_OK; /* else: the batched kernel */
     const int blocks = (N + 127) / 128, groups = K / 128;
     void* params[] = {&p};
-    /* up to 32 tokens no weight is rounded: gemm_int4_tc_exact or the mma.sync kernels, the faster one.  us, mma.sync / tcgen05, at 12 tokens: 17408 -> 5120
-     * 34.4 / 31.0, 6144 -> 5120 17.8 / 13.0, 1024 -> 1024 6.8 / 6.3 (matrices that are split along K), 5120 -> 17408 23.9 / 24.5, 5120 -> 34816 39.1 / 49.0
-     * (whole columns: two CTAs per SM against one); at 32 tokens 47.7 / 32.8, 24.5 / 13.9, 11.3 / 6.9, 34.7 / 28.6, 54.7 / 57.8; at 8 tokens 28.8 / 27.8,
-     * 14.4 / 13.0, 5.6 / 5.4, 20.0 / 24.4, 32.6 / 48.6 */
+    /* up to 32 tokens no weight is rounded: gemm_int4_tc_exact16 / 32 or the mma.sync kernels, the faster one.  us, mma.sync / tcgen05, at 12 tokens:
+     * 17408 -> 5120 34.4 / 27.1, 6144 -> 5120 17.8 / 12.6, 1024 -> 1024 6.9 / 5.3 (matrices that are split along K), 5120 -> 17408 23.9 / 24.5,
+     * 5120 -> 34816 39.1 / 49.0 (whole columns: two CTAs per SM against one); at 32 tokens 46.9 / 31.3, 24.5 / 14.5, 11.3 / 6.3, 34.6 / 28.2, 54.7 / 57;
+     * at 8 tokens 28.8 / 27.8, 14.4 / 13.0, 5.6 / 5.4, 20.0 / 24.4, 32.6 / 48.6 */
     const int exact = B > 8 && B <= 32 && !(flags & (LB_GEMM_MMA_SYNC | LB_GEMM_TCGEN05)) && (B > 16 ? blocks : 2 * blocks) <= c->sm_count;
     if (exact || (B > 32 && !(flags & LB_GEMM_MMA_SYNC)) || (flags & LB_GEMM_TCGEN05)) {
         const int nt = B > 128 ? 256 : B > 64 ? 128 : B > 32 ? 64 : B > 16 ? 32 : 16;
@@ -273,8 +273,8 @@ LB_API int lb_gemm_int4(lb_ctx* c, uint64_t qweight, uint64_t scales, uint64_t q
         if (ksplit > 8) ksplit = 8;
         while (ksplit > 1 && (groups / ksplit < 4 || tc_clusters(c, ksplit) < blocks)) ksplit--;
         if (ksplit < 1) ksplit = 1;
-        return lb_launch_cluster(c, exact ? LBK_gemm_int4_tc_exact : nt > 128 ? LBK_gemm_int4_tc_256 : LBK_gemm_int4_tc, (unsigned)blocks, (unsigned)ksplit, 1,
-                                 exact ? LB_TC_EXACT_THREADS : LB_TC_THREADS, smem, params, 1, (unsigned)ksplit);
+        return lb_launch_cluster(c, exact ? (nt > 16 ? LBK_gemm_int4_tc_exact32 : LBK_gemm_int4_tc_exact16) : nt > 128 ? LBK_gemm_int4_tc_256 : LBK_gemm_int4_tc, (unsigned)blocks, (unsigned)ksplit, 1,
+                                 exact ? (nt > 16 ? LB_TC_EXACT32_THREADS : LB_TC_EXACT16_THREADS) : LB_TC_THREADS, smem, params, 1, (unsigned)ksplit);
     }
     const int rows = B > 32 ? 64 : B > 16 ? 32 : B > 8 ? 16 : 8; /* token rows the CTA stages */
     const int kernel = B > 32 ? LBK_gemm_int4_mma_b64 : B > 16 ? LBK_gemm_int4_mma_b32 : B > 8 ? LBK_gemm_int4_mma_b16 : LBK_gemm_int4_mma_b8;

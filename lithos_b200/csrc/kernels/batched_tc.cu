@@ -54,13 +54,13 @@ __device__ __forceinline__ uint32_t tc_h2_bits(__half2 h) { return *reinterpret_
 __device__ __forceinline__ __half2 tc_bits_h2(uint32_t u) { return *reinterpret_cast<__half2*>(&u); }
 // byte I of a packed word (q0 | q1 << 4) as the fp16 pair ((q0 - z) s, (q1 - z) s), EXACT: (q0 - z, q1 - z): (1024 + q0, 1024 + 16 q1) by
 // mask-and-or, (q0 - z, q1 - z) by one fma with (1, 1/16) and (-(1024 + z), -(64 + z)), both exact, then the scale
-template <bool EXACT, int I>
+template <int EXACT, int I>
 __device__ __forceinline__ uint32_t tc_pair(uint32_t w, __half2 mul, __half2 add, __half2 s) {
     const uint32_t v = __byte_perm(w, 0u, 0x4040u | I | (I << 8));
     const __half2 q = __hfma2(tc_bits_h2(tc_lop3_and_or(v, 0x00f0000fu, 0x64006400u)), mul, add);
     return tc_h2_bits(EXACT ? q : __hmul2(q, s));
 }
-template <bool EXACT>
+template <int EXACT>
 __device__ __forceinline__ uint4 tc_word(uint32_t w, __half2 mul, __half2 add, __half2 s) {
     return make_uint4(tc_pair<EXACT, 0>(w, mul, add, s), tc_pair<EXACT, 1>(w, mul, add, s), tc_pair<EXACT, 2>(w, mul, add, s), tc_pair<EXACT, 3>(w, mul, add, s));
 }
@@ -90,9 +90,10 @@ __device__ __forceinline__ void tc_store_y(const lb_bgemm_params& p, size_t o, f
     else reinterpret_cast<__half*>(p.y)[o] = __float2half_rn(v);
 }
 
-// SETS: converting sets of four warps (a set = the 128 columns).
+// SETS: converting sets of four warps (a set = the 128 columns); the exact kernels have fewer, their reading warps need the registers (spilling there cost
+// 20 %: 17408 -> 5120 at 32 tokens 38.2 us with three sets, 31.3 with two; at 16 tokens 31.0 with registers for 32 tokens, 27.1 with those for 16).
 // HALVES (129..256 tokens): a K-group of activations is 64 KB, so they have a ring of their own of 64-k halves, seven of which fit beside four weight stages.
-template <bool EXACT, int SETS, bool HALVES>
+template <int EXACT, int SETS, bool HALVES> // EXACT: 0, or the tokens the product carries (16, 32)
 __device__ __forceinline__ void gemm_int4_tc_body(const lb_bgemm_params& p, unsigned char* tc_smem) {
     __shared__ __align__(8) uint64_t bar_free[TC_STAGES]; // a stage's products are done (tcgen05.commit)
     __shared__ __align__(8) uint64_t bar_full[TC_STAGES]; // a stage's weights are in place (one arrival per warp of the set) and its activations have landed (transaction bytes)
@@ -101,7 +102,7 @@ __device__ __forceinline__ void gemm_int4_tc_body(const lb_bgemm_params& p, unsi
     __shared__ __align__(8) uint64_t bar_done;
     __shared__ uint32_t tmem_base_slot;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int NT = EXACT ? (p.B > 16 ? 32 : 16) : p.B > 128 ? 256 : p.B > 64 ? 128 : p.B > 32 ? 64 : p.B > 16 ? 32 : 16; // tokens the product carries (rows past B are zero)
+    const int NT = EXACT ? EXACT : p.B > 128 ? 256 : p.B > 64 ? 128 : p.B > 32 ? 64 : p.B > 16 ? 32 : 16; // tokens the product carries (rows past B are zero)
     const uint32_t a0 = EXACT ? TC_ACCS * 32u : NT > 64 ? (uint32_t)NT : 64u; // first column of the weight stages
     // Stages: what tensor memory and shared memory hold.  At least SETS: a set waits for the K-group `stages` back with the parity of an mbarrier, and with fewer
     // stages it could be two phases ahead of it.
@@ -137,7 +138,7 @@ __device__ __forceinline__ void gemm_int4_tc_body(const lb_bgemm_params& p, unsi
     pdl_wait();
 
     bool failed = false;
-    float sum[EXACT ? 32 : 1]; // EXACT: the reading warps' sums, one per token
+    float sum[EXACT ? EXACT : 1]; // EXACT: the reading warps' sums, one per token
     constexpr int CV_WARPS = 4 * SETS;
     if (warp < CV_WARPS) {
         // ---------------- converting warps: set i takes the K-groups i, i + SETS, ... ----------------
@@ -298,9 +299,9 @@ __device__ __forceinline__ void gemm_int4_tc_body(const lb_bgemm_params& p, unsi
         uint16_t sc[TC_ACCS];
 #pragma unroll
         for (int u = 0; u < TC_ACCS; ++u) sc[u] = live && u < n_groups ? __ldg(sptr + (size_t)u * p.N) : (uint16_t)0;
-        float part[32]; // the sums of up to eight K-groups: two levels, so that a long K slice is no less exact than a short one
+        float part[EXACT ? EXACT : 1]; // the sums of up to eight K-groups: two levels, so that a long K slice is no less exact than a short one
 #pragma unroll
-        for (int j = 0; j < 32; ++j) sum[j] = part[j] = 0.f;
+        for (int j = 0; j < EXACT; ++j) sum[j] = part[j] = 0.f;
         int st = 0;
         uint32_t ph = 0u;
         for (int i0 = 0; i0 < n_groups && !failed; i0 += TC_ACCS) {
@@ -320,22 +321,22 @@ __device__ __forceinline__ void gemm_int4_tc_body(const lb_bgemm_params& p, unsi
                     uint32_t r[16];
                     tmem_ld16(tmem + lanes + (uint32_t)(32 * u), r);
                     tmem_ld_wait();
+                    if (EXACT > 16) { // half of the tokens after the other: sums, parts and all 32 results would not fit the registers
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) part[j] = fmaf(s, __uint_as_float(r[j]), part[j]);
-                    if (NT > 16) {
+                        for (int j = 0; j < 16; ++j) part[j] = fmaf(s, __uint_as_float(r[j]), part[j]);
                         tmem_ld16(tmem + lanes + (uint32_t)(32 * u + 16), r);
                         tmem_ld_wait();
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) part[16 + j] = fmaf(s, __uint_as_float(r[j]), part[16 + j]);
                     }
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&bar_read[u]);
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) part[EXACT - 16 + j] = fmaf(s, __uint_as_float(r[j]), part[EXACT - 16 + j]);
                 }
             }
             if ((i0 & TC_ACCS) || i0 + TC_ACCS >= n_groups) {
 #pragma unroll
-                for (int j = 0; j < 32; ++j) {
+                for (int j = 0; j < EXACT; ++j) {
                     sum[j] += part[j];
                     part[j] = 0.f;
                 }
@@ -350,8 +351,7 @@ __device__ __forceinline__ void gemm_int4_tc_body(const lb_bgemm_params& p, unsi
     // accumulator: TMEM lane = column of the tile, TMEM column = token
     if (!failed && EXACT && warp >= CV_WARPS + 2) {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) {
-            if (j >= NT) continue;
+        for (int j = 0; j < EXACT; ++j) {
             if (KS > 1) pt[j * TC_PSTRIDE + 32 * (warp & 3) + lane] = sum[j];
             else if (live && j < p.B) tc_store_y(p, (size_t)j * p.N + n, sum[j]);
         }
@@ -401,13 +401,17 @@ __device__ __forceinline__ void gemm_int4_tc_body(const lb_bgemm_params& p, unsi
 
 extern "C" __global__ void __launch_bounds__(LB_TC_THREADS, 1) gemm_int4_tc(const __grid_constant__ lb_bgemm_params p) { // 9..128 tokens
     extern __shared__ __align__(1024) unsigned char tc_smem[];
-    gemm_int4_tc_body<false, 4, false>(p, tc_smem);
+    gemm_int4_tc_body<0, 4, false>(p, tc_smem);
 }
 extern "C" __global__ void __launch_bounds__(LB_TC_THREADS, 1) gemm_int4_tc_256(const __grid_constant__ lb_bgemm_params p) { // 129..256 tokens
     extern __shared__ __align__(1024) unsigned char tc_smem[];
-    gemm_int4_tc_body<false, 4, true>(p, tc_smem);
+    gemm_int4_tc_body<0, 4, true>(p, tc_smem);
 }
-extern "C" __global__ void __launch_bounds__(LB_TC_EXACT_THREADS, 1) gemm_int4_tc_exact(const __grid_constant__ lb_bgemm_params p) { // up to 32 tokens
+extern "C" __global__ void __launch_bounds__(LB_TC_EXACT16_THREADS, 1) gemm_int4_tc_exact16(const __grid_constant__ lb_bgemm_params p) { // up to 16 tokens
     extern __shared__ __align__(1024) unsigned char tc_smem[];
-    gemm_int4_tc_body<true, 3, false>(p, tc_smem);
+    gemm_int4_tc_body<16, 3, false>(p, tc_smem);
+}
+extern "C" __global__ void __launch_bounds__(LB_TC_EXACT32_THREADS, 1) gemm_int4_tc_exact32(const __grid_constant__ lb_bgemm_params p) { // 17..32 tokens
+    extern __shared__ __align__(1024) unsigned char tc_smem[];
+    gemm_int4_tc_body<32, 2, false>(p, tc_smem);
 }

@@ -140,7 +140,8 @@ typedef struct {
 
 /* ---- batched int4 projection: Y[B,N] = X[B,K] W ------------------------- */
 #define LB_TC_THREADS 576       /* gemm_int4_tc, gemm_int4_tc_256: 16 converting warps, the issuing and the activation warp */
-#define LB_TC_EXACT_THREADS 576 /* gemm_int4_tc_exact: 12 converting warps, those two, and four warps that scale and add the K-groups' products */
+#define LB_TC_EXACT16_THREADS 576 /* gemm_int4_tc_exact16: 12 converting warps, those two, and four warps that scale and add the K-groups' products */
+#define LB_TC_EXACT32_THREADS 448 /* gemm_int4_tc_exact32: 8 converting warps, so that the sums of 32 tokens stay in registers */
 #define LB_TC_X_HALVES 7        /* gemm_int4_tc_256: 64-k halves of a K-group's activations in shared memory (32 KB each) */
 typedef struct {
     /* gemm_int4_tc: CUtensorMap over X [B, K] fp16, box 64 k x NT tokens, 128-byte swizzle */
