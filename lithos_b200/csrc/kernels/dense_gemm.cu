@@ -125,8 +125,9 @@ extern "C" __global__ void __launch_bounds__(LB_DG_THREADS, 1) gemm_bf16_tc(cons
     pdl_wait();
     const int n_tiles = p.plan_tiles ? p.plan_n[0] * p.tiles[0] : (p.tiles[0] + p.tiles[1]) * p.t_tiles;
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0) {
         // ---------------- operands ----------------
+        if (tc_elect()) {
         int s = 0, issued = 0;
         uint32_t ph = 0;
         bool ok = true;
@@ -151,8 +152,11 @@ extern "C" __global__ void __launch_bounds__(LB_DG_THREADS, 1) gemm_bf16_tc(cons
                 if (--s < 0) { s = S - 1; ph ^= 1u; }
                 tc_wait(&bar_full[s], ph);
             }
-    } else if (warp == 1 && lane == 0) {
+        }
+        __syncwarp();
+    } else if (warp == 1) {
         // ---------------- products ----------------
+        if (tc_elect()) {
         const uint32_t idesc = tc_idesc_bf16(LB_DG_ROWS, (uint32_t)NT);
         int s = 0, it = 0;
         uint32_t ph = 0;
@@ -183,7 +187,9 @@ extern "C" __global__ void __launch_bounds__(LB_DG_THREADS, 1) gemm_bf16_tc(cons
             }
             if (ok) tc_commit(&bar_acc[b]);
         }
-    } else if (warp >= 2) {
+        }
+        __syncwarp();
+    } else {
         // ---------------- epilogue: warp w reads the tensor-memory lanes 32 (w % 4) .. + 31 ----------------
         const int quad = warp & 3;
         int it = 0;
