@@ -362,9 +362,7 @@ int lb_launch(lb_ctx* c, int kernel, unsigned gx, unsigned gy, unsigned gz, unsi
     return lb_launch_cluster(c, kernel, gx, gy, gz, bx, smem, params, pdl, 1);
 }
 
-/* cluster_y > 1: the gy CTAs of a column are launched as one thread-block cluster (gy % cluster_y == 0) */
-int lb_launch_cluster(lb_ctx* c, int kernel, unsigned gx, unsigned gy, unsigned gz, unsigned bx, unsigned smem,
-                      void** params, int pdl, unsigned cluster_y) {
+static int launch(lb_ctx* c, int kernel, unsigned gx, unsigned gy, unsigned gz, unsigned bx, unsigned smem, void** params, int pdl, unsigned cluster_x, unsigned cluster_y) {
     if (!c->fn[kernel]) return lb_fail(c, LB_ERR_NO_KERNEL, "kernel %s not loaded", k_kernel_names[kernel]);
     if (gx == 0 || gy == 0 || gz == 0) return lb_fail(c, LB_ERR_INVALID, "empty grid for %s", k_kernel_names[kernel]);
     if ((int)smem > c->max_smem_optin - ((c->fn_static_smem[kernel] + 1023) & ~1023))
@@ -384,10 +382,11 @@ int lb_launch_cluster(lb_ctx* c, int kernel, unsigned gx, unsigned gy, unsigned 
         attr[na].value.programmaticStreamSerializationAllowed = 1;
         na++;
     }
-    if (cluster_y > 1) {
+    if (cluster_x > 1 || cluster_y > 1) {
+        if (gx % cluster_x) return lb_fail(c, LB_ERR_INVALID, "grid.x %u not a multiple of the cluster size %u", gx, cluster_x);
         if (gy % cluster_y) return lb_fail(c, LB_ERR_INVALID, "grid.y %u not a multiple of the cluster size %u", gy, cluster_y);
         attr[na].id = CU_LAUNCH_ATTRIBUTE_CLUSTER_DIMENSION;
-        attr[na].value.clusterDim.x = 1;
+        attr[na].value.clusterDim.x = cluster_x;
         attr[na].value.clusterDim.y = cluster_y;
         attr[na].value.clusterDim.z = 1;
         na++;
@@ -400,6 +399,17 @@ int lb_launch_cluster(lb_ctx* c, int kernel, unsigned gx, unsigned gy, unsigned 
     if (r != CUDA_SUCCESS) return lb_cu(c, r, k_kernel_names[kernel]);
     c->launches++;
     return LB_OK;
+}
+
+/* cluster_y > 1: the gy CTAs of a column are launched as one thread-block cluster (gy % cluster_y == 0) */
+int lb_launch_cluster(lb_ctx* c, int kernel, unsigned gx, unsigned gy, unsigned gz, unsigned bx, unsigned smem,
+                      void** params, int pdl, unsigned cluster_y) {
+    return launch(c, kernel, gx, gy, gz, bx, smem, params, pdl, 1, cluster_y);
+}
+
+/* `pairs` clusters of two CTAs, neighbours in x: a kernel with cta_group::2 instructions is refused any other shape */
+int lb_launch_pairs(lb_ctx* c, int kernel, unsigned pairs, unsigned bx, unsigned smem, void** params, int pdl) {
+    return launch(c, kernel, 2 * pairs, 1, 1, bx, smem, params, pdl, 2, 1);
 }
 
 /* ---- generic module load + launch --------------------------------------------

@@ -128,6 +128,7 @@ int lb_driver_load(char* err, size_t errlen); /* LB_OK or LB_ERR_NO_DRIVER */
     X(rows_gemv_ln)                   \
     X(rows_gemv_experts)              \
     X(gemm_bf16_tc)                   \
+    X(gemm_bf16_tc_pair)              \
     X(gemm_f32_simt)                  \
     X(norm_rows2)                     \
     X(norm_rows_any)                  \
@@ -252,6 +253,7 @@ int lb_launch(lb_ctx* c, int kernel, unsigned gx, unsigned gy, unsigned gz, unsi
               int pdl);
 int lb_launch_cluster(lb_ctx* c, int kernel, unsigned gx, unsigned gy, unsigned gz, unsigned bx, unsigned smem,
                       void** params, int pdl, unsigned cluster_y);
+int lb_launch_pairs(lb_ctx* c, int kernel, unsigned pairs, unsigned bx, unsigned smem, void** params, int pdl);
 
 unsigned char* lb_map_file(const char* path, size_t* bytes); /* lb_safetensors.c: a whole file, read-only */
 

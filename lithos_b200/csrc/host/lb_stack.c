@@ -522,14 +522,18 @@ static double product_cost(const lb_ctx* c, int row_tiles, int T, int* nt_out) {
     return best;
 }
 
-static int launch_tc(lb_ctx* c, lb_dgemm_params* p, int tiles) { /* operand stages, accumulator columns, CTAs */
-    const int stage = LB_DG_ROWS * LB_DG_KB * 2 + p->NT * LB_DG_KB * 2;
+/* operand stages, accumulator columns, CTAs; pair: tiles of 256 weight rows (p->tiles counts those), half of a tile's tokens per CTA */
+static int launch_tc(lb_ctx* c, lb_dgemm_params* p, int tiles, int pair) {
+    const int stage = LB_DG_ROWS * LB_DG_KB * 2 + (pair ? p->NT / 2 : p->NT) * LB_DG_KB * 2, slots = pair ? c->sm_count / 2 : c->sm_count;
     p->stages = 200 * 1024 / stage;
     if (p->stages > LB_DG_MAX_STAGES) p->stages = LB_DG_MAX_STAGES;
     for (p->tmem_cols = 32; p->tmem_cols < 2 * p->NT;) p->tmem_cols *= 2;
     void* params[] = {p};
-    return lb_launch(c, LBK_gemm_bf16_tc, (unsigned)(tiles < c->sm_count ? tiles : c->sm_count), 1, 1, LB_DG_THREADS, (unsigned)(p->stages * stage), params, 1);
+    const unsigned n = (unsigned)(tiles < slots ? tiles : slots);
+    if (pair) return lb_launch_pairs(c, LBK_gemm_bf16_tc_pair, n, LB_DG_THREADS, (unsigned)(p->stages * stage), params, 1);
+    return lb_launch(c, LBK_gemm_bf16_tc, n, 1, 1, LB_DG_THREADS, (unsigned)(p->stages * stage), params, 1);
 }
+static int pair_tiles(const lb_dgemm_params* p, int i) { return (p->rows[i] + 2 * LB_DG_ROWS - 1) / (2 * LB_DG_ROWS); }
 
 /* one or two products Y = X W^T of a chunk (w[1] may be NULL) */
 typedef struct { const st_mat* w; CUdeviceptr x; CUdeviceptr y; int y_mode, ld_y; int ld_x, head, head_p; } st_prod; /* ld_x 0: K; head: LB_DY_HEADS */
@@ -552,13 +556,19 @@ static int launch_products(lb_model* m, const st_prod* pr, int n, int T) {
     void* params[] = {&p};
     if (S->esz == 4)
         return lb_launch(c, LBK_gemm_f32_simt, (unsigned)((p.rows[0] + 63) / 64 + (p.rows[1] + 63) / 64), (unsigned)((T + 63) / 64), 1, 256, 0, params, 1);
+    /* Whole token tiles run on CTA pairs where that does not take more waves (their tiles are larger) and a CTA has 8192 columns of k to go through: its rate is
+     * higher (us, single / pair, 1024 tokens: 30720 rows of 4096 203 / 196, 4096 rows of 16384 113 / 108, 2048 rows of 8192, 2048 tokens, 65 / 64), but pairs
+     * start about a microsecond later (2048 rows of 4096, 2048 tokens, 41.4 / 43) */
+    const int tiles = (p.tiles[0] + p.tiles[1]) * p.t_tiles, tiles2 = (pair_tiles(&p, 0) + pair_tiles(&p, 1)) * p.t_tiles, slots2 = c->sm_count / 2;
+    const int waves2 = (tiles2 + slots2 - 1) / slots2, pair = p.NT == 256 && waves2 <= (tiles + c->sm_count - 1) / c->sm_count && waves2 * p.K >= 8192;
     for (int i = 0; i < n; i++) {
         CUtensorMap tm;
         memcpy(p.tmap_w[i], &pr[i].w->tmap, sizeof tm);
-        LB_TRY(map_rows_ld(c, &tm, pr[i].x, T, p.K, p.ld_x, p.NT));
+        LB_TRY(map_rows_ld(c, &tm, pr[i].x, T, p.K, p.ld_x, pair ? p.NT / 2 : p.NT));
         memcpy(p.tmap_x[i], &tm, sizeof tm);
+        if (pair) p.tiles[i] = pair_tiles(&p, i);
     }
-    return launch_tc(c, &p, (p.tiles[0] + p.tiles[1]) * p.t_tiles);
+    return launch_tc(c, &p, pair ? tiles2 : tiles, pair);
 }
 
 /* the expert products of a chunk: `n` assignments sorted by expert, tile by tile of the plan */
@@ -598,7 +608,7 @@ static int launch_experts(lb_model* m, const lb_stack_layer* D, const st_mat* w,
     memcpy(p.tmap_w[0], &w->tmap, sizeof tm);
     LB_TRY(map_rows(c, &tm, x, n, p.K, p.NT));
     memcpy(p.tmap_x[0], &tm, sizeof tm);
-    return launch_tc(c, &p, max_tt * p.tiles[0]);
+    return launch_tc(c, &p, max_tt * p.tiles[0], 0);
 }
 static int launch_plan(lb_model* m, int i, int pos0, int T, CUdeviceptr plan) {
     const stack_t* S = S_of(m);

@@ -21,23 +21,30 @@ __device__ __forceinline__ void dg_tma(uint32_t dst_smem, const void* tmap, int 
                  : "memory");
 }
 
+__device__ __forceinline__ void dg_tma2(uint32_t dst_smem, const void* tmap, int k, int row, uint32_t cluster_bar) { // into this CTA, bytes counted at either CTA's barrier
+    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst_smem),
+                 "l"(tmap), "r"(k), "r"(row), "r"(cluster_bar)
+                 : "memory");
+}
+
 // tile t of a launch: product m, weight rows from row (row in its matrix: n0), tokens tok .. end - 1.  With experts a token tile is an entry
 // of the plan and the expert's rows are rows of the stack.
 struct dg_tile { int m, row, n0, tok, end; };
+template <int ROWS>
 __device__ __forceinline__ dg_tile dg_find(const lb_dgemm_params& p, int t) {
     dg_tile d;
     if (p.plan_tiles) {
         const int tt = t / p.tiles[0];
         const int4 e = __ldg(reinterpret_cast<const int4*>(p.plan_tiles) + tt);
         d.m = 0;
-        d.n0 = (t - tt * p.tiles[0]) * LB_DG_ROWS;
+        d.n0 = (t - tt * p.tiles[0]) * ROWS;
         d.row = e.x * p.expert_rows + d.n0;
         d.tok = e.y;
         d.end = e.z;
     } else {
         const int rt = t / p.t_tiles, tt = t - rt * p.t_tiles;
         d.m = rt >= p.tiles[0];
-        d.row = d.n0 = (d.m ? rt - p.tiles[0] : rt) * LB_DG_ROWS;
+        d.row = d.n0 = (d.m ? rt - p.tiles[0] : rt) * ROWS;
         d.tok = tt * p.NT;
         d.end = p.T;
     }
@@ -98,13 +105,16 @@ __device__ __forceinline__ void dg_finish(const lb_dgemm_params& p, int m, uint3
     }
 }
 
-extern "C" __global__ void __launch_bounds__(LB_DG_THREADS, 1) gemm_bf16_tc(const __grid_constant__ lb_dgemm_params p) {
-    extern __shared__ __align__(1024) unsigned char dg_sm[];
+template <bool PAIR>
+__device__ __forceinline__ void gemm_bf16_body(const lb_dgemm_params& p, unsigned char* dg_sm) {
+    constexpr int ROWS = PAIR ? 2 * LB_DG_ROWS : LB_DG_ROWS;
     __shared__ __align__(8) uint64_t bar_full[LB_DG_MAX_STAGES], bar_empty[LB_DG_MAX_STAGES], bar_acc[2], bar_free[2];
     __shared__ uint32_t tmem_slot;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int S = p.stages, NT = p.NT;
-    const uint32_t a_bytes = LB_DG_ROWS * LB_DG_KB * 2, b_bytes = (uint32_t)NT * LB_DG_KB * 2, stage_bytes = a_bytes + b_bytes;
+    const uint32_t a_bytes = LB_DG_ROWS * LB_DG_KB * 2, b_bytes = (uint32_t)(PAIR ? NT / 2 : NT) * LB_DG_KB * 2, stage_bytes = a_bytes + b_bytes;
+    const int rank = PAIR ? (int)tc2_rank() : 0;
+    const int tile0 = PAIR ? (int)blockIdx.x >> 1 : (int)blockIdx.x, step = PAIR ? (int)gridDim.x >> 1 : (int)gridDim.x;
     const int ksteps = p.K / LB_DG_KB;
     if (tid == 0) {
         for (int s = 0; s < S; ++s) {
@@ -113,13 +123,17 @@ extern "C" __global__ void __launch_bounds__(LB_DG_THREADS, 1) gemm_bf16_tc(cons
         }
         for (int s = 0; s < 2; ++s) {
             mbar_init(&bar_acc[s], 1);
-            mbar_init(&bar_free[s], 4);
+            mbar_init(&bar_free[s], PAIR ? 8 : 4);
         }
         mbar_fence_init();
     }
-    if (warp == 1) tmem_alloc(&tmem_slot, (uint32_t)p.tmem_cols);
+    if (warp == 1) {
+        if (PAIR) tmem_alloc2(&tmem_slot, (uint32_t)p.tmem_cols);
+        else tmem_alloc(&tmem_slot, (uint32_t)p.tmem_cols);
+    }
     tc_fence_before();
     __syncthreads();
+    if (PAIR) tc2_sync(); // both CTAs have their barriers and their tensor memory
     tc_fence_after();
     const uint32_t tmem = tmem_slot;
     pdl_wait();
@@ -131,23 +145,29 @@ extern "C" __global__ void __launch_bounds__(LB_DG_THREADS, 1) gemm_bf16_tc(cons
         int s = 0, issued = 0;
         uint32_t ph = 0;
         bool ok = true;
-        for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-            const dg_tile d = dg_find(p, tile);
+        for (int tile = tile0; tile < n_tiles && ok; tile += step) {
+            const dg_tile d = dg_find<ROWS>(p, tile);
             for (int k = 0; k < ksteps; ++k) {
                 if (issued >= S && !tc_wait(&bar_empty[s], ph ^ 1u)) {
                     ok = false;
                     if (p.status) atomicExch(p.status, DG_FAIL_EMPTY);
                     break;
                 }
-                mbar_arrive_expect_tx(&bar_full[s], stage_bytes);
+                if (rank == 0) mbar_arrive_expect_tx(&bar_full[s], PAIR ? 2 * stage_bytes : stage_bytes);
                 const uint32_t dst = smem_u32(dg_sm) + (uint32_t)s * stage_bytes;
-                dg_tma(dst, p.tmap_w[d.m], k * LB_DG_KB, d.row, &bar_full[s]);
-                dg_tma(dst + a_bytes, p.tmap_x[d.m], k * LB_DG_KB, d.tok, &bar_full[s]);
+                if (PAIR) { // a CTA brings its 128 weight rows and its half of the tokens; the first one's barrier counts all of it
+                    const uint32_t full = tc2_leader(&bar_full[s]);
+                    dg_tma2(dst, p.tmap_w[d.m], k * LB_DG_KB, d.row + rank * LB_DG_ROWS, full);
+                    dg_tma2(dst + a_bytes, p.tmap_x[d.m], k * LB_DG_KB, d.tok + rank * (NT / 2), full);
+                } else {
+                    dg_tma(dst, p.tmap_w[d.m], k * LB_DG_KB, d.row, &bar_full[s]);
+                    dg_tma(dst + a_bytes, p.tmap_x[d.m], k * LB_DG_KB, d.tok, &bar_full[s]);
+                }
                 ++issued;
                 if (++s == S) { s = 0; ph ^= 1u; }
             }
         }
-        if (!ok) // nothing may still be on its way into this CTA's shared memory when it ends
+        if (!ok && rank == 0) // nothing may still be on its way into this CTA's shared memory when it ends
             for (int i = 0; i < S && i < issued; ++i) {
                 if (--s < 0) { s = S - 1; ph ^= 1u; }
                 tc_wait(&bar_full[s], ph);
@@ -156,14 +176,14 @@ extern "C" __global__ void __launch_bounds__(LB_DG_THREADS, 1) gemm_bf16_tc(cons
         __syncwarp();
     } else if (warp == 1) {
         // ---------------- products ----------------
-        if (tc_elect()) {
-        const uint32_t idesc = tc_idesc_bf16(LB_DG_ROWS, (uint32_t)NT);
+        if (rank == 0 && tc_elect()) {
+        const uint32_t idesc = tc_idesc_bf16(ROWS, (uint32_t)NT);
         int s = 0, it = 0;
         uint32_t ph = 0;
         bool ok = true;
-        for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x, ++it) {
+        for (int tile = tile0; tile < n_tiles && ok; tile += step, ++it) {
             const int b = it & 1;
-            if (it >= 2 && !tc_wait(&bar_free[b], (uint32_t)((it >> 1) - 1) & 1u)) { // the epilogue has read this accumulator
+            if (it >= 2 && !(PAIR ? tc2_wait(&bar_free[b], (uint32_t)((it >> 1) - 1) & 1u) : tc_wait(&bar_free[b], (uint32_t)((it >> 1) - 1) & 1u))) { // the epilogue has read this accumulator
                 ok = false;
                 if (p.status) atomicExch(p.status, DG_FAIL_ACC);
                 break;
@@ -180,12 +200,16 @@ extern "C" __global__ void __launch_bounds__(LB_DG_THREADS, 1) gemm_bf16_tc(cons
                 const uint32_t base = smem_u32(dg_sm) + (uint32_t)s * stage_bytes;
                 const uint64_t ad = tc_smem_desc(base, 16, 1024), bd = tc_smem_desc(base + a_bytes, 16, 1024);
 #pragma unroll
-                for (int kk = 0; kk < LB_DG_KB / 16; ++kk)
-                    tc_mma(d, ad + (uint64_t)(kk * 2), bd + (uint64_t)(kk * 2), idesc, (k > 0 || kk > 0) ? 1u : 0u);
-                tc_commit(&bar_empty[s]);
+                for (int kk = 0; kk < LB_DG_KB / 16; ++kk) {
+                    if (PAIR) tc2_mma(d, ad + (uint64_t)(kk * 2), bd + (uint64_t)(kk * 2), idesc, (k > 0 || kk > 0) ? 1u : 0u);
+                    else tc_mma(d, ad + (uint64_t)(kk * 2), bd + (uint64_t)(kk * 2), idesc, (k > 0 || kk > 0) ? 1u : 0u);
+                }
+                if (PAIR) tc2_commit(&bar_empty[s]);
+                else tc_commit(&bar_empty[s]);
                 if (++s == S) { s = 0; ph ^= 1u; }
             }
-            if (ok) tc_commit(&bar_acc[b]);
+            if (ok && PAIR) tc2_commit(&bar_acc[b]);
+            else if (ok) tc_commit(&bar_acc[b]);
         }
         }
         __syncwarp();
@@ -193,10 +217,10 @@ extern "C" __global__ void __launch_bounds__(LB_DG_THREADS, 1) gemm_bf16_tc(cons
         // ---------------- epilogue: warp w reads the tensor-memory lanes 32 (w % 4) .. + 31 ----------------
         const int quad = warp & 3;
         int it = 0;
-        for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++it) {
+        for (int tile = tile0; tile < n_tiles; tile += step, ++it) {
             const int b = it & 1;
-            const dg_tile d = dg_find(p, tile);
-            const int m = d.m, n = d.n0 + quad * 32 + lane, t0 = d.tok;
+            const dg_tile d = dg_find<ROWS>(p, tile);
+            const int m = d.m, n = d.n0 + rank * LB_DG_ROWS + quad * 32 + lane, t0 = d.tok;
             const bool got = tc_wait(&bar_acc[b], (uint32_t)(it >> 1) & 1u);
             if (!__all_sync(0xffffffffu, got)) {
                 if (lane == 0 && p.status) atomicExch(p.status, DG_FAIL_ACC);
@@ -216,16 +240,32 @@ extern "C" __global__ void __launch_bounds__(LB_DG_THREADS, 1) gemm_bf16_tc(cons
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&bar_free[b]);
+            if (lane == 0) {
+                if (PAIR) tc2_arrive(tc2_leader(&bar_free[b]));
+                else mbar_arrive(&bar_free[b]);
+            }
         }
     }
     pdl_launch_dependents();
     __syncthreads();
+    if (PAIR) tc2_sync(); // nobody leaves while the other may still signal its barriers or multiply from its shared memory
     if (warp == 1) {
         tc_fence_after();
-        tmem_dealloc(tmem, (uint32_t)p.tmem_cols);
+        if (PAIR) tmem_dealloc2(tmem, (uint32_t)p.tmem_cols);
+        else tmem_dealloc(tmem, (uint32_t)p.tmem_cols);
     }
 }
+extern "C" __global__ void __launch_bounds__(LB_DG_THREADS, 1) gemm_bf16_tc(const __grid_constant__ lb_dgemm_params p) {
+    extern __shared__ __align__(1024) unsigned char dg_sm[];
+    gemm_bf16_body<false>(p, dg_sm);
+}
+// CTA pairs (clusters of two, neighbours in x): a tile is 256 weight rows x NT tokens, each CTA brings 128 rows and half of the tokens, so a
+// product's operands are two thirds of the bytes from L2 at NT = 256.
+extern "C" __global__ void __launch_bounds__(LB_DG_THREADS, 1) gemm_bf16_tc_pair(const __grid_constant__ lb_dgemm_params p) {
+    extern __shared__ __align__(1024) unsigned char dg_sm[];
+    gemm_bf16_body<true>(p, dg_sm);
+}
+
 
 // ---- fp32 ----------------------------------------------------------------------------------------------------------
 #define SG_TN 64 // weight rows per tile
