@@ -68,16 +68,13 @@ __device__ __forceinline__ void tc2_commit(uint64_t* bar) { // the barrier of bo
 __device__ __forceinline__ void tc2_arrive(uint32_t cluster_bar) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
 }
-__device__ __forceinline__ bool tc2_wait(uint64_t* bar, uint32_t parity) { // as tc_wait, for a barrier that the other CTA arrives at
-    for (uint32_t i = 0; i < (1u << 24); ++i) {
-        uint32_t ok;
-        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                     : "=r"(ok)
-                     : "r"(smem_u32(bar)), "r"(parity)
-                     : "memory");
-        if (ok) return true;
-    }
-    return false;
+__device__ __forceinline__ bool tc2_try_wait(uint64_t* bar, uint32_t parity) { // as mbar_try_wait, for a barrier that the other CTA arrives at
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok)
+                 : "r"(smem_u32(bar)), "r"(parity)
+                 : "memory");
+    return ok != 0;
 }
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) { // 32 lanes x 16 consecutive columns
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
@@ -110,9 +107,23 @@ __device__ __forceinline__ bool tc_test_wait(uint64_t* bar, uint32_t parity) { /
                  : "memory");
     return ok != 0;
 }
-// Bounded wait of the single-thread roles (and of one lane of a warp) on a pipeline mbarrier: 16M polls at most, no global timer.
-__device__ __forceinline__ bool tc_wait(uint64_t* bar, uint32_t parity) {
-    for (uint32_t i = 0; i < (1u << 24); ++i)
-        if (mbar_try_wait(bar, parity)) return true;
+// Bounded waits of the single-thread roles (and of one lane of a warp) on a pipeline mbarrier.  A poll may suspend the thread for as long as the
+// hardware likes, so the bound is LB_WAIT_NS of the clock beside a number of polls; the clock is read every 16th poll, which a wait of ordinary
+// length (a few polls) never reaches.
+template <typename Poll> __device__ __forceinline__ bool tc_wait_by(Poll poll) {
+    uint64_t t0 = 0;
+    for (uint32_t i = 1; i < (1u << 24); ++i) {
+        if (poll()) return true;
+        if (i & 15u) continue;
+        const uint64_t t = globaltimer_ns();
+        if (t0 == 0) t0 = t;
+        else if (t - t0 > LB_WAIT_NS) break;
+    }
     return false;
+}
+__device__ __forceinline__ bool tc_wait(uint64_t* bar, uint32_t parity) {
+    return tc_wait_by([&] { return mbar_try_wait(bar, parity); });
+}
+__device__ __forceinline__ bool tc2_wait(uint64_t* bar, uint32_t parity) {
+    return tc_wait_by([&] { return tc2_try_wait(bar, parity); });
 }
