@@ -127,7 +127,10 @@ __device__ __forceinline__ void gemm_int4_tc_body(const lb_bgemm_params& p, unsi
         mbar_init(&bar_done, 1);
         mbar_fence_init();
     }
-    if (warp == 0) tmem_alloc(&tmem_base_slot, TC_TMEM_COLS);
+    if (warp == 0) {
+        __syncwarp(); // lane 0 comes from the barriers; the allocation is one of the whole warp
+        tmem_alloc(&tmem_base_slot, TC_TMEM_COLS);
+    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -135,6 +138,10 @@ __device__ __forceinline__ void gemm_int4_tc_body(const lb_bgemm_params& p, unsi
     const uint32_t lanes = (uint32_t)(32 * (warp & 3)) << 16; // a warp reaches the tensor-memory lanes 32 (warp % 4) .. + 31
     const int n = blockIdx.x * TC_COLS + 32 * (warp & 3) + lane; // this thread's column
     const bool live = n < p.N;
+    // Lanes past the last column (N % 32 == 16) load the last column's words, so that no load splits a warp in front of its tensor-memory
+    // instructions, which the whole warp has to execute together; their products stay in lanes that nobody stores.  A warp without any column loads nothing.
+    const bool any_live = n - lane < p.N;
+    const int nl = min(n, p.N - 1);
     pdl_wait();
 
     bool failed = false;
@@ -144,9 +151,9 @@ __device__ __forceinline__ void gemm_int4_tc_body(const lb_bgemm_params& p, unsi
         // ---------------- converting warps: set i takes the K-groups i, i + SETS, ... ----------------
         const int set = warp >> 2;
         const size_t N = (size_t)p.N;
-        const uint32_t* qptr = p.qweight + (size_t)(g_begin + set) * 16 * N + n;
-        const uint16_t* sptr = p.scales + (size_t)(g_begin + set) * N + n;
-        const uint32_t* zptr = p.qzeros ? p.qzeros + (size_t)(g_begin + set) * (N / 8) + (n >> 3) : nullptr;
+        const uint32_t* qptr = p.qweight + (size_t)(g_begin + set) * 16 * N + nl;
+        const uint16_t* sptr = p.scales + (size_t)(g_begin + set) * N + nl;
+        const uint32_t* zptr = p.qzeros ? p.qzeros + (size_t)(g_begin + set) * (N / 8) + (nl >> 3) : nullptr;
         tc_group ring[2]; // the set's next two K-groups
         auto load_words = [&](tc_group& w, int c) { // a quarter of a K-group's words; the last one steps to the next K-group
 #pragma unroll
@@ -165,13 +172,13 @@ __device__ __forceinline__ void gemm_int4_tc_body(const lb_bgemm_params& p, unsi
             for (int j = 0; j < 16; ++j) ring[u].w[j] = 0u;
             ring[u].s = 0u;
             ring[u].zw = 0x88888888u;
-            if (live && set + SETS * u < n_groups) {
+            if (any_live && set + SETS * u < n_groups) {
 #pragma unroll
                 for (int c = 0; c < 4; ++c) load_words(ring[u], c);
             }
         }
         const __half2 mul = tc_bits_h2(0x2C003C00u); // (1, 1/16)
-        const int zshift = 4 * (n & 7);
+        const int zshift = 4 * (nl & 7);
         int st = set; // stage (and its phase) of the K-group the set works on
         uint32_t ph = 0u;
         for (int g0 = set; g0 < n_groups && !failed; g0 += 2 * SETS) {
@@ -182,7 +189,7 @@ __device__ __forceinline__ void gemm_int4_tc_body(const lb_bgemm_params& p, unsi
                     const uint32_t z = (ring[u].zw >> zshift) & 0xFu;
                     const __half2 add = tc_bits_h2((0xE400u + z) | ((0xD400u + (z << 4)) << 16)); // (-(1024 + z), -(64 + z))
                     const __half2 sc = tc_bits_h2((ring[u].s & 0xFFFFu) * 0x10001u);
-                    const bool more = live && g + 2 * SETS < n_groups;
+                    const bool more = any_live && g + 2 * SETS < n_groups;
                     // the stage held the K-group `stages` back: wait until its products are done (lane 0 waits for its warp; the vote orders the
                     // others behind it).  Suspended waits, here and wherever else a wait is not on the critical path: lanes that spin on
                     // mbarriers slow every other wait of the SM down.
@@ -295,10 +302,10 @@ __device__ __forceinline__ void gemm_int4_tc_body(const lb_bgemm_params& p, unsi
         __syncwarp();
     } else if (EXACT) {
         // ---------------- reading warps: sum += scale * (the K-group's products) ----------------
-        const uint16_t* sptr = p.scales + (size_t)g_begin * p.N + n;
+        const uint16_t* sptr = p.scales + (size_t)g_begin * p.N + nl;
         uint16_t sc[TC_ACCS];
 #pragma unroll
-        for (int u = 0; u < TC_ACCS; ++u) sc[u] = live && u < n_groups ? __ldg(sptr + (size_t)u * p.N) : (uint16_t)0;
+        for (int u = 0; u < TC_ACCS; ++u) sc[u] = any_live && u < n_groups ? __ldg(sptr + (size_t)u * p.N) : (uint16_t)0;
         float part[EXACT ? EXACT : 1]; // the sums of up to eight K-groups: two levels, so that a long K slice is no less exact than a short one
 #pragma unroll
         for (int j = 0; j < EXACT; ++j) sum[j] = part[j] = 0.f;
@@ -310,7 +317,7 @@ __device__ __forceinline__ void gemm_int4_tc_body(const lb_bgemm_params& p, unsi
                 const int it = i0 + u;
                 if (it < n_groups && !failed) {
                     const float s = __half2float(__ushort_as_half(sc[u]));
-                    if (live && it + TC_ACCS < n_groups) sc[u] = __ldg(sptr + (size_t)(it + TC_ACCS) * p.N);
+                    if (any_live && it + TC_ACCS < n_groups) sc[u] = __ldg(sptr + (size_t)(it + TC_ACCS) * p.N);
                     if (lane == 0 && !mbar_wait(&bar_free[st], ph)) {
                         failed = true;
                         if (p.status) atomicExch(p.status, TC_FAIL_FREE);
@@ -359,6 +366,7 @@ __device__ __forceinline__ void gemm_int4_tc_body(const lb_bgemm_params& p, unsi
     if (!failed && !EXACT && warp < CV_WARPS) {
         for (int c = warp >> 2; c < NT / 16; c += SETS) { // the sets share the tokens
             uint32_t r[16];
+            __syncwarp(); // the stores before are some lanes' only
             tmem_ld16(tmem + lanes + (uint32_t)(c * 16), r);
             tmem_ld_wait();
 #pragma unroll

@@ -63,6 +63,7 @@ __device__ __forceinline__ void dg_finish(const lb_dgemm_params& p, int m, uint3
     const int hn = MODE == LB_DY_HEADS ? n / p.head[m] : 0, col = MODE == LB_DY_HEADS ? hn * p.head_p[m] + (n - hn * p.head[m]) : n;
     for (int c = 0; c < n_t; c += 16) {
         uint32_t r[16];
+        __syncwarp(); // the stores before are some lanes' only (rows that end inside the warp, (gate, up) pairs)
         tmem_ld16(acc + (uint32_t)c, r);
         tmem_ld_wait();
         if (MODE == LB_DY_HEADS || MODE == LB_DY_RELU2) {
