@@ -103,6 +103,8 @@ int lb_driver_load(char* err, size_t errlen); /* LB_OK or LB_ERR_NO_DRIVER */
     X(deltanet_step_f32)              \
     X(deltanet_one_bf16)              \
     X(deltanet_one_f32)               \
+    X(deltanet_two_bf16)              \
+    X(deltanet_two_f32)               \
     X(deltanet_layer_fused)           \
     X(attn_decode_split)              \
     X(attn_decode_mma)                \

@@ -147,62 +147,75 @@ __device__ __forceinline__ void dn_read(const float* row, uint64_t (&r)[4][2]) {
     }
 }
 
-// One step, where a trip to memory is all that counts: a thread holds 32 rows of one column (rows 8 q4 + 32 j + i), so that a warp's loads of
-// the state are whole sectors, all of them in flight at once behind one load per thread of k and q.  The sums are those of a run, in the
-// same order: four running sums per group of four rows, groups 2 q4 and 2 q4 + 1 first, then the column's four lanes.  (48 heads: see
-// deltanet_body; 3.8 us with the lanes of a run, whose 8-byte loads take two passes each, 4.2 us with k and q read by every thread.)
+// One or two steps, where a trip to memory is all that counts: a thread holds 32 rows of one column (rows 8 q4 + 32 j + i), so that a warp's loads
+// of the state are whole sectors, all of them in flight at once, ahead of g, beta and v and behind one load per thread of k and q.  The sums are those
+// of a run, in the same order: four running sums per group of four rows, groups 2 q4 and 2 q4 + 1 first, then the column's four lanes.
+// A single step lets its successor start as soon as its loads are on their way; two steps do not (4.8 -> 6.0 us at 96 heads).
+// us a step at 16 / 32 / 48 / 96 value heads, states not in L2 (in brackets what a run of one or two steps takes with deltanet_body): one, bf16 2.35 /
+// 2.47 / 3.07 / 4.07, fp32 2.30 / 2.41 / 3.03 / 4.13; two, bf16 2.57 / 2.71 / 3.59 / 4.71 [3.07 / 3.28 / 3.99 / 4.82], fp32 2.56 / 2.78 / 3.74 / 4.99
+// [3.04 / 3.30 / 3.96 / 4.66].
 __device__ __forceinline__ float dn_column_sum(const float (&c)[8]) {
     float x = ((c[0] + c[1]) + (c[2] + c[3])) + ((c[4] + c[5]) + (c[6] + c[7]));
     x += __shfl_xor_sync(0xffffffffu, x, 1);
     return x + __shfl_xor_sync(0xffffffffu, x, 2);
 }
-template <typename T>
-__device__ __forceinline__ void deltanet_one(const lb_deltanet_params& p) {
+template <typename T, int STEPS>
+__device__ __forceinline__ void deltanet_few(const lb_deltanet_params& p) {
     const int h = blockIdx.x, kh = h / (p.HV / p.HK), q4 = threadIdx.x & 3, j0 = blockIdx.y * DN_COLS + (threadIdx.x >> 2);
     float* S = p.state + (size_t)h * DN_D * DN_D + (size_t)(8 * q4) * DN_D + j0;
-    const size_t oi = (size_t)h * DN_D + j0;
-    constexpr int N = dn_in<T>::N;
-    __shared__ __align__(16) float kq[2][DN_D];
+    const size_t oi = (size_t)h * DN_D + j0, ld = (size_t)p.HV * DN_D;
+    constexpr int N = dn_in<T>::N, PIECES = 2 * DN_D / N; // 16-byte pieces of a token's k and q
+    static_assert(STEPS * PIECES <= DN_THREADS, "a thread brings at most one piece");
+    __shared__ __align__(16) float kq[STEPS][2][DN_D];
+    float s[4][8], c[8], g[STEPS], beta[STEPS], v[STEPS];
     pdl_wait();
     uint4 piece = make_uint4(0u, 0u, 0u, 0u);
-    if (threadIdx.x < 2 * DN_D / N)
-        piece = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(threadIdx.x < DN_D / N ? p.k : p.q) + (size_t)kh * DN_D) + threadIdx.x % (DN_D / N));
-    const float g = p.g[h], beta = p.beta[h];
-    const float v = sizeof(T) == 2 ? bf16_bits_to_f32(reinterpret_cast<const uint16_t*>(p.v)[oi]) : reinterpret_cast<const float*>(p.v)[oi];
-    float s[4][8], c[8];
+    const int pu = threadIdx.x / PIECES, pe = threadIdx.x % PIECES;
+    if (threadIdx.x < STEPS * PIECES)
+        piece = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(pe < DN_D / N ? p.k : p.q) + ((size_t)pu * p.HK + kh) * DN_D) + pe % (DN_D / N));
 #pragma unroll
     for (int j = 0; j < 4; ++j)
 #pragma unroll
         for (int i = 0; i < 8; ++i) asm volatile("ld.global.f32 %0, [%1];" : "=f"(s[j][i]) : "l"(S + (size_t)(32 * j + i) * DN_D) : "memory");
-    if (threadIdx.x < 2 * DN_D / N) dn_in<T>::put(&kq[threadIdx.x / (DN_D / N)][threadIdx.x % (DN_D / N) * N], piece);
-    __syncthreads();
-    float k[4][8], q[4][8];
+    if (STEPS == 1) pdl_launch_dependents();
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int i = 0; i < 8; i += 4) {
-            *reinterpret_cast<float4*>(&k[j][i]) = *reinterpret_cast<const float4*>(&kq[0][32 * j + 8 * q4 + i]);
-            *reinterpret_cast<float4*>(&q[j][i]) = *reinterpret_cast<const float4*>(&kq[1][32 * j + 8 * q4 + i]);
-        }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        c[i] = __fmul_rn(k[0][i], s[0][i]);
-#pragma unroll
-        for (int j = 1; j < 4; ++j) c[i] = __fmaf_rn(k[j][i], s[j][i], c[i]);
+    for (int u = 0; u < STEPS; ++u) {
+        g[u] = p.g[u * p.HV + h];
+        beta[u] = p.beta[u * p.HV + h];
+        v[u] = sizeof(T) == 2 ? bf16_bits_to_f32(reinterpret_cast<const uint16_t*>(p.v)[oi + u * ld]) : reinterpret_cast<const float*>(p.v)[oi + u * ld];
     }
-    const float d = beta * (v - dn_column_sum(c));
+    if (threadIdx.x < STEPS * PIECES) dn_in<T>::put(&kq[pu][pe / (DN_D / N)][pe % (DN_D / N) * N], piece);
+    __syncthreads();
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+    for (int u = 0; u < STEPS; ++u) {
+        float k[4][8], q[4][8];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            s[j][i] = __fmaf_rn(k[j][i], d, __fmul_rn(g, s[j][i]));
-            c[i] = j ? __fmaf_rn(q[j][i], s[j][i], c[i]) : __fmul_rn(q[j][i], s[j][i]);
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int i = 0; i < 8; i += 4) {
+                *reinterpret_cast<float4*>(&k[j][i]) = *reinterpret_cast<const float4*>(&kq[u][0][32 * j + 8 * q4 + i]);
+                *reinterpret_cast<float4*>(&q[j][i]) = *reinterpret_cast<const float4*>(&kq[u][1][32 * j + 8 * q4 + i]);
+            }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            c[i] = __fmul_rn(k[0][i], s[0][i]);
+#pragma unroll
+            for (int j = 1; j < 4; ++j) c[i] = __fmaf_rn(k[j][i], s[j][i], c[i]);
         }
-    float o = dn_column_sum(c);
-    pdl_launch_dependents();
-    if (q4 == 0) {
-        if (p.z) o *= siluf_dev(p.z[oi]);
-        p.out[oi] = o;
+        const float d = beta[u] * (v[u] - dn_column_sum(c));
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                s[j][i] = __fmaf_rn(k[j][i], d, __fmul_rn(g[u], s[j][i]));
+                c[i] = j ? __fmaf_rn(q[j][i], s[j][i], c[i]) : __fmul_rn(q[j][i], s[j][i]);
+            }
+        float o = dn_column_sum(c);
+        if (STEPS > 1 && u == STEPS - 1) pdl_launch_dependents();
+        if (q4 == 0) {
+            if (p.z) o *= siluf_dev(p.z[oi + u * ld]);
+            p.out[oi + u * ld] = o;
+        }
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j)
@@ -314,8 +327,10 @@ extern "C" __global__ void __launch_bounds__(DN_THREADS) deltanet_step_bf16(cons
                                                                             int n_steps) {
     deltanet_body<__nv_bfloat16>(p, n_steps);
 }
-extern "C" __global__ void __launch_bounds__(DN_THREADS) deltanet_one_bf16(const __grid_constant__ lb_deltanet_params p) { deltanet_one<__nv_bfloat16>(p); }
-extern "C" __global__ void __launch_bounds__(DN_THREADS) deltanet_one_f32(const __grid_constant__ lb_deltanet_params p) { deltanet_one<float>(p); }
+extern "C" __global__ void __launch_bounds__(DN_THREADS) deltanet_one_bf16(const __grid_constant__ lb_deltanet_params p) { deltanet_few<__nv_bfloat16, 1>(p); }
+extern "C" __global__ void __launch_bounds__(DN_THREADS) deltanet_one_f32(const __grid_constant__ lb_deltanet_params p) { deltanet_few<float, 1>(p); }
+extern "C" __global__ void __launch_bounds__(DN_THREADS) deltanet_two_bf16(const __grid_constant__ lb_deltanet_params p) { deltanet_few<__nv_bfloat16, 2>(p); }
+extern "C" __global__ void __launch_bounds__(DN_THREADS) deltanet_two_f32(const __grid_constant__ lb_deltanet_params p) { deltanet_few<float, 2>(p); }
 extern "C" __global__ void __launch_bounds__(DN_THREADS) deltanet_step_f32(const __grid_constant__ lb_deltanet_params p,
                                                                            int n_steps) {
     deltanet_body<float>(p, n_steps);

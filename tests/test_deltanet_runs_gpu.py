@@ -1,5 +1,5 @@
-"""GPU: a run of DeltaNet steps is its steps one by one, bit for bit, whatever its length (runs of eight tokens, read-outs four at a time),
-and both are the oracle's to fp32 rounding (sums of 128 terms, 2^-24 each, errors shrink with the state: 1e-5 of the largest value)."""
+"""GPU: a run of DeltaNet steps is its steps one by one, bit for bit, whatever its length (one step and two have kernels of their own; runs of
+eight tokens, read-outs four at a time), and both are the oracle's to fp32 rounding (sums of 128 terms, 2^-24 each, errors shrink with the state: 1e-5 of the largest value)."""
 import numpy as np
 import pytest
 
@@ -14,7 +14,7 @@ class View:
 
 
 @pytest.mark.parametrize("T", [1, 2, 3, 4, 5, 7, 8, 9, 16, 23])
-@pytest.mark.parametrize("heads", [(3, 1), (4, 2), (2, 2)])
+@pytest.mark.parametrize("heads", [(3, 1), (4, 2), (2, 2), (76, 4)])  # 76: more CTAs than two per SM, so two steps take the run's kernel
 @pytest.mark.parametrize("f32", [False, True])
 @pytest.mark.parametrize("off", [0, 4])  # the state on an 8-byte boundary and beside one
 def test_run_equals_steps(ctx, lb, oracle, T, heads, f32, off):
