@@ -210,11 +210,10 @@ LB_API int lb_gemv_int4_host(lb_ctx* c, const uint32_t* qweight, const uint16_t*
  * of one cluster (<= 8); the slice count fills the SMs without starting a second wave and leaves
  * every slice at least four K-groups. */
 
-/* clusters of k CTAs of the tcgen05 kernels (one CTA per SM) that run at once: the SMs of a GPC do not all divide by k, and one
- * cluster too many doubles the time (4096 -> 2048 at 48 tokens: 14.2 us as 16 clusters of 8, 8.0 as clusters of what fits) */
-static int tc_clusters(lb_ctx* c, int k) {
-    if (k <= 1) return c->sm_count;
-    if (!c->tc_clusters[k]) {
+/* clusters of k CTAs of a kernel that run at once, asked once per k (slot) */
+static int clusters_at_once(lb_ctx* c, int kernel, int k, unsigned threads, unsigned smem, int per_sm, int* slot) {
+    if (k <= 1) return c->sm_count * per_sm;
+    if (!*slot) {
         CUlaunchConfig cfg;
         memset(&cfg, 0, sizeof cfg);
         CUlaunchAttribute attr;
@@ -222,14 +221,47 @@ static int tc_clusters(lb_ctx* c, int k) {
         attr.id = CU_LAUNCH_ATTRIBUTE_CLUSTER_DIMENSION;
         attr.value.clusterDim.x = 1; attr.value.clusterDim.y = (unsigned)k; attr.value.clusterDim.z = 1;
         cfg.gridDimX = (unsigned)c->sm_count; cfg.gridDimY = (unsigned)k; cfg.gridDimZ = 1;
-        cfg.blockDimX = LB_TC_THREADS; cfg.blockDimY = cfg.blockDimZ = 1;
-        cfg.sharedMemBytes = LB_TC_X_HALVES * 256 * 128;
+        cfg.blockDimX = threads; cfg.blockDimY = cfg.blockDimZ = 1;
+        cfg.sharedMemBytes = smem;
         cfg.attrs = &attr; cfg.numAttrs = 1;
         int n = 0;
-        if (!c->fn[LBK_gemm_int4_tc_256] || lb_drv.OccupancyMaxActiveClusters(&n, c->fn[LBK_gemm_int4_tc_256], &cfg) != CUDA_SUCCESS || n < 1) n = c->sm_count / k;
-        c->tc_clusters[k] = n;
+        if (!c->fn[kernel] || lb_drv.OccupancyMaxActiveClusters(&n, c->fn[kernel], &cfg) != CUDA_SUCCESS || n < 1) n = c->sm_count * per_sm / k;
+        *slot = n;
     }
-    return c->tc_clusters[k];
+    return *slot;
+}
+
+/* K slices (CTAs of a cluster) of the tcgen05 kernels, one CTA per SM: the SMs of a GPC do not all divide by the slices, and one cluster
+ * too many doubles the time (4096 -> 2048 at 48 tokens: 14.2 us as 16 clusters of 8, 8.0 as clusters of what fits) */
+static int tc_slices(lb_ctx* c, int blocks, int groups) {
+    int k = c->sm_count / blocks;
+    if (k > 8) k = 8;
+    while (k > 1 && (groups / k < 4 || clusters_at_once(c, LBK_gemm_int4_tc_256, k, LB_TC_THREADS, LB_TC_X_HALVES * 256 * 128, 1, &c->tc_clusters[k]) < blocks)) k--;
+    return k < 1 ? 1 : k;
+}
+/* K slices of the mma.sync kernels, two CTAs per SM */
+static int mma_slices(const lb_ctx* c, int blocks, int groups) {
+    int k = 1;
+    while (k < 8 && blocks * k < c->sm_count * 3 / 2 && groups / (k * 2) >= 4) k *= 2;
+    return k;
+}
+
+/* 9..32 tokens without a flag: gemm_int4_tc_exact16 / 32 (1) or the mma.sync kernels (0); neither rounds a weight.  us, mma.sync / tcgen05:
+ * matrices split along K: 17408 -> 5120 at 12 tokens 33.9 / 27.1, at 32 47.5 / 31.1; 1024 -> 1024 6.9 / 5.3, 11.4 / 6.3
+ * short columns, where the start counts: K = 512 at 9 tokens 4.8 / 4.9, 640 5.5 / 5.3; K = 256 at 17 tokens 5.0 / 5.2, 384 5.7 / 5.5
+ * whole columns up to 16 tokens (two CTAs per SM against one): 5120 -> 17408 at 12 tokens 23.9 / 24.5; up to 32 tokens 34.6 / 28.0, 5120 -> 34816 54.7 / 57
+ * up to 16 tokens, long columns of which mma.sync makes twice as many slices and all of its clusters run at once (29..32 and 56..70 blocks, fewer
+ *   by one above 12 tokens): 17408 -> 7168 at 12 tokens 35.2 / 37.9, 8192 -> 7168 19.6 / 20.3, 6144 -> 7168 16.1 / 16.3 (at 16 16.5 / 16.4), 5120 -> 7168 14.5 / 14.3;
+ *   one block more than fits: 8192 -> 9216 31.3 / 20.6
+ * or four times as many while two thirds of the SMs have no tcgen05 CTA (46..49 blocks): 17408 -> 5888 35.6 / 37.6, 11008 -> 5888 26.2 / 25.6 */
+static int exact_on_tc(lb_ctx* c, int B, int blocks, int groups) {
+    if (groups <= (B > 16 ? 2 : 4)) return 0;
+    if (B > 16) return blocks <= c->sm_count;
+    if (2 * blocks > c->sm_count) return 0;
+    const int tc = tc_slices(c, blocks, groups), mma = mma_slices(c, blocks, groups);
+    if (groups >= (B > 12 ? 64 : 48) && mma >= 2 * tc && blocks < clusters_at_once(c, LBK_gemm_int4_mma_b16, mma, 256, 4 * 16 * 320, 2, &c->mma_clusters[mma]) - (B > 12)) return 0;
+    if (groups >= 112 && mma >= 4 * tc && 3 * blocks * tc < 2 * c->sm_count) return 0;
+    return 1;
 }
 
 LB_API int lb_gemm_int4(lb_ctx* c, uint64_t qweight, uint64_t scales, uint64_t qzeros, uint64_t x, uint64_t y, int K, int N,
@@ -251,11 +283,7 @@ LB_API int lb_gemm_int4(lb_ctx* c, uint64_t qweight, uint64_t scales, uint64_t q
         if (lb_gemv_int4(c, qweight, scales, qzeros, x, y, K, N, flags & LB_GEMV_Y_F32) == LB_OK) return LB_OK; /* else: the batched kernel */
     const int blocks = (N + 127) / 128, groups = K / 128;
     void* params[] = {&p};
-    /* up to 32 tokens no weight is rounded: gemm_int4_tc_exact16 / 32 or the mma.sync kernels, the faster one.  us, mma.sync / tcgen05, at 12 tokens:
-     * 17408 -> 5120 34.4 / 27.1, 6144 -> 5120 17.8 / 12.6, 1024 -> 1024 6.9 / 5.3 (matrices that are split along K), 5120 -> 17408 23.9 / 24.5,
-     * 5120 -> 34816 39.1 / 49.0 (whole columns: two CTAs per SM against one); at 32 tokens 46.9 / 31.3, 24.5 / 14.5, 11.3 / 6.3, 34.6 / 28.2, 54.7 / 57;
-     * at 8 tokens 28.8 / 27.8, 14.4 / 13.0, 5.6 / 5.4, 20.0 / 24.4, 32.6 / 48.6 */
-    const int exact = B > 8 && B <= 32 && !(flags & (LB_GEMM_MMA_SYNC | LB_GEMM_TCGEN05)) && (B > 16 ? blocks : 2 * blocks) <= c->sm_count;
+    const int exact = B > 8 && B <= 32 && !(flags & (LB_GEMM_MMA_SYNC | LB_GEMM_TCGEN05)) && exact_on_tc(c, B, blocks, groups);
     if (exact || (B > 32 && !(flags & LB_GEMM_MMA_SYNC)) || (flags & LB_GEMM_TCGEN05)) {
         const int nt = B > 128 ? 256 : B > 64 ? 128 : B > 32 ? 64 : B > 16 ? 32 : 16;
         const unsigned smem = nt > 128 ? (unsigned)(LB_TC_X_HALVES * nt * 128) : (unsigned)((nt > 64 ? 6 : 7) * nt * 256); /* activation stages; the partial tile [nt][132] fp32 fits over them */
@@ -269,18 +297,14 @@ LB_API int lb_gemm_int4(lb_ctx* c, uint64_t qweight, uint64_t scales, uint64_t q
                                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                                              CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE));
         memcpy(p.tmap_x, &tm, sizeof tm);
-        int ksplit = c->sm_count / blocks;
-        if (ksplit > 8) ksplit = 8;
-        while (ksplit > 1 && (groups / ksplit < 4 || tc_clusters(c, ksplit) < blocks)) ksplit--;
-        if (ksplit < 1) ksplit = 1;
+        const int ksplit = tc_slices(c, blocks, groups);
         return lb_launch_cluster(c, exact ? (nt > 16 ? LBK_gemm_int4_tc_exact32 : LBK_gemm_int4_tc_exact16) : nt > 128 ? LBK_gemm_int4_tc_256 : LBK_gemm_int4_tc, (unsigned)blocks, (unsigned)ksplit, 1,
                                  exact ? (nt > 16 ? LB_TC_EXACT32_THREADS : LB_TC_EXACT16_THREADS) : LB_TC_THREADS, smem, params, 1, (unsigned)ksplit);
     }
     const int rows = B > 32 ? 64 : B > 16 ? 32 : B > 8 ? 16 : 8; /* token rows the CTA stages */
     const int kernel = B > 32 ? LBK_gemm_int4_mma_b64 : B > 16 ? LBK_gemm_int4_mma_b32 : B > 8 ? LBK_gemm_int4_mma_b16 : LBK_gemm_int4_mma_b8;
     const unsigned smem = (unsigned)((B > 16 ? 3 : 4) * rows * 320); /* activation ring (the partial tile reuses it) */
-    int ksplit = 1;
-    while (ksplit < 8 && blocks * ksplit < c->sm_count * 3 / 2 && groups / (ksplit * 2) >= 4) ksplit *= 2;
+    const int ksplit = mma_slices(c, blocks, groups);
     return lb_launch_cluster(c, kernel, (unsigned)blocks, (unsigned)ksplit, 1, 256, smem, params, 1, (unsigned)ksplit);
 }
 

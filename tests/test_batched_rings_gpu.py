@@ -48,3 +48,27 @@ def test_rings(ctx, lb, groups, N, zeros, f32):
     for d in d_w:
         if d:
             d.free()
+
+
+@pytest.mark.parametrize("K,N,B,tc", [
+    (512, 1024, 16, False), (640, 1024, 16, True), (256, 1024, 17, False), (384, 1024, 17, True),                # short columns
+    (8192, 7168, 12, False), (8192, 8832, 16, False), (8192, 9216, 9, True), (5120, 7168, 12, True),             # twice the slices, and all of them at once
+    (14336, 5888, 12, False), (11008, 5888, 12, True),                                                           # four times, and idle SMs
+    (1024, 9472, 16, True), (1024, 9600, 16, False), (1024, 9600, 17, True), (1024, 18944, 32, True), (1024, 18960, 32, False)])
+def test_which_kernel(ctx, lb, K, N, B, tc):
+    """9 to 32 tokens run on tensor memory where that is the faster way (148 SMs); both ways are exact, so their results differ in the last bits only"""
+    if ctx.sm_count != 148:
+        pytest.skip("the sizes are those of 148 SMs")
+    qw, sc, qz, _ = gptq_case(K, N, seed=K + N)
+    d_w, d_x = [ctx.to_device(a) for a in (qw, sc, qz)], ctx.to_device(lb_mod.fill_normal(B * K, N, 42, dtype="f16"))
+    got = []
+    for flag in (0, lb.GEMM_MMA_SYNC):
+        d_y = ctx.to_device(np.full(B * N, np.nan, dtype=np.float32))
+        ctx.gemm_int4(*d_w, d_x, d_y, K, N, B, lb.GEMV_Y_F32 | flag)
+        got.append(d_y.download(np.float32, B * N))
+        d_y.free()
+    assert ctx.device_status() == 0 and np.isfinite(got[0]).all()
+    assert np.array_equal(*got) != tc
+    assert np.linalg.norm(got[0] - got[1]) <= 2 * 1.7e-5 * np.linalg.norm(got[1])
+    for d in (*d_w, d_x):
+        d.free()
