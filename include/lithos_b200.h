@@ -76,6 +76,9 @@ void lb_set_chain_reserve(lb_ctx* ctx, int bytes);
  * as tagged 8-byte words that the consumer's loads wait on, and no grid barrier separates the two; off: a grid barrier
  * between every pair of entries.  Same results either way (the words carry the same fp32 / fp16 values). */
 void lb_set_chain_mailbox(lb_ctx* ctx, int on);
+/* which products of a bf16 prompt chunk run on pairs of CTAs: 1 (default) those that are faster so, 0 none, 2 all of them in tiles of 256 tokens
+ * (cross-checks: the results are the same bits).  Returns how many did since the last call. */
+uint64_t lb_set_product_pairs(lb_ctx* ctx, int mode);
 /* Profiling hook: while buf != 0, every persistent-chain launch made (or captured) afterwards writes, for each SM and
  * chain entry, eight stamps of the SM's thread 0 into buf as u64 [SMs][LB_GEMV_CHAIN_MAX][8]: [0] %globaltimer (ns) when
  * the entry is reached, then the SM's cycle counter at [1] entry reached, [2] grid barrier left, [3] input vector arrived,

@@ -112,6 +112,7 @@ def lib() -> C.CDLL:
     sig("lb_set_chain_reserve", None, vp, i32)
     sig("lb_set_chain_timeline", None, vp, u64)
     sig("lb_set_chain_mailbox", None, vp, i32)
+    sig("lb_set_product_pairs", C.c_uint64, vp, i32)
     sig("lb_gemv_packed_copy", u64, vp, u64, i32, i32, i32)
     sig("lb_gemv_pack_version", i32)
     sig("lb_gptq_dequant", i32, vp, u64, u64, u64, u64, i32, i32)
@@ -309,6 +310,10 @@ class Context:
         """hand vectors between consecutive GEMVs of a chain through tagged words (default) or through a grid barrier"""
         lib().lb_set_chain_mailbox(self.h, 1 if on else 0)
 
+    def set_product_pairs(self, mode: int) -> int:
+        """Products of a bf16 prompt chunk on CTA pairs: 1 (default) where that is faster, 0 never, 2 always; how many ran so since the last call."""
+        return int(lib().lb_set_product_pairs(self.h, mode))
+
     def set_pdl(self, on: bool):
         lib().lb_set_pdl(self.h, 1 if on else 0)
 
@@ -370,7 +375,7 @@ class Context:
                                             _ptr(x), _ptr(y), K, N, flags, 1 if weights_resident else 0))
 
     def gemm_int4(self, qweight, scales, qzeros, x, y, K, N, B, flags=0):
-        """Y[B,N] = X[B,K] W for up to 64 tokens; the weights are read once for the whole batch."""
+        """Y[B,N] = X[B,K] W for up to 256 tokens; the weights are read once for the whole batch."""
         self._check(lib().lb_gemm_int4(self.h, qweight.ptr, scales.ptr, qzeros.ptr if qzeros else 0, x.ptr, y.ptr, K, N, B, flags))
 
     def gptq_dequant(self, qweight, scales, qzeros, w_out, K, N):

@@ -208,6 +208,7 @@ LB_API int lb_init_images(int device, const char* kernel_dir, const char* images
     LB_CU(c, lb_drv.MemAlloc(&c->chain_mail, (size_t)LB_CHAIN_MAX_OPS * LB_CHAIN_MAIL_WORDS * 8));
     LB_CU(c, lb_drv.MemsetD8Async(c->chain_mail, 0, (size_t)LB_CHAIN_MAX_OPS * LB_CHAIN_MAIL_WORDS * 8, c->stream));
     c->chain_mailbox = 1;
+    c->product_pairs = 1;
     LB_CU(c, lb_drv.MemAlloc(&c->dev_status, 256));
     LB_CU(c, lb_drv.MemsetD8Async(c->dev_status, 0, 256, c->stream));
     c->flush_bytes = (size_t)256 << 20;
@@ -246,6 +247,13 @@ LB_API void lb_launch_count_reset(lb_ctx* c) { if (c) c->launches = 0; }
 LB_API void lb_set_pdl(lb_ctx* c, int on) { if (c) c->pdl = on ? 1 : 0; }
 LB_API void lb_set_chain_timeline(lb_ctx* c, uint64_t buf) { if (c) c->chain_timeline = (CUdeviceptr)buf; }
 LB_API void lb_set_chain_mailbox(lb_ctx* c, int on) { if (c) c->chain_mailbox = on ? 1 : 0; }
+LB_API uint64_t lb_set_product_pairs(lb_ctx* c, int mode) {
+    if (!c) return 0;
+    const uint64_t n = c->n_product_pairs;
+    c->n_product_pairs = 0;
+    if (mode >= 0 && mode <= 2) c->product_pairs = mode;
+    return n;
+}
 LB_API void lb_set_chain_reserve(lb_ctx* c, int bytes) { if (c && bytes >= 0 && bytes <= 128 * 1024) c->chain_reserve = bytes; }
 
 LB_API int lb_device_status(lb_ctx* c, uint32_t* out) {

@@ -552,6 +552,7 @@ static int launch_products(lb_model* m, const st_prod* pr, int n, int T) {
         p.head[i] = pr[i].head; p.head_p[i] = pr[i].head_p;
     }
     product_cost(c, p.tiles[0] + p.tiles[1], T, &p.NT);
+    if (c->product_pairs == 2) p.NT = 256;
     p.t_tiles = (T + p.NT - 1) / p.NT;
     void* params[] = {&p};
     if (S->esz == 4)
@@ -560,7 +561,9 @@ static int launch_products(lb_model* m, const st_prod* pr, int n, int T) {
      * higher (us, single / pair, 1024 tokens: 30720 rows of 4096 203 / 196, 4096 rows of 16384 113 / 108, 2048 rows of 8192, 2048 tokens, 65 / 64), but pairs
      * start about a microsecond later (2048 rows of 4096, 2048 tokens, 41.4 / 43) */
     const int tiles = (p.tiles[0] + p.tiles[1]) * p.t_tiles, tiles2 = (pair_tiles(&p, 0) + pair_tiles(&p, 1)) * p.t_tiles, slots2 = c->sm_count / 2;
-    const int waves2 = (tiles2 + slots2 - 1) / slots2, pair = p.NT == 256 && waves2 <= (tiles + c->sm_count - 1) / c->sm_count && waves2 * p.K >= 8192;
+    const int waves2 = (tiles2 + slots2 - 1) / slots2;
+    const int pair = c->product_pairs == 2 || (c->product_pairs && p.NT == 256 && waves2 <= (tiles + c->sm_count - 1) / c->sm_count && waves2 * p.K >= 8192);
+    c->n_product_pairs += (uint64_t)pair;
     for (int i = 0; i < n; i++) {
         CUtensorMap tm;
         memcpy(p.tmap_w[i], &pr[i].w->tmap, sizeof tm);
