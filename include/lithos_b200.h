@@ -197,16 +197,20 @@ int lb_gemv_chain_supports(lb_ctx* ctx, int K, int N, int swiglu);
  * buffers as lb_gemv_int4 (read once for the whole batch), x fp16 [B,K] row-major, y fp32 [B,N]
  * (flags = LB_GEMV_Y_F32) or fp16 [B,N] (flags = 0).  K % 128 == 0, N % 16 == 0.
  * One token is handed to the GEMV kernel of lb_gemv_int4.
- * 33..256 tokens run on the 5th-generation tensor cores (tcgen05.mma, accumulators in tensor memory):
- * the weights are dequantised to fp16 - (q - z) * s, q - z exact, one fp16 rounding for the scale -
- * and handed to the tensor cores through tensor memory (129..256 tokens: one
- * product of 128 columns x 256 tokens per k step, the weights converted once for all of them).  Up to 32 tokens use mma.sync (faster there, measured):
- * q - z stays exact and the group scale multiplies the group's fp32 sum, so row b of Y equals
- * lb_gemv_int4 on row b of X to fp32 rounding.  LB_GEMM_TCGEN05 forces the tensor-memory kernel for
- * 9 tokens or more, LB_GEMM_MMA_SYNC the mma.sync kernels for every size up to 64 tokens (cross-checks).
+ * 2..32 tokens round no weight: q - z stays exact and the group scale multiplies the group's fp32 sum, so row b of Y
+ * equals lb_gemv_int4 on row b of X to fp32 rounding.  2..8 tokens run on mma.sync, 9..32 on mma.sync or on the
+ * 5th-generation tensor cores (tcgen05.mma, accumulators in tensor memory), whichever is faster for K, N and B.
+ * 33..256 tokens run on tcgen05 with the weights dequantised to fp16 - (q - z) * s, q - z exact, one fp16 rounding for
+ * the scale - and handed to the tensor cores through tensor memory (129..256 tokens: one product of 128 columns x 256
+ * tokens per k step, the weights converted once for all of them).
+ * A row's bits do not depend on its place or on the rows that travel with it, but on the kernel, and so on how many rows
+ * there are: they are the same within 2..8 tokens and the sizes of 9..32 that run on mma.sync, within the sizes of 9..32
+ * that run on tcgen05, and within 33..256.
+ * LB_GEMM_MMA_SYNC forces the mma.sync kernels for every size up to 64 tokens (the same bits up to 32),
+ * LB_GEMM_TCGEN05 the kernel that rounds the weights to fp16 for 9 tokens or more (the same bits from 9 to 256).
  * Overwrites y.  x and y must not overlap. */
 #define LB_GEMM_MMA_SYNC (1 << 4) /* flags: use the mma.sync kernels for every batch size */
-#define LB_GEMM_TCGEN05 (1 << 5)  /* flags: use the tcgen05 kernel (B >= 9) */
+#define LB_GEMM_TCGEN05 (1 << 5)  /* flags: use the tcgen05 kernel with fp16 weights (B >= 9) */
 #define LB_GEMM_MAX_BATCH 256
 int lb_gemm_int4(lb_ctx* ctx, uint64_t qweight, uint64_t scales, uint64_t qzeros, uint64_t x_f16, uint64_t y, int K,
                  int N, int B, int flags);
@@ -223,7 +227,7 @@ int lb_dense_bf16_gemv(lb_ctx* ctx, uint64_t w_bf16, uint64_t x, uint64_t y_f32,
  * (inference/decay_gate.ls:28-57, inference/recur.ls:45-55).
  * state fp32 [HV,128,128] in place; q,k [n_steps,HK,128]; v, z, out [n_steps,HV,128];
  * g, beta fp32 [n_steps,HV]; z == 0 skips the silu(z) gate.  in_is_f32 selects fp32
- * (else bf16) q/k/v.  n_steps > 1 runs consecutive tokens with the state held on chip. */
+ * (else bf16) q/k/v.  n_steps > 1 runs consecutive tokens with the state held on chip and gives the bits of single steps. */
 int lb_deltanet_step(lb_ctx* ctx, uint64_t state, uint64_t q, uint64_t k, uint64_t v, uint64_t z, uint64_t g,
                      uint64_t beta, uint64_t out, int HV, int HK, int n_steps, int in_is_f32);
 int lb_decay_gate(lb_ctx* ctx, uint64_t a, uint64_t a_log, uint64_t dt_bias, uint64_t b, uint64_t g_out,

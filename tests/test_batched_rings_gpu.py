@@ -72,3 +72,38 @@ def test_which_kernel(ctx, lb, K, N, B, tc):
     assert np.linalg.norm(got[0] - got[1]) <= 2 * 1.7e-5 * np.linalg.norm(got[1])
     for d in (*d_w, d_x):
         d.free()
+
+
+def test_rows_and_their_batch(ctx, lb):
+    """what the header says of a row's bits: whoever travels with it they are the same within 2 to 8 tokens and mma.sync at 9 to 32, within 9 to 32 tokens
+    on tensor memory, and from 33 tokens on; and between the first two never more than rounding apart"""
+    K, N = 2048, 1168
+    qw, sc, qz, _ = gptq_case(K, N, seed=5)
+    d_w = [ctx.to_device(a) for a in (qw, sc, qz)]
+    X = lb_mod.fill_normal(256 * K, 6, 43, dtype="f16").reshape(256, K)
+
+    def run(rows, flag=0):
+        x = np.ascontiguousarray(X[rows])
+        d_x, d_y = ctx.to_device(x), ctx.to_device(np.full(len(x) * N, np.nan, dtype=np.float32))
+        ctx.gemm_int4(*d_w, d_x, d_y, K, N, len(x), lb.GEMV_Y_F32 | flag)
+        y = d_y.download(np.float32, len(x) * N).reshape(len(x), N)
+        d_x.free()
+        d_y.free()
+        return y
+
+    perm = np.random.default_rng(7).permutation(256)
+    mma, tc, many = run(range(32), lb.GEMM_MMA_SYNC), run(range(32)), run(range(256))
+    for B in (2, 5, 8):
+        assert np.array_equal(run(range(B)), mma[:B]), B
+    for B in (9, 12, 16, 17, 25):
+        assert np.array_equal(run(range(B)), tc[:B]), B
+        assert np.array_equal(run(range(B), lb.GEMM_MMA_SYNC), mma[:B]), B
+    for B in (33, 64, 65, 128, 129, 200):
+        assert np.array_equal(run(range(B)), many[:B]), B
+    for B in (9, 16, 17, 32):
+        assert np.array_equal(run(range(B), lb.GEMM_TCGEN05), many[:B]), B
+    assert np.array_equal(run(perm[perm < 32]), tc[perm[perm < 32]]) and np.array_equal(run(perm), many[perm])
+    assert np.linalg.norm(tc - mma) <= 2 * 1.7e-5 * np.linalg.norm(mma)
+    assert ctx.device_status() == 0
+    for d in d_w:
+        d.free()
