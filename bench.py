@@ -498,7 +498,7 @@ def bench_small_configs(ctx, lb):
     us = timed(ctx.end_capture(), NS)
     algo = 2 * HV * 128 * 128 * 4
     out["deltanet_step"] = {"workload": "config1: one Gated DeltaNet decode step, 48 value / 16 key heads, fp32 state [48,128,128]; 64 rotating states (201 MB > L2)",
-                            "kernel": "deltanet_step_bf16", "us_per_launch": round(us, 2), "algorithmic_bytes": algo, "GBps": round(algo / us / 1e3, 1),
+                            "kernel": "deltanet_one_bf16", "us_per_launch": round(us, 2), "algorithmic_bytes": algo, "GBps": round(algo / us / 1e3, 1),
                             "frac_of_measured_peak": round(algo / us / 1e3 / peak, 3)}
     for b in (st, q, k, v, g, beta, o):
         b.free()
@@ -1000,9 +1000,10 @@ def bench_timeline(args, rank, local, world, dist):
 
 def bench_batched(args, local):
     """--workload batched: the batched int4 projection sweep: the four projection shapes of the
-    model at batch 1 / 4 / 16 / 64, fp16 N(0,1) activations, each launch reading a weight set that is not in L2
-    (the sets of a shape rotate and together exceed the 126 MB L2).  One JSON line with one record per
-    (shape, batch): microseconds per launch and algorithmic GB/s (weights + scales + zero-points + X + Y)."""
+    model, fp16 N(0,1) activations, each launch reading a weight set that is not in L2 (the sets of a shape rotate
+    and together exceed the 126 MB L2).  One JSON line with one record per (shape, batch, path): the call without a
+    flag (default) and the kernels that a flag forces; microseconds per launch and algorithmic GB/s (weights + scales
+    + zero-points + X + Y)."""
     import lithos_b200 as lb
     ctx = lb.Context(local)
     peak, which = measured_hbm_peak()
@@ -1022,7 +1023,19 @@ def bench_batched(args, local):
         wbytes = K // 8 * N * 4 + K // 128 * N * 2 + K // 128 * (N // 8) * 4
         d_x = ctx.to_device(lb.fill_normal(max(batches + [128]) * K, 300, 4, dtype="f16"))
         d_y = ctx.alloc(max(batches + [128]) * N * 4)
-        for B, flag in [(B, f) for B in batches for f in ((lb.GEMM_TCGEN05,) if B > 64 else (lb.GEMM_TCGEN05, lb.GEMM_MMA_SYNC) if B > 8 else (0, lb.GEMM_MMA_SYNC) if B == 1 else (0,))]:
+
+        def bits(B, flag):
+            w = dev[0]
+            ctx.gemm_int4(w[0], w[1], w[2], d_x, d_y, K, N, B, lb.GEMV_Y_F32 | flag)
+            return d_y.download(np.uint32, B * N)
+
+        for B, flag in [(B, f) for B in batches for f in ((0, lb.GEMM_MMA_SYNC) if B == 1 else (0,) if B <= 8 or B > 64 else (0, lb.GEMM_TCGEN05, lb.GEMM_MMA_SYNC))]:
+            if flag or B == 1:
+                path = "gemv_int4" if not flag else "gemm_int4_tc" if flag == lb.GEMM_TCGEN05 else "gemm_int4_mma"
+            elif B <= 8 or (B <= 32 and np.array_equal(bits(B, 0), bits(B, lb.GEMM_MMA_SYNC))):
+                path = "gemm_int4_mma"
+            else:  # up to 32 tokens the two ways differ in the last bits
+                path = "gemm_int4_tc_exact%d" % (16 if B <= 16 else 32) if B <= 32 else "gemm_int4_tc" if B <= 128 else "gemm_int4_tc_256"
             ctx.begin_capture()
             for j in range(reps):
                 w = dev[j % sets]
@@ -1037,7 +1050,7 @@ def bench_batched(args, local):
                 graph.launch()
             us = ctx.timer_stop() * 1e3 / (n * reps)
             algo = wbytes + B * K * 2 + B * N * 4
-            sweep.append({"shape": name, "K": K, "N": N, "batch": B, "path": "tcgen05" if flag == lb.GEMM_TCGEN05 else "mma.sync" if (B > 1 or flag) else "gemv", "default": (flag == lb.GEMM_TCGEN05) == (B > 32) if B > 8 else flag == 0,
+            sweep.append({"shape": name, "K": K, "N": N, "batch": B, "path": path, "default": flag == 0,
                           "us": round(us, 2), "GBps": round(algo / us / 1e3, 1),
                           "frac_of_hbm_peak": round(algo / us / 1e3 / peak, 3), "TFLOPs": round(2.0 * B * K * N / us / 1e6, 1)})
             graph.destroy()
@@ -1050,7 +1063,7 @@ def bench_batched(args, local):
     ctx.close()
     return {"metric": "batched int4 projection sweep (config 4)", "unit": "us per launch", "n_gpus": 1, "data": "synthetic",
             "higher_is_better": False, "dtype": "int4 weights, fp16 activations, fp32 accumulation", "peak": peak, "peak_source": which,
-            "kernels": "gemm_int4_tc, gemm_int4_tc_256, gemm_int4_tc_exact16/32 (tcgen05.mma 128 x NT x 16, accumulator and converted weights in TMEM), gemm_int4_mma_b8/b16/b32/b64 (mma.sync m16n8k16)", "l2": "weight sets of a shape rotate, together > L2", "sweep": sweep}
+            "kernels": "gemm_int4_tc, gemm_int4_tc_256, gemm_int4_tc_exact16/32 (tcgen05.mma 128 x NT x 16, accumulator and converted weights in TMEM), gemm_int4_mma_b8/b16/b32/b64 (mma.sync m16n8k16), gemv_int4", "l2": "weight sets of a shape rotate, together > L2", "sweep": sweep}
 
 
 def reference_decode(args, rank):
