@@ -195,7 +195,8 @@ int lb_gemv_chain(lb_ctx* ctx, const lb_gemv_op* ops, int n_ops);
 int lb_gemv_chain_supports(lb_ctx* ctx, int K, int N, int swiglu);
 /* Batched projection: Y[B,N] = X[B,K] W for B = 1..LB_GEMM_MAX_BATCH tokens, W in the same three GPTQ
  * buffers as lb_gemv_int4 (read once for the whole batch), x fp16 [B,K] row-major, y fp32 [B,N]
- * (flags = LB_GEMV_Y_F32) or fp16 [B,N] (flags = 0).  K % 128 == 0, N % 16 == 0.
+ * (flags = LB_GEMV_Y_F32) or fp16 [B,N] (flags = 0).  K % 128 == 0, N % 16 == 0, x 16-byte aligned (LB_GEMM_MMA_SYNC
+ * also wants qweight 8-byte and scales 4-byte aligned).
  * One token is handed to the GEMV kernel of lb_gemv_int4.
  * 2..32 tokens round no weight: q - z stays exact and the group scale multiplies the group's fp32 sum, so row b of Y
  * equals lb_gemv_int4 on row b of X to fp32 rounding.  2..8 tokens run on mma.sync, 9..32 on mma.sync or on the

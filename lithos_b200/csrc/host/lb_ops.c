@@ -283,11 +283,13 @@ LB_API int lb_gemm_int4(lb_ctx* c, uint64_t qweight, uint64_t scales, uint64_t q
         if (lb_gemv_int4(c, qweight, scales, qzeros, x, y, K, N, flags & LB_GEMV_Y_F32) == LB_OK) return LB_OK; /* else: the batched kernel */
     const int blocks = (N + 127) / 128, groups = K / 128;
     void* params[] = {&p};
-    const int exact = B > 8 && B <= 32 && !(flags & (LB_GEMM_MMA_SYNC | LB_GEMM_TCGEN05)) && exact_on_tc(c, B, blocks, groups);
+    if (x & 15) return lb_fail(c, LB_ERR_INVALID, "lb_gemm_int4: x must be 16-byte aligned");
+    const int mma_ok = ((qweight & 7) | (scales & 3)) == 0; /* the mma.sync kernels load the words and scales of two columns at once */
+    if ((flags & LB_GEMM_MMA_SYNC) && !mma_ok) return lb_fail(c, LB_ERR_INVALID, "lb_gemm_int4: LB_GEMM_MMA_SYNC wants qweight 8-byte and scales 4-byte aligned");
+    const int exact = B <= 32 && !(flags & (LB_GEMM_MMA_SYNC | LB_GEMM_TCGEN05)) && (!mma_ok || (B > 8 && exact_on_tc(c, B, blocks, groups)));
     if (exact || (B > 32 && !(flags & LB_GEMM_MMA_SYNC)) || (flags & LB_GEMM_TCGEN05)) {
         const int nt = B > 128 ? 256 : B > 64 ? 128 : B > 32 ? 64 : B > 16 ? 32 : 16;
         const unsigned smem = nt > 128 ? (unsigned)(LB_TC_X_HALVES * nt * 128) : (unsigned)((nt > 64 ? 6 : 7) * nt * 256); /* activation stages; the partial tile [nt][132] fp32 fits over them */
-        if (x & 15) return lb_fail(c, LB_ERR_INVALID, "lb_gemm_int4: x must be 16-byte aligned");
         CUtensorMap tm; /* X [B, K] fp16, box = 64 k (128 bytes) x NT tokens, laid down with the 128-byte swizzle */
         cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)B};
         cuuint64_t strides[1] = {(cuuint64_t)K * 2};

@@ -18,8 +18,8 @@
 // What bound it before was the issuing thread, not the conversion: its K-group took 0.85 us whatever the tokens, also with loads, conversion and
 // stores taken out.  Its role is now entered by elect.sync (37.3 -> 26.8 us, 5120 -> 17408 at 16 tokens), its warp's other lanes rest instead of
 // polling beside it (-> 22.4), waits off its path are suspended ones and it waits for one barrier per K-group (-> 19.8).
-// Now, us at 48 / 100 / 256 tokens, before -> after: 5120 -> 17408 36.6 -> 20.3, 40.9 -> 23.0, 48.3 -> 39.1; 17408 -> 5120 42.7 -> 23.3, 48.2 -> 25.1,
-// 57.8 -> 42.1.  Up to 128 tokens the issuing thread (about 750 cycles per K-group) and the conversion (1100 cycles of a set, 4 sets) bound it; at 256 the
+// Now, us at 48 / 100 / 256 tokens, before -> after: 5120 -> 17408 36.6 -> 20.3, 40.9 -> 22.9, 48.3 -> 41.8; 17408 -> 5120 42.7 -> 23.2, 48.2 -> 25.0,
+// 57.8 -> 46.5.  Up to 128 tokens the issuing thread (about 750 cycles per K-group) and the conversion (1100 cycles of a set, 4 sets) bound it; at 256 the
 // activations' trip from L2 (64 KB per K-group and SM, 1024 cycles at 64 B per cycle) and the products (1024 cycles).
 // EXACT (up to 32 tokens): the weights go in as q - z, exact; every K-group has an accumulator of its own (four in turn), and
 // four more warps (a thread per column) read it and add scale * sum in fp32, so no weight is ever rounded.
@@ -415,7 +415,7 @@ extern "C" __global__ void __launch_bounds__(LB_TC_THREADS, 1) gemm_int4_tc_256(
     extern __shared__ __align__(1024) unsigned char tc_smem[];
     gemm_int4_tc_body<0, 4, true>(p, tc_smem);
 }
-extern "C" __global__ void __launch_bounds__(LB_TC_EXACT16_THREADS, 1) gemm_int4_tc_exact16(const __grid_constant__ lb_bgemm_params p) { // up to 16 tokens
+extern "C" __global__ void __launch_bounds__(LB_TC_EXACT16_THREADS, 1) gemm_int4_tc_exact16(const __grid_constant__ lb_bgemm_params p) { // 1..16 tokens
     extern __shared__ __align__(1024) unsigned char tc_smem[];
     gemm_int4_tc_body<16, 3, false>(p, tc_smem);
 }

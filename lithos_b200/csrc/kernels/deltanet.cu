@@ -21,9 +21,9 @@
 // step needs nothing from another warp: both sums over the rows end in three shuffles, and what the warps of a CTA share, the operands of
 // DN_RUN tokens in fp32, costs one block barrier per DN_RUN tokens.  A thread loads its piece of the run after next into registers and
 // stores it a run later, so the chain of a step (dot, three shuffles, update) meets no trip to L2.  The read-outs of four tokens are summed
-// together (seven shuffles instead of twelve), in the order of a single one: the same bits for one step and for many.
-// 48 heads, bf16 (us before -> after; before: a column's rows in four lanes, 16 reads of k and q and a barrier a token): 3.15 -> 3.20 at one
-// step, 5.0 -> 4.3 at 4, 38 -> 24 at 64, 144 -> 87 at 256.  Two warps per scheduler now take 620 cycles a token, of which 256 are the
+// together (seven shuffles instead of 24), in the order of a single one: the same bits for one step and for many.
+// 48 heads, bf16 (us before -> after; before: a column's rows in four lanes, 16 reads of k and q and a barrier a token): 5.0 -> 4.2 at 4 steps,
+// 38 -> 24 at 64, 144 -> 86 at 256.  Two warps per scheduler now take 620 cycles a token, of which 256 are the
 // multiply-adds' and 440 one warp's chain; reading the next token's k ahead moved it by 3 % either way.
 #define DN_RUN 8
 template <typename T> struct dn_in; // element type of q, k, v: 16 bytes of them, and how they go to shared memory as fp32

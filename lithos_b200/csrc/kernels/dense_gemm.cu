@@ -143,75 +143,75 @@ __device__ __forceinline__ void gemm_bf16_body(const lb_dgemm_params& p, unsigne
     if (warp == 0) {
         // ---------------- operands ----------------
         if (tc_elect()) {
-        int s = 0, issued = 0;
-        uint32_t ph = 0;
-        bool ok = true;
-        for (int tile = tile0; tile < n_tiles && ok; tile += step) {
-            const dg_tile d = dg_find<ROWS>(p, tile);
-            for (int k = 0; k < ksteps; ++k) {
-                if (issued >= S && !tc_wait(&bar_empty[s], ph ^ 1u)) {
-                    ok = false;
-                    if (p.status) atomicExch(p.status, DG_FAIL_EMPTY);
-                    break;
+            int s = 0, issued = 0;
+            uint32_t ph = 0;
+            bool ok = true;
+            for (int tile = tile0; tile < n_tiles && ok; tile += step) {
+                const dg_tile d = dg_find<ROWS>(p, tile);
+                for (int k = 0; k < ksteps; ++k) {
+                    if (issued >= S && !tc_wait(&bar_empty[s], ph ^ 1u)) {
+                        ok = false;
+                        if (p.status) atomicExch(p.status, DG_FAIL_EMPTY);
+                        break;
+                    }
+                    if (rank == 0) mbar_arrive_expect_tx(&bar_full[s], PAIR ? 2 * stage_bytes : stage_bytes);
+                    const uint32_t dst = smem_u32(dg_sm) + (uint32_t)s * stage_bytes;
+                    if (PAIR) { // a CTA brings its 128 weight rows and its half of the tokens; the first one's barrier counts all of it
+                        const uint32_t full = tc2_leader(&bar_full[s]);
+                        dg_tma2(dst, p.tmap_w[d.m], k * LB_DG_KB, d.row + rank * LB_DG_ROWS, full);
+                        dg_tma2(dst + a_bytes, p.tmap_x[d.m], k * LB_DG_KB, d.tok + rank * (NT / 2), full);
+                    } else {
+                        dg_tma(dst, p.tmap_w[d.m], k * LB_DG_KB, d.row, &bar_full[s]);
+                        dg_tma(dst + a_bytes, p.tmap_x[d.m], k * LB_DG_KB, d.tok, &bar_full[s]);
+                    }
+                    ++issued;
+                    if (++s == S) { s = 0; ph ^= 1u; }
                 }
-                if (rank == 0) mbar_arrive_expect_tx(&bar_full[s], PAIR ? 2 * stage_bytes : stage_bytes);
-                const uint32_t dst = smem_u32(dg_sm) + (uint32_t)s * stage_bytes;
-                if (PAIR) { // a CTA brings its 128 weight rows and its half of the tokens; the first one's barrier counts all of it
-                    const uint32_t full = tc2_leader(&bar_full[s]);
-                    dg_tma2(dst, p.tmap_w[d.m], k * LB_DG_KB, d.row + rank * LB_DG_ROWS, full);
-                    dg_tma2(dst + a_bytes, p.tmap_x[d.m], k * LB_DG_KB, d.tok + rank * (NT / 2), full);
-                } else {
-                    dg_tma(dst, p.tmap_w[d.m], k * LB_DG_KB, d.row, &bar_full[s]);
-                    dg_tma(dst + a_bytes, p.tmap_x[d.m], k * LB_DG_KB, d.tok, &bar_full[s]);
+            }
+            if (!ok && rank == 0) // nothing may still be on its way into this CTA's shared memory when it ends
+                for (int i = 0; i < S && i < issued; ++i) {
+                    if (--s < 0) { s = S - 1; ph ^= 1u; }
+                    tc_wait(&bar_full[s], ph);
                 }
-                ++issued;
-                if (++s == S) { s = 0; ph ^= 1u; }
-            }
-        }
-        if (!ok && rank == 0) // nothing may still be on its way into this CTA's shared memory when it ends
-            for (int i = 0; i < S && i < issued; ++i) {
-                if (--s < 0) { s = S - 1; ph ^= 1u; }
-                tc_wait(&bar_full[s], ph);
-            }
         }
         __syncwarp();
     } else if (warp == 1) {
         // ---------------- products ----------------
         if (rank == 0 && tc_elect()) {
-        const uint32_t idesc = tc_idesc_bf16(ROWS, (uint32_t)NT);
-        int s = 0, it = 0;
-        uint32_t ph = 0;
-        bool ok = true;
-        for (int tile = tile0; tile < n_tiles && ok; tile += step, ++it) {
-            const int b = it & 1;
-            if (it >= 2 && !(PAIR ? tc2_wait(&bar_free[b], (uint32_t)((it >> 1) - 1) & 1u) : tc_wait(&bar_free[b], (uint32_t)((it >> 1) - 1) & 1u))) { // the epilogue has read this accumulator
-                ok = false;
-                if (p.status) atomicExch(p.status, DG_FAIL_ACC);
-                break;
-            }
-            tc_fence_after();
-            const uint32_t d = tmem + (uint32_t)(b * NT);
-            for (int k = 0; k < ksteps; ++k) {
-                if (!tc_wait(&bar_full[s], ph)) {
+            const uint32_t idesc = tc_idesc_bf16(ROWS, (uint32_t)NT);
+            int s = 0, it = 0;
+            uint32_t ph = 0;
+            bool ok = true;
+            for (int tile = tile0; tile < n_tiles && ok; tile += step, ++it) {
+                const int b = it & 1;
+                if (it >= 2 && !(PAIR ? tc2_wait(&bar_free[b], (uint32_t)((it >> 1) - 1) & 1u) : tc_wait(&bar_free[b], (uint32_t)((it >> 1) - 1) & 1u))) { // the epilogue has read this accumulator
                     ok = false;
-                    if (p.status) atomicExch(p.status, DG_FAIL_FULL);
+                    if (p.status) atomicExch(p.status, DG_FAIL_ACC);
                     break;
                 }
                 tc_fence_after();
-                const uint32_t base = smem_u32(dg_sm) + (uint32_t)s * stage_bytes;
-                const uint64_t ad = tc_smem_desc(base, 16, 1024), bd = tc_smem_desc(base + a_bytes, 16, 1024);
+                const uint32_t d = tmem + (uint32_t)(b * NT);
+                for (int k = 0; k < ksteps; ++k) {
+                    if (!tc_wait(&bar_full[s], ph)) {
+                        ok = false;
+                        if (p.status) atomicExch(p.status, DG_FAIL_FULL);
+                        break;
+                    }
+                    tc_fence_after();
+                    const uint32_t base = smem_u32(dg_sm) + (uint32_t)s * stage_bytes;
+                    const uint64_t ad = tc_smem_desc(base, 16, 1024), bd = tc_smem_desc(base + a_bytes, 16, 1024);
 #pragma unroll
-                for (int kk = 0; kk < LB_DG_KB / 16; ++kk) {
-                    if (PAIR) tc2_mma(d, ad + (uint64_t)(kk * 2), bd + (uint64_t)(kk * 2), idesc, (k > 0 || kk > 0) ? 1u : 0u);
-                    else tc_mma(d, ad + (uint64_t)(kk * 2), bd + (uint64_t)(kk * 2), idesc, (k > 0 || kk > 0) ? 1u : 0u);
+                    for (int kk = 0; kk < LB_DG_KB / 16; ++kk) {
+                        if (PAIR) tc2_mma(d, ad + (uint64_t)(kk * 2), bd + (uint64_t)(kk * 2), idesc, (k > 0 || kk > 0) ? 1u : 0u);
+                        else tc_mma(d, ad + (uint64_t)(kk * 2), bd + (uint64_t)(kk * 2), idesc, (k > 0 || kk > 0) ? 1u : 0u);
+                    }
+                    if (PAIR) tc2_commit(&bar_empty[s]);
+                    else tc_commit(&bar_empty[s]);
+                    if (++s == S) { s = 0; ph ^= 1u; }
                 }
-                if (PAIR) tc2_commit(&bar_empty[s]);
-                else tc_commit(&bar_empty[s]);
-                if (++s == S) { s = 0; ph ^= 1u; }
+                if (ok && PAIR) tc2_commit(&bar_acc[b]);
+                else if (ok) tc_commit(&bar_acc[b]);
             }
-            if (ok && PAIR) tc2_commit(&bar_acc[b]);
-            else if (ok) tc_commit(&bar_acc[b]);
-        }
         }
         __syncwarp();
     } else {
@@ -266,7 +266,6 @@ extern "C" __global__ void __launch_bounds__(LB_DG_THREADS, 1) gemm_bf16_tc_pair
     extern __shared__ __align__(1024) unsigned char dg_sm[];
     gemm_bf16_body<true>(p, dg_sm);
 }
-
 
 // ---- fp32 ----------------------------------------------------------------------------------------------------------
 #define SG_TN 64 // weight rows per tile

@@ -20,6 +20,11 @@ import lithos_b200 as lb_mod
 pytestmark = pytest.mark.gpu
 
 
+class View:
+    def __init__(self, b, off):
+        self.ptr = b.ptr + off
+
+
 @pytest.mark.parametrize("groups", [1, 3, 4, 5, 7, 8, 13, 36])
 @pytest.mark.parametrize("N", [48, 1168])
 @pytest.mark.parametrize("zeros", [True, False])
@@ -107,3 +112,32 @@ def test_rows_and_their_batch(ctx, lb):
     assert ctx.device_status() == 0
     for d in d_w:
         d.free()
+
+
+def test_alignment(ctx, lb):
+    """packed words and scales on their own boundaries only (the mma.sync kernels load two at once) are taken by the exact tcgen05 kernels at any size
+    up to 32 tokens, forced mma.sync refuses them, and so does every path an x beside a 16-byte boundary"""
+    for K, N, sizes in ((512, 1168, (1, 2, 8, 9, 16, 17, 32, 33, 200)), (256, 48, (2, 17))):
+        qw, sc, qz, _ = gptq_case(K, N, seed=N)
+        W = orc.gptq_dequant(qw, sc, qz, K, N).astype(np.float64)
+        X = lb_mod.fill_normal(256 * K, 8, 44, dtype="f16").reshape(256, K)
+        bufs = [ctx.to_device(np.concatenate([np.zeros(1, a.dtype), a.ravel()])) for a in (qw, sc)]
+        d_q, d_s = (View(b, a.itemsize) for b, a in zip(bufs, (qw, sc)))
+        d_z, d_y = ctx.to_device(qz), ctx.alloc(256 * N * 4)
+        for B in sizes:
+            d_x = ctx.to_device(np.concatenate([np.zeros(4, np.float16), X[:B].ravel()]))
+            for y32 in (lb.GEMV_Y_F32, 0):
+                with pytest.raises(lb_mod.LithosError):
+                    ctx.gemm_int4(d_q, d_s, d_z, View(d_x, 8), d_y, K, N, B, y32)
+            if B <= 64:
+                with pytest.raises(lb_mod.LithosError):
+                    ctx.gemm_int4(d_q, d_s, d_z, d_x, d_y, K, N, B, lb.GEMV_Y_F32 | lb.GEMM_MMA_SYNC)
+            d_x.free()
+            d_x = ctx.to_device(np.ascontiguousarray(X[:B]))
+            ctx.gemm_int4(d_q, d_s, d_z, d_x, d_y, K, N, B, lb.GEMV_Y_F32)
+            y, want = d_y.download(np.float32, B * N).reshape(B, N), X[:B].astype(np.float64) @ W
+            assert ctx.device_status() == 0
+            assert np.linalg.norm(y - want) <= (1.7e-5 if B <= 32 else 1e-3) * np.linalg.norm(want), B
+            d_x.free()
+        for b in (*bufs, d_z, d_y):
+            b.free()
