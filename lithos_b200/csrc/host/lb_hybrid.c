@@ -605,10 +605,10 @@ static void hybrid_destroy(lb_model* m) {
         layer_t* L = &m->L[l];
         q4_mat* q[] = {&L->w_in, &L->w_out, &L->w_gateup, &L->w_down};
         for (int i = 0; i < 4; i++) {
-            if (q[i]->qweight) lb_drv.MemFree(q[i]->qweight);
             if (q[i]->scales) lb_drv.MemFree(q[i]->scales);
             if (q[i]->qzeros) lb_drv.MemFree(q[i]->qzeros);
-            if (q[i]->packed) lb_drv.MemFree(q[i]->packed);
+            lb_free(m->c, q[i]->qweight); /* both through lb_free: lb_gemv_int4 must not find this pair for the next buffer at either address */
+            lb_free(m->c, q[i]->packed);
         }
         CUdeviceptr p[] = {L->input_norm, L->post_norm, L->proj_a, L->proj_b, L->a_log, L->dt_bias, L->conv_w, L->dn_norm,
                            L->dn_state, L->conv_ring, L->q_norm, L->k_norm, L->k_cache, L->v_cache, L->dn_params,

@@ -228,3 +228,17 @@ def test_gemv_int4_reads_the_packed_copy_once_there_is_one(ctx, lb, oracle):
     for b in d + [d_x, y0, y1, y2, y3]:
         b.free()
 
+
+
+def test_a_closed_model_leaves_no_packed_copies(ctx, lb):
+    """buffers at the addresses of a closed model's matrices are not taken for them: lb_gemv_int4 would read the freed packed copy (nothing is launched)"""
+    from lithos_b200 import model as M
+    for rank in (0, 1):
+        m = M.Model(ctx, M.tiny(max_ctx=16), rank, 2)       # a shard: its down projection is 1024 x 1024
+        m.fill_synthetic(5)
+        m.close()
+    bufs = [ctx.alloc(1024 // 8 * 1024 * 4) for _ in range(64)]
+    found = [b for b in bufs if ctx.gemv_packed_copy(b, 1024, 1024)]
+    for b in bufs:
+        b.free()
+    assert not found
