@@ -37,6 +37,7 @@
 
 __device__ __forceinline__ uint32_t tc_cluster_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
 __device__ __forceinline__ void tc_cluster_sync() {
+    __syncwarp(); // .aligned: the whole warp together, also behind code of some lanes only
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 __device__ __forceinline__ float4 tc_ld_cluster4(const float* local_ptr, uint32_t rank) { // 16-byte aligned
@@ -397,7 +398,6 @@ __device__ __forceinline__ void gemm_int4_tc_body(const lb_bgemm_params& p, unsi
                 }
             }
         }
-        __syncwarp();
         tc_cluster_sync(); // nobody leaves while a neighbour still reads its tile
     }
     __syncthreads();

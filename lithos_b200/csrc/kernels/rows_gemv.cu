@@ -13,6 +13,7 @@
 #include "params.h"
 
 __device__ __forceinline__ void rg_cluster_sync() {
+    __syncwarp(); // .aligned: the whole warp together, also behind code of some lanes only
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 __device__ __forceinline__ float2 rg_ld_cluster(const float* local_ptr, uint32_t rank) {

@@ -41,6 +41,7 @@ __device__ __forceinline__ void tc_commit(uint64_t* bar) { // the barrier fires 
 // ---- CTA pairs (cta_group::2): two CTAs of a cluster, M = 256 rows in the tensor memory of both, half of B in the shared memory of each -----------------
 __device__ __forceinline__ uint32_t tc2_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
 __device__ __forceinline__ void tc2_sync() { // both CTAs, all threads
+    __syncwarp(); // .aligned: the whole warp together, also behind code of some lanes only
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 __device__ __forceinline__ uint32_t tc2_leader(const void* p) { // the first CTA's copy of a shared variable, as a cluster address
