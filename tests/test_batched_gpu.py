@@ -2,8 +2,8 @@
 
 Row b of Y must equal the oracle's batch-1 GEMV of row b of X:
   max|y - y_ref| / max|y_ref| <= 1e-3 per row (the GEMV tolerance; the mma.sync kernels keep q - z exact up to
-  32 tokens and accumulate in fp32, observed error near 1e-6; the tcgen05 kernel, 9..64 tokens, and the 64-token
-  mma.sync variant multiply fp16-rounded weights, error near 2e-4), and must equal lb_gemv_int4 on the same row
+  32 tokens and accumulate in fp32, observed error near 1e-6; the tcgen05 kernel that LB_GEMM_TCGEN05 forces, 9..256
+  tokens, and the 64-token mma.sync variant multiply fp16-rounded weights, error near 2e-4), and must equal lb_gemv_int4 on the same row
   to the same tolerance.  Both paths are run at every size they accept (flags LB_GEMM_MMA_SYNC / LB_GEMM_TCGEN05).
   Results may not depend on the batch a row travels in (checked bit-exactly between batch sizes that use
   the same arithmetic).
