@@ -243,7 +243,7 @@ typedef struct {
     uint16_t* v_cache;
     float* out;           /* fp32 [HQ,256] */
     float* scratch;       /* split partials: [HKV][splits][G][(256 acc) + m + l] */
-    uint32_t* counters;   /* one per kv head, zero between launches */
+    uint32_t* counters;   /* zero between launches: one per kv head; attn_decode_mma: arrivals [kv], finished [8 + kv] */
     const int* pos_ptr;   /* when non-NULL the position is read from device memory (graph replay) */
     int32_t pos;          /* position of the new token; rows [0,pos] are attended */
     int32_t HQ, HKV;
@@ -256,8 +256,6 @@ typedef struct {
     float eps;
     double rope_freq[64]; /* theta^(-i/(rot_dims/2)), i < rot_dims/2 <= 64, computed on the host in double */
     uint32_t* status;     /* device status word for bounded waits (attn_decode_mma); may be NULL */
-    int32_t coop;         /* attn_decode_mma: the grid fits the SMs one CTA each, so the CTAs of a KV head may wait for each
-                             other and share the slice merge (counters[kv] arrivals, counters[8 + kv] finished) */
     int32_t max_ctx;      /* rows the caches hold (0 = not checked): a position outside [0, max_ctx) sets status
                              LB_DEV_POS_RANGE and the kernel returns without reading or writing a cache row */
 } lb_attn_params;
