@@ -202,8 +202,8 @@ int lb_gemv_chain_supports(lb_ctx* ctx, int K, int N, int swiglu);
  * equals lb_gemv_int4 on row b of X to fp32 rounding.  2..8 tokens run on mma.sync, 9..32 on mma.sync or on the
  * 5th-generation tensor cores (tcgen05.mma, accumulators in tensor memory), whichever is faster for K, N and B.
  * 33..256 tokens run on tcgen05 with the weights dequantised to fp16 - (q - z) * s, q - z exact, one fp16 rounding for
- * the scale - and handed to the tensor cores through tensor memory (129..256 tokens: one product of 128 columns x 256
- * tokens per k step, the weights converted once for all of them).
+ * the scale - and handed to the tensor cores through tensor memory (one product of 128 columns x all tokens per k
+ * step, the weights converted once for all of them).
  * A row's bits do not depend on its place or on the rows that travel with it, but on the kernel, and so on how many rows
  * there are: they are the same within 2..8 tokens and the sizes of 9..32 that run on mma.sync, within the sizes of 9..32
  * that run on tcgen05, and within 33..256.

@@ -288,8 +288,8 @@ LB_API int lb_gemm_int4(lb_ctx* c, uint64_t qweight, uint64_t scales, uint64_t q
     if ((flags & LB_GEMM_MMA_SYNC) && !mma_ok) return lb_fail(c, LB_ERR_INVALID, "lb_gemm_int4: LB_GEMM_MMA_SYNC wants qweight 8-byte and scales 4-byte aligned");
     const int exact = B <= 32 && !(flags & (LB_GEMM_MMA_SYNC | LB_GEMM_TCGEN05)) && (!mma_ok || (B > 8 && exact_on_tc(c, B, blocks, groups)));
     if (exact || (B > 32 && !(flags & LB_GEMM_MMA_SYNC)) || (flags & LB_GEMM_TCGEN05)) {
-        const int nt = B > 128 ? 256 : B > 64 ? 128 : B > 32 ? 64 : B > 16 ? 32 : 16;
-        const unsigned smem = nt > 128 ? (unsigned)(LB_TC_X_HALVES * nt * 128) : (unsigned)((nt > 64 ? 6 : 7) * nt * 256); /* activation stages; the partial tile [nt][132] fp32 fits over them */
+        const int nt = exact ? (B > 16 ? 32 : 16) : LB_TC_NT(B), halves = nt > LB_TC_HALVES_FROM;
+        const unsigned smem = halves ? (unsigned)(LB_TC_X_HALVES * nt * 128) : (unsigned)((exact ? 7 : LB_TC_STAGES(nt)) * nt * 256); /* activation stages; the partial tile [nt][132] fp32 fits over them */
         CUtensorMap tm; /* X [B, K] fp16, box = 64 k (128 bytes) x NT tokens, laid down with the 128-byte swizzle */
         cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)B};
         cuuint64_t strides[1] = {(cuuint64_t)K * 2};
@@ -300,7 +300,7 @@ LB_API int lb_gemm_int4(lb_ctx* c, uint64_t qweight, uint64_t scales, uint64_t q
                                              CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE));
         memcpy(p.tmap_x, &tm, sizeof tm);
         const int ksplit = tc_slices(c, blocks, groups);
-        return lb_launch_cluster(c, exact ? (nt > 16 ? LBK_gemm_int4_tc_exact32 : LBK_gemm_int4_tc_exact16) : nt > 128 ? LBK_gemm_int4_tc_256 : LBK_gemm_int4_tc, (unsigned)blocks, (unsigned)ksplit, 1,
+        return lb_launch_cluster(c, exact ? (nt > 16 ? LBK_gemm_int4_tc_exact32 : LBK_gemm_int4_tc_exact16) : halves ? LBK_gemm_int4_tc_256 : LBK_gemm_int4_tc, (unsigned)blocks, (unsigned)ksplit, 1,
                                  exact ? (nt > 16 ? LB_TC_EXACT32_THREADS : LB_TC_EXACT16_THREADS) : LB_TC_THREADS, smem, params, 1, (unsigned)ksplit);
     }
     const int rows = B > 32 ? 64 : B > 16 ? 32 : B > 8 ? 16 : 8; /* token rows the CTA stages */

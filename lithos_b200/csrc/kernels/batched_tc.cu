@@ -20,7 +20,10 @@
 // polling beside it (-> 22.4), waits off its path are suspended ones and it waits for one barrier per K-group (-> 19.8).
 // Now, us at 48 / 100 / 256 tokens, before -> after: 5120 -> 17408 36.6 -> 20.3, 40.9 -> 22.9, 48.3 -> 41.8; 17408 -> 5120 42.7 -> 23.2, 48.2 -> 25.0,
 // 57.8 -> 46.5.  Up to 128 tokens the issuing thread (about 750 cycles per K-group) and the conversion (1100 cycles of a set, 4 sets) bound it; at 256 the
-// activations' trip from L2 (64 KB per K-group and SM, 1024 cycles at 64 B per cycle) and the products (1024 cycles).
+// activations' trip from L2 (64 KB per K-group and SM, 1024 cycles at 64 B per cycle) and the products (1104 cycles: 128 x N x 16 with A in tensor memory
+// takes about 10 + N / 2).  So a product carries no more tokens than there are, in steps of 16 (before: 64, 128 or 256), and up to 160 whole stages of
+// activations, one barrier a K-group.  us, before -> after: 5120 -> 17408 at 75 tokens 26.1 -> 24.6, 136 39.5 -> 29.9, 150 40.5 -> 31.9, 192 42.7 -> 36.6, 240
+// 45.6 -> 44.0; 17408 -> 5120 at 150 43.9 -> 34.3; 2048 -> 4096 at 150 11.4 -> 10.0.
 // EXACT (up to 32 tokens): the weights go in as q - z, exact; every K-group has an accumulator of its own (four in turn), and
 // four more warps (a thread per column) read it and add scale * sum in fp32, so no weight is ever rounded.
 // Epilogue: without a K split straight from tensor memory (or the EXACT sums in registers) to global memory, 32 neighbouring columns of a token
@@ -93,7 +96,7 @@ __device__ __forceinline__ void tc_store_y(const lb_bgemm_params& p, size_t o, f
 
 // SETS: converting sets of four warps (a set = the 128 columns); the exact kernels have fewer, their reading warps need the registers (spilling there cost
 // 20 %: 17408 -> 5120 at 32 tokens 38.2 us with three sets, 31.3 with two; at 16 tokens 31.0 with registers for 32 tokens, 27.1 with those for 16).
-// HALVES (129..256 tokens): a K-group of activations is 64 KB, so they have a ring of their own of 64-k halves, seven of which fit beside four weight stages.
+// HALVES (161..256 tokens): a K-group of activations is 64 KB, so they have a ring of their own of 64-k halves, seven of which fit beside four weight stages.
 template <int EXACT, int SETS, bool HALVES> // EXACT: 0, or the tokens the product carries (16, 32)
 __device__ __forceinline__ void gemm_int4_tc_body(const lb_bgemm_params& p, unsigned char* tc_smem) {
     __shared__ __align__(8) uint64_t bar_free[TC_STAGES]; // a stage's products are done (tcgen05.commit)
@@ -103,11 +106,11 @@ __device__ __forceinline__ void gemm_int4_tc_body(const lb_bgemm_params& p, unsi
     __shared__ __align__(8) uint64_t bar_done;
     __shared__ uint32_t tmem_base_slot;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int NT = EXACT ? EXACT : p.B > 128 ? 256 : p.B > 64 ? 128 : p.B > 32 ? 64 : p.B > 16 ? 32 : 16; // tokens the product carries (rows past B are zero)
+    const int NT = EXACT ? EXACT : LB_TC_NT(p.B); // tokens the product carries (rows past B are zero)
     const uint32_t a0 = EXACT ? TC_ACCS * 32u : NT > 64 ? (uint32_t)NT : 64u; // first column of the weight stages
     // Stages: what tensor memory and shared memory hold.  At least SETS: a set waits for the K-group `stages` back with the parity of an mbarrier, and with fewer
     // stages it could be two phases ahead of it.
-    const int stages = (int)((TC_TMEM_COLS - a0) / 64u); // 256 tokens 4, 128 tokens 6, fewer 7 (EXACT: 6)
+    const int stages = (int)((TC_TMEM_COLS - a0) / 64u); // LB_TC_STAGES: 256 tokens 4, 128 tokens 6, up to 64 7 (EXACT: 6)
     const uint32_t x_stage_bytes = (uint32_t)NT * 256u, x_half = (uint32_t)NT * 128u; // a 64-k half: NT rows of 128 bytes
     unsigned char* x_smem = tc_smem;                          // [stages][NT * 256], HALVES: [LB_TC_X_HALVES][NT * 128]
     float* pt = reinterpret_cast<float*>(tc_smem);            // [NT][TC_PSTRIDE], over the activation stages once the products are done
@@ -407,11 +410,11 @@ __device__ __forceinline__ void gemm_int4_tc_body(const lb_bgemm_params& p, unsi
     }
 }
 
-extern "C" __global__ void __launch_bounds__(LB_TC_THREADS, 1) gemm_int4_tc(const __grid_constant__ lb_bgemm_params p) { // 9..128 tokens
+extern "C" __global__ void __launch_bounds__(LB_TC_THREADS, 1) gemm_int4_tc(const __grid_constant__ lb_bgemm_params p) { // 9..160 tokens
     extern __shared__ __align__(1024) unsigned char tc_smem[];
     gemm_int4_tc_body<0, 4, false>(p, tc_smem);
 }
-extern "C" __global__ void __launch_bounds__(LB_TC_THREADS, 1) gemm_int4_tc_256(const __grid_constant__ lb_bgemm_params p) { // 129..256 tokens
+extern "C" __global__ void __launch_bounds__(LB_TC_THREADS, 1) gemm_int4_tc_256(const __grid_constant__ lb_bgemm_params p) { // 161..256 tokens
     extern __shared__ __align__(1024) unsigned char tc_smem[];
     gemm_int4_tc_body<0, 4, true>(p, tc_smem);
 }

@@ -142,7 +142,10 @@ typedef struct {
 #define LB_TC_THREADS 576       /* gemm_int4_tc, gemm_int4_tc_256: 16 converting warps, the issuing and the activation warp */
 #define LB_TC_EXACT16_THREADS 576 /* gemm_int4_tc_exact16: 12 converting warps, those two, and four warps that scale and add the K-groups' products */
 #define LB_TC_EXACT32_THREADS 448 /* gemm_int4_tc_exact32: 8 converting warps, so that the sums of 32 tokens stay in registers */
-#define LB_TC_X_HALVES 7        /* gemm_int4_tc_256: 64-k halves of a K-group's activations in shared memory (32 KB each) */
+#define LB_TC_NT(B) (((B) + 15) & ~15)  /* gemm_int4_tc, gemm_int4_tc_256: tokens a product carries */
+#define LB_TC_STAGES(nt) ((512 - ((nt) > 64 ? (nt) : 64)) / 64) /* weight stages of 64 columns beside the accumulator in tensor memory */
+#define LB_TC_HALVES_FROM 160           /* more tokens a product: gemm_int4_tc_256 (five whole stages of 160 tokens are 200 KB) */
+#define LB_TC_X_HALVES 7        /* gemm_int4_tc_256: 64-k halves of a K-group's activations in shared memory (32 KB each at 256 tokens) */
 typedef struct {
     /* gemm_int4_tc: CUtensorMap over X [B, K] fp16, box 64 k x NT tokens, 128-byte swizzle */
     unsigned char tmap_x[128] __attribute__((aligned(64)));
