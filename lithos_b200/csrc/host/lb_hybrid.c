@@ -686,11 +686,14 @@ static int hybrid_pf_layer(lb_model* m, pf_set* w, int l, int pos0, int T) {
         p.ld = ld; p.HQ = m->HQ; p.HKV = m->HKV; p.pos0 = pos0; p.T = T; p.rot_dims = cfg->rot_dims; p.eps = cfg->eps;
         for (int i = 0; i < cfg->rot_dims / 2; i++)
             p.rope_freq[i] = exp2(-log2((double)cfg->rope_theta) * (double)i / (double)(cfg->rot_dims / 2));
-        void* params[] = {&p};
+        p.status = (uint32_t*)c->dev_status;
+        lb_ac_maps maps;
+        const int kv_ld = m->HKV * 256;
+        LB_TRY(lb_ac_fill(c, &maps, L->k_cache, kv_ld, 0, 0, 0, L->v_cache, kv_ld, 256, pos0 + T));
+        void* params[] = {&p, &maps};
         LB_TRY(lb_launch(c, LBK_pf_attn_prepare, (unsigned)T, 1, 1, 256, 0, params, 1));
         const int rows = T * (m->HQ / m->HKV);
-        LB_TRY(lb_launch(c, LBK_pf_attn_chunk, (unsigned)((rows + LB_PF_ATTN_ROWS - 1) / LB_PF_ATTN_ROWS), (unsigned)m->HKV, 1,
-                         LB_PF_ATTN_THREADS, LB_PF_ATTN_SMEM, params, 1));
+        LB_TRY(lb_launch(c, LBK_pf_attn_chunk, (unsigned)((rows + LB_AC_ROWS - 1) / LB_AC_ROWS), (unsigned)m->HKV, 1, LB_AC_THREADS, LB_AC_SMEM, params, 1));
     }
     LB_TRY(gemm(m, &L->w_out, w->hy.mix16, w->hy.y, T));
     /* MLP */

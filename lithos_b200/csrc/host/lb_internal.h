@@ -11,6 +11,7 @@
 #include <cuda.h> /* types and enums only: the driver itself is bound at run time */
 
 #include "lithos_b200.h"
+#include "../kernels/params.h"
 
 #define LB_API __attribute__((visibility("default")))
 
@@ -152,6 +153,7 @@ int lb_driver_load(char* err, size_t errlen); /* LB_OK or LB_ERR_NO_DRIVER */
     X(wattn_chunk_64)                 \
     X(wattn_chunk_128)                \
     X(wattn_chunk_256)                \
+    X(wattn_chunk_tc)                 \
     X(da_step_64)                     \
     X(da_step_128)                    \
     X(da_step_256)                    \
@@ -257,6 +259,8 @@ int lb_launch(lb_ctx* c, int kernel, unsigned gx, unsigned gy, unsigned gz, unsi
               int pdl);
 int lb_launch_cluster(lb_ctx* c, int kernel, unsigned gx, unsigned gy, unsigned gz, unsigned bx, unsigned smem,
                       void** params, int pdl, unsigned cluster_y);
+/* tensor maps for the chunk attention on tcgen05: keys and values of rows 0..rows-1 */
+int lb_ac_fill(lb_ctx* c, lb_ac_maps* m, CUdeviceptr k, int k_ld, CUdeviceptr tail, int tail_w, int tail_ld, CUdeviceptr v, int v_ld, int vdim, int rows);
 int lb_launch_pairs(lb_ctx* c, int kernel, unsigned pairs, unsigned bx, unsigned smem, void** params, int pdl);
 
 unsigned char* lb_map_file(const char* path, size_t* bytes); /* lb_safetensors.c: a whole file, read-only */

@@ -421,6 +421,23 @@ LB_API int lb_attention_decode(lb_ctx* c, uint64_t q, uint64_t k_new, uint64_t v
     return lb_launch(c, LBK_attn_decode_mma, (unsigned)HKV, (unsigned)p.splits, 1, 256, lb_attn_mma_smem(G), params, 1);
 }
 
+/* tensor maps of a chunk's keys and values: `rows` rows of `ld` bf16 values, read in boxes of 64 features x box_rows */
+static int ac_map(lb_ctx* c, unsigned char* out, CUdeviceptr p, int width, int ld, int rows, int box_rows) {
+    CUtensorMap tm;
+    cuuint64_t dims[2] = {(cuuint64_t)width, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)ld * 2};
+    cuuint32_t box[2] = {64, (cuuint32_t)box_rows}, es[2] = {1, 1};
+    LB_CU(c, lb_drv.TensorMapEncodeTiled(&tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (void*)p, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                         CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE));
+    memcpy(out, &tm, sizeof tm);
+    return LB_OK;
+}
+int lb_ac_fill(lb_ctx* c, lb_ac_maps* m, CUdeviceptr k, int k_ld, CUdeviceptr tail, int tail_w, int tail_ld, CUdeviceptr v, int v_ld, int vdim, int rows) {
+    memset(m, 0, sizeof *m);
+    LB_TRY(ac_map(c, m->k, k, k_ld, k_ld, rows, 128));
+    if (tail) LB_TRY(ac_map(c, m->tail, tail, tail_w, tail_ld, rows, 128));
+    return ac_map(c, m->v, v, v_ld, v_ld, rows, 8192 / vdim);
+}
+
 LB_API int lb_rmsnorm(lb_ctx* c, uint64_t x, uint64_t res, uint64_t w, uint64_t y, uint64_t sum_out, int rows, int D,
                       float eps, int one_plus_w) {
     if (!c || !x || !w || !y || rows <= 0 || D <= 0) return lb_fail(c, LB_ERR_INVALID, "lb_rmsnorm: bad argument");

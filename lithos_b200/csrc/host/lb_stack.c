@@ -829,6 +829,20 @@ static void norm_adds(const lb_model* m, const pf_set* w, int i, lb_norm2_params
 }
 static int has_experts(const stack_t* S, int i) { return i >= 0 && S->d.layer[i].ff && S->d.layer[i].ff_kind == LB_FF_EXPERTS; }
 
+/* a chunk's attention: on tcgen05 where heads are whole 64s of features, on mma.sync otherwise */
+static int launch_wattn_chunk(lb_ctx* c, lb_wattn_params* p) {
+    const int rows = p->T * (p->H / p->KV), own = p->dim_p - p->tail_p;
+    lb_ac_maps maps;
+    void* params[] = {p, &maps};
+    if (own % 64 == 0 && p->tail_p % 64 == 0 && p->dim_p <= 256 && (p->vdim_p == 64 || p->vdim_p == 128 || p->vdim_p == 256)) {
+        LB_TRY(lb_ac_fill(c, &maps, (CUdeviceptr)p->k_cache, p->KV * own, (CUdeviceptr)p->k_tail, p->tail_p, p->tail_ld, (CUdeviceptr)p->v_cache, p->KV * p->vdim_p, p->vdim_p, p->pos0 + p->T));
+        return lb_launch(c, LBK_wattn_chunk_tc, (unsigned)((rows + LB_AC_ROWS - 1) / LB_AC_ROWS), (unsigned)p->KV, 1, LB_AC_THREADS, LB_AC_SMEM, params, 1);
+    }
+    const unsigned smem = (unsigned)(2 * LB_WA_ROWS * (2 * p->dim_p + 16) + 2 * LB_WA_KV * (2 * p->dim_p + 2 * p->vdim_p + 32));
+    return lb_launch(c, p->vdim_p <= 64 ? LBK_wattn_chunk_64 : p->vdim_p <= 128 ? LBK_wattn_chunk_128 : LBK_wattn_chunk_256,
+                     (unsigned)((rows + LB_WA_ROWS - 1) / LB_WA_ROWS), (unsigned)p->KV, 1, LB_WA_THREADS, smem, params, 1);
+}
+
 static int pf_latent(lb_model* m, pf_set* w, int i, int pos0, int T) {
     lb_ctx* c = m->c;
     stack_t* S = S_of(m);
@@ -858,10 +872,7 @@ static int pf_latent(lb_model* m, pf_set* w, int i, int pos0, int T) {
     a.sink = D->sink; a.sink_w = (const uint16_t*)L->sink; a.status = (uint32_t*)c->dev_status;
     a.H = a.KV = D->heads; a.dim = D->dim + D->rot_dim; a.dim_p = kd; a.vdim = D->vdim; a.vdim_p = L->vdim_p;
     a.pos0 = pos0; a.T = T; a.max_ctx = S->d.max_ctx; a.cat = (void*)w->st.cat; a.cat_ld = L->out.K;
-    void* aparams[] = {&a};
-    const unsigned smem = (unsigned)(2 * LB_WA_ROWS * (2 * kd + 16) + 2 * LB_WA_KV * (2 * kd + 2 * L->vdim_p + 32));
-    return lb_launch(c, L->vdim_p <= 64 ? LBK_wattn_chunk_64 : L->vdim_p <= 128 ? LBK_wattn_chunk_128 : LBK_wattn_chunk_256,
-                     (unsigned)((T + LB_WA_ROWS - 1) / LB_WA_ROWS), (unsigned)D->heads, 1, LB_WA_THREADS, smem, aparams, 1);
+    return launch_wattn_chunk(c, &a);
 }
 
 static int pf_ssm(lb_model* m, pf_set* w, int i, int pos0, int T) {
@@ -955,10 +966,7 @@ static int stack_pf_layer(lb_model* m, pf_set* w, int i, int pos0, int T) {
         } else {
             p.qh = (uint16_t*)w->st.q; p.ql = (uint16_t*)w->st.k;
             LB_TRY(lb_launch(c, LBK_wattn_prepare_bf16, (unsigned)T, 1, 1, 256, 0, params, 1));
-            const int rows = T * (D->heads / D->kv_heads);
-            const unsigned smem = (unsigned)(2 * LB_WA_ROWS * (2 * L->dim_p + 16) + 2 * LB_WA_KV * (2 * L->dim_p + 2 * L->vdim_p + 32));
-            LB_TRY(lb_launch(c, L->vdim_p <= 64 ? LBK_wattn_chunk_64 : L->vdim_p <= 128 ? LBK_wattn_chunk_128 : LBK_wattn_chunk_256,
-                             (unsigned)((rows + LB_WA_ROWS - 1) / LB_WA_ROWS), (unsigned)D->kv_heads, 1, LB_WA_THREADS, smem, params, 1));
+            LB_TRY(launch_wattn_chunk(c, &p));
         }
     } else {
         lb_decay_params2 p;

@@ -227,12 +227,21 @@ typedef struct {
     int32_t ld, HQ, HKV, pos0, T, rot_dims;
     float eps;
     double rope_freq[64];     /* theta^(-i/(rot_dims/2)), computed on the host in double */
+    uint32_t* status;
 } lb_pf_attn_params;
-/* pf_attn_chunk: query rows per CTA (16 per warp), threads, dynamic shared memory (two query tiles of ROWS x 528 B, two
- * stages of 32 K rows + 32 V rows x 528 B) */
-#define LB_PF_ATTN_ROWS 32
-#define LB_PF_ATTN_THREADS 64
-#define LB_PF_ATTN_SMEM (2 * LB_PF_ATTN_ROWS * 528 + 2 * 2 * 32 * 528)
+/* ---- chunk attention on tcgen05 (attention_tc.cuh) ------------------------- */
+#define LB_AC_ROWS 128      /* query rows per CTA */
+#define LB_AC_THREADS 192
+#define LB_AC_UNIT 16384    /* bytes of a ring unit: 64 features x 128 keys, or vdim features x 8192 / vdim keys */
+#define LB_AC_MAX_UNITS 10
+#define LB_AC_SMEM 229376   /* what queries (two terms of 128 rows) and ring share */
+#define LB_AC_RING(dim) ((LB_AC_SMEM - 512 * (dim)) / LB_AC_UNIT)
+#define LB_AC_UNITS(dim) (LB_AC_RING(dim) < LB_AC_MAX_UNITS ? LB_AC_RING(dim) : LB_AC_MAX_UNITS)
+typedef struct {
+    unsigned char k[128] __attribute__((aligned(64)));    /* tensor maps, boxes of 64 features x 128 rows: keys [rows, KV heads * own features] ... */
+    unsigned char tail[128] __attribute__((aligned(64))); /* ... the features that the KV heads share [rows, tail] ... */
+    unsigned char v[128] __attribute__((aligned(64)));    /* ... and values [rows, KV heads * vdim], boxes of 64 features x 8192 / vdim rows */
+} lb_ac_maps;
 
 /* ---- GQA decode attention ------------------------------------------------- */
 typedef struct {

@@ -243,185 +243,41 @@ extern "C" __global__ void __launch_bounds__(256) pf_attn_prepare(const __grid_c
     }
 }
 
-#define PA_ROWS LB_PF_ATTN_ROWS   // query rows per CTA
-#define PA_WARPS (PA_ROWS / 16)  // warps per CTA, 16 query rows each
-#define PA_KV 32                 // cache rows per staged block
-#define PA_STRIDE 528            // bytes per staged row: 512 + 16 (8 rows on 8 different bank groups)
-#define PA_THREADS LB_PF_ATTN_THREADS
-// dynamic shared memory: qh | ql [PA_ROWS][528], then two stages of K | V [PA_KV][528]
-static_assert(PA_THREADS == 32 * PA_WARPS && LB_PF_ATTN_SMEM == 2 * PA_ROWS * PA_STRIDE + 2 * 2 * PA_KV * PA_STRIDE, "launch geometry");
-
-__device__ __forceinline__ void pa_mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ void pa_ldsm(uint32_t addr, uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(addr));
-}
-__device__ __forceinline__ void pa_ldsm_t(uint32_t addr, uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(addr));
-}
-__device__ __forceinline__ void pa_cp16(uint32_t dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void pa_split(float x, float y, uint32_t& hi, uint32_t& lo) {
-    const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
-    const float2 hf = __bfloat1622float2(h);
-    const __nv_bfloat162 l = __floats2bfloat162_rn(x - hf.x, y - hf.y);
-    hi = *reinterpret_cast<const uint32_t*>(&h);
-    lo = *reinterpret_cast<const uint32_t*>(&l);
-}
-
-// grid (ceil(T*G / PA_ROWS), HKV), block PA_THREADS.  Query row R of a KV head = (token R / G, head R % G): a warp's 16 rows
-// are 16/G consecutive tokens, so their causal limits differ by a few rows only.  S = Q K^T and O = P V as
-// mma.sync.m16n8k16 bf16 with Q and P split into two bf16 terms (the decode kernel's precision: 16 bits of Q and P, K and V
-// exact in bf16), online soft-max per row in the four lanes that hold the row, cache rows staged 32 at a time by cp.async
-// in two stages shared by the CTA's warps.  The M side is query rows x heads here, which is why this is not the decode
-// kernel with a loop around it: a cache row is read once per CTA instead of once per token.
-extern "C" __global__ void __launch_bounds__(PA_THREADS) pf_attn_chunk(const __grid_constant__ lb_pf_attn_params p) {
-    extern __shared__ __align__(16) unsigned char pa_sm[];
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const int fg = lane >> 2, ft = lane & 3;
-    const int kv = blockIdx.y, G = p.HQ / p.HKV;
-    const int R0 = blockIdx.x * PA_ROWS;
-    const int n_rows = p.T * G;
-    unsigned char* qh_s = pa_sm;
-    unsigned char* ql_s = qh_s + PA_ROWS * PA_STRIDE;
-    unsigned char* kv_s = ql_s + PA_ROWS * PA_STRIDE; // stage st: K at st * 2 * PA_KV * PA_STRIDE, V after it
-    pdl_wait();
-
-    // the CTA's query rows (rows past the chunk repeat the last one; they are never stored)
-    for (int i = t; i < PA_ROWS * 32; i += PA_THREADS) {
-        const int r = i >> 5, c = i & 31;
-        const int R = min(R0 + r, n_rows - 1), s = R / G, g = R - s * G;
-        const size_t src = (((size_t)s * p.HQ + kv * G + g) * AT_D) * 2 + c * 16;
-        pa_cp16(smem_u32(qh_s + r * PA_STRIDE + c * 16), reinterpret_cast<const unsigned char*>(p.qh) + src);
-        pa_cp16(smem_u32(ql_s + r * PA_STRIDE + c * 16), reinterpret_cast<const unsigned char*>(p.ql) + src);
+// grid (ceil(T*G / 128), HKV), block LB_AC_THREADS: all tokens of the chunk, token s over the cache rows [0, pos0 + s].  Query row R of a KV head = (token
+// R / G, head R % G), so a cache row is read once per 128 rows instead of once per token; the tiles that see most keys start first.
+#include "attention_tc.cuh"
+struct pf_chunk_rows {
+    const lb_pf_attn_params& p;
+    int kv, G;
+    const uint16_t *qh, *ql;
+    __device__ __forceinline__ size_t q_at(int R) const { return ((size_t)(R / G) * p.HQ + kv * G + R % G) * AT_D; }
+    __device__ __forceinline__ int lim(int R) const { return p.pos0 + R / G; }
+    __device__ __forceinline__ int low(int) const { return 0; }
+    __device__ __forceinline__ float m0(int) const { return -1e30f; }
+    __device__ __forceinline__ float l0() const { return 0.f; }
+    __device__ __forceinline__ void table(unsigned char*, int) const {}
+    // out[s][hq][d..d+15] = fp16( O / l * sigmoid(gate) )
+    __device__ __forceinline__ void store(unsigned char*, int, int R, int d, const uint32_t (&r)[16], float inv) const {
+        const int s = R / G, hq = kv * G + R % G;
+        const float* gate = p.proj + (size_t)s * p.ld + (size_t)hq * 512 + 256 + d;
+        uint32_t o[8];
+#pragma unroll
+        for (int j = 0; j < 16; j += 4) {
+            const float4 g = *reinterpret_cast<const float4*>(gate + j);
+            const __half2 a = __floats2half2_rn(__uint_as_float(r[j]) * inv * sigmoidf_dev(g.x), __uint_as_float(r[j + 1]) * inv * sigmoidf_dev(g.y));
+            const __half2 b = __floats2half2_rn(__uint_as_float(r[j + 2]) * inv * sigmoidf_dev(g.z), __uint_as_float(r[j + 3]) * inv * sigmoidf_dev(g.w));
+            o[j / 2] = *reinterpret_cast<const uint32_t*>(&a);
+            o[j / 2 + 1] = *reinterpret_cast<const uint32_t*>(&b);
+        }
+        uint4* dst = reinterpret_cast<uint4*>(p.out + ((size_t)s * p.HQ + hq) * AT_D + d);
+        dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
+        dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
     }
-    // last cache row any row of this CTA may see, and of this warp
-    const int s_cta = min(R0 + PA_ROWS - 1, n_rows - 1) / G;
-    const int last_row = p.pos0 + s_cta;
-    const int n_blocks = last_row / PA_KV + 1;
-    const size_t row_bytes = (size_t)p.HKV * AT_D * 2;
-    auto stage = [&](int b) { // rows past the last one repeat it (finite values; masked below)
-        unsigned char* dst = kv_s + (b & 1) * (2 * PA_KV * PA_STRIDE);
-        for (int i = t; i < 2 * PA_KV * 32; i += PA_THREADS) {
-            const int which = i / (PA_KV * 32), r = (i >> 5) % PA_KV, c = i & 31;
-            const int row = min(b * PA_KV + r, last_row);
-            const unsigned char* base = reinterpret_cast<const unsigned char*>(which ? p.v_cache : p.k_cache);
-            pa_cp16(smem_u32(dst + (which * PA_KV + r) * PA_STRIDE + c * 16), base + (size_t)row * row_bytes + (size_t)kv * AT_D * 2 + c * 16);
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    stage(0);
-
-    // rows fg and fg+8 of the warp's tile
-    int lim[2];
-#pragma unroll
-    for (int i = 0; i < 2; ++i) lim[i] = p.pos0 + min(R0 + warp * 16 + fg + 8 * i, n_rows - 1) / G;
-    const int warp_last = p.pos0 + min(R0 + warp * 16 + 15, n_rows - 1) / G;
-    float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
-    float acc[32][4];
-#pragma unroll
-    for (int nb = 0; nb < 32; ++nb) acc[nb][0] = acc[nb][1] = acc[nb][2] = acc[nb][3] = 0.f;
-    // ldmatrix lane addresses.  A (Q rows, x4): (rows 0-7, dims c..c+7), (rows 8-15, c), (rows 0-7, c+8), (rows 8-15, c+8)
-    const uint32_t a_off = (warp * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * PA_STRIDE + (lane >> 4) * 16;
-    const uint32_t qh_lane = smem_u32(qh_s) + a_off, ql_lane = smem_u32(ql_s) + a_off;
-    // K (x4): (rows 0-7, dims c..c+7), (rows 0-7, c+8), (rows 8-15, c), (rows 8-15, c+8)
-    const uint32_t k_off = ((lane & 7) + ((lane >> 4) << 3)) * PA_STRIDE + ((lane >> 3) & 1) * 16;
-    // V (x4, transposed): (rows 0-7, dims d..d+7), (rows 8-15, d), (rows 0-7, d+8), (rows 8-15, d+8)
-    const uint32_t v_off = ((lane & 7) + ((lane >> 3) & 1) * 8) * PA_STRIDE + (lane >> 4) * 16;
-
-    for (int b = 0; b < n_blocks; ++b) {
-        if (b + 1 < n_blocks) {
-            stage(b + 1);
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-        } else {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-        }
-        __syncthreads();
-        if (b * PA_KV <= warp_last) {
-            const uint32_t k_addr = smem_u32(kv_s + (b & 1) * (2 * PA_KV * PA_STRIDE)), v_addr = k_addr + PA_KV * PA_STRIDE;
-            float sc[4][4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) sc[j][0] = sc[j][1] = sc[j][2] = sc[j][3] = 0.f;
-#pragma unroll
-            for (int c = 0; c < 16; ++c) {
-                uint32_t h0, h1, h2, h3, l0, l1, l2, l3;
-                pa_ldsm(qh_lane + c * 32, h0, h1, h2, h3);
-                pa_ldsm(ql_lane + c * 32, l0, l1, l2, l3);
-#pragma unroll
-                for (int jj = 0; jj < 2; ++jj) {
-                    uint32_t b00, b01, b10, b11;
-                    pa_ldsm(k_addr + k_off + jj * 16 * PA_STRIDE + c * 32, b00, b01, b10, b11);
-                    pa_mma(sc[2 * jj], h0, h1, h2, h3, b00, b01);
-                    pa_mma(sc[2 * jj], l0, l1, l2, l3, b00, b01);
-                    pa_mma(sc[2 * jj + 1], h0, h1, h2, h3, b10, b11);
-                    pa_mma(sc[2 * jj + 1], l0, l1, l2, l3, b10, b11);
-                }
-            }
-            // sc[j][0..1]: row fg, cache rows b*32 + 8j + 2ft, +1; sc[j][2..3]: row fg+8
-            float corr[2];
-            uint32_t ph[4][2], pl[4][2]; // [j][row half]: the probabilities as bf16 pairs
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                float mx = -INFINITY;
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const int r0 = b * PA_KV + 8 * j + 2 * ft;
-                    if (r0 > lim[i]) sc[j][2 * i] = -INFINITY;
-                    if (r0 + 1 > lim[i]) sc[j][2 * i + 1] = -INFINITY;
-                    mx = fmaxf(mx, fmaxf(sc[j][2 * i], sc[j][2 * i + 1]));
-                }
-                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-                const float m_new = fmaxf(m_run[i], mx); // finite from block 0 on: cache row 0 is visible to every query row
-                corr[i] = exp2f(m_run[i] - m_new);       // exp2f(-inf) = 0 on the first block
-                float ps = 0.f;
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const float p0 = exp2f(sc[j][2 * i] - m_new), p1 = exp2f(sc[j][2 * i + 1] - m_new);
-                    ps += p0 + p1;
-                    pa_split(p0, p1, ph[j][i], pl[j][i]);
-                }
-                ps += __shfl_xor_sync(0xffffffffu, ps, 1);
-                ps += __shfl_xor_sync(0xffffffffu, ps, 2);
-                l_run[i] = fmaf(l_run[i], corr[i], ps);
-                m_run[i] = m_new;
-            }
-            // O += P V: k-step kk = cache rows 16kk..16kk+15 (score blocks 2kk, 2kk+1), n-block nb = dims 8nb..8nb+7
-#pragma unroll
-            for (int nb = 0; nb < 32; nb += 2) {
-                acc[nb][0] *= corr[0]; acc[nb][1] *= corr[0]; acc[nb][2] *= corr[1]; acc[nb][3] *= corr[1];
-                acc[nb + 1][0] *= corr[0]; acc[nb + 1][1] *= corr[0]; acc[nb + 1][2] *= corr[1]; acc[nb + 1][3] *= corr[1];
-#pragma unroll
-                for (int kk = 0; kk < 2; ++kk) {
-                    uint32_t v0, v1, v2, v3;
-                    pa_ldsm_t(v_addr + v_off + kk * 16 * PA_STRIDE + nb * 16, v0, v1, v2, v3);
-                    pa_mma(acc[nb], ph[2 * kk][0], ph[2 * kk][1], ph[2 * kk + 1][0], ph[2 * kk + 1][1], v0, v1);
-                    pa_mma(acc[nb], pl[2 * kk][0], pl[2 * kk][1], pl[2 * kk + 1][0], pl[2 * kk + 1][1], v0, v1);
-                    pa_mma(acc[nb + 1], ph[2 * kk][0], ph[2 * kk][1], ph[2 * kk + 1][0], ph[2 * kk + 1][1], v2, v3);
-                    pa_mma(acc[nb + 1], pl[2 * kk][0], pl[2 * kk][1], pl[2 * kk + 1][0], pl[2 * kk + 1][1], v2, v3);
-                }
-            }
-        }
-        __syncthreads(); // every warp is done with this stage before block b+2 overwrites it
-    }
-
-    // out[s][hq][dim] = fp16( O / l * sigmoid(gate) ): lane (fg, ft) holds dims 8nb + 2ft, +1 of rows fg and fg+8
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        const int R = R0 + warp * 16 + fg + 8 * i;
-        if (R >= n_rows) continue;
-        const int s = R / G, hq = kv * G + (R - s * G);
-        const float inv = 1.0f / l_run[i];
-        const float* gate = p.proj + (size_t)s * p.ld + (size_t)hq * 512 + 256;
-        __half2* dst = reinterpret_cast<__half2*>(p.out + ((size_t)s * p.HQ + hq) * AT_D);
-#pragma unroll
-        for (int nb = 0; nb < 32; ++nb) {
-            const float2 gt = *reinterpret_cast<const float2*>(gate + 8 * nb + 2 * ft);
-            dst[4 * nb + ft] = __floats2half2_rn(acc[nb][2 * i] * inv * sigmoidf_dev(gt.x), acc[nb][2 * i + 1] * inv * sigmoidf_dev(gt.y));
-        }
-    }
+};
+extern "C" __global__ void __launch_bounds__(LB_AC_THREADS, 1) pf_attn_chunk(const __grid_constant__ lb_pf_attn_params p, const __grid_constant__ lb_ac_maps maps) {
+    extern __shared__ __align__(1024) unsigned char pa_sm[];
+    __shared__ ac_shared sh;
+    const int G = p.HQ / p.HKV, n_rows = p.T * G, R0 = (int)(gridDim.x - 1 - blockIdx.x) * AC_ROWS;
+    const pf_chunk_rows c = {p, (int)blockIdx.y, G, p.qh, p.ql};
+    attn_chunk_tc(c, maps, sh, pa_sm, (int)blockIdx.y, R0, n_rows, 0, p.pos0 + min(R0 + AC_ROWS - 1, n_rows - 1) / G, AT_D, AT_D, AT_D, LB_AC_UNITS(AT_D), p.status);
 }

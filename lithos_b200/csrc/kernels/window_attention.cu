@@ -6,9 +6,10 @@
 // Scores, weights and sums are fp32; angles are reduced in double.
 //   wattn_rows_*   one query token per CTA row: the decode step (positions cut into slices merged by the last CTA), and prompts in fp32
 //   wattn_prepare  a prompt chunk's keys and values into the cache; its queries as two bf16 terms
-//   wattn_chunk_*  a prompt chunk on the tensor cores
+//   wattn_chunk_tc a prompt chunk on the tensor cores (attention_tc.cuh), heads of whole 64s of features; wattn_chunk_*: other sizes, mma.sync
 #include "mma_sync.cuh"
 #include "rotate.cuh"
+#include "attention_tc.cuh"
 
 struct wa_angles { // cosines and sines of a position: key / query pairs and value pairs
     float ck[LB_WA_MAX_DIM / 2], sk[LB_WA_MAX_DIM / 2], cv[LB_WA_MAX_DIM / 2], sv[LB_WA_MAX_DIM / 2];
@@ -498,3 +499,60 @@ __device__ __forceinline__ void wattn_chunk_body(const lb_wattn_params& p) {
 extern "C" __global__ void __launch_bounds__(LB_WA_THREADS) wattn_chunk_64(const __grid_constant__ lb_wattn_params p) { wattn_chunk_body<8>(p); }
 extern "C" __global__ void __launch_bounds__(LB_WA_THREADS) wattn_chunk_128(const __grid_constant__ lb_wattn_params p) { wattn_chunk_body<16>(p); }
 extern "C" __global__ void __launch_bounds__(LB_WA_THREADS) wattn_chunk_256(const __grid_constant__ lb_wattn_params p) { wattn_chunk_body<32>(p); }
+
+// The same on tcgen05 (attention_tc.cuh), where keys (own part and tail) are whole 64s of features and values 64, 128 or 256.
+// grid (ceil(T G / 128), KV), block LB_AC_THREADS; the tiles that see most keys start first.
+struct wa_chunk_rows {
+    const lb_wattn_params& p;
+    int kv, G;
+    const uint16_t *qh, *ql;
+    __device__ __forceinline__ size_t q_at(int R) const { return ((size_t)(R / G) * p.H + kv * G + R % G) * p.dim_p; }
+    __device__ __forceinline__ int lim(int R) const { return p.pos0 + R / G; }
+    __device__ __forceinline__ int low(int R) const { return p.block > 0 ? lim(R) / p.block * p.block : 0; }
+    __device__ __forceinline__ float m0(int R) const { return !p.sink ? -1e30f : p.sink_w ? bf16_bits_to_f32(p.sink_w[kv * G + R % G]) * 1.4426950408889634f : 0.f; }
+    __device__ __forceinline__ float l0() const { return p.sink ? 1.f : 0.f; }
+    // rotated values: cosine and sine of every (token, pair) of the tile, [tokens][vdim / 2]; the tile's heads of a token share them
+    __device__ __forceinline__ void table(unsigned char* sm, int R0) const {
+        if (!p.freq_v) return;
+        const int pairs = p.vdim / 2, s0 = R0 / G, tokens = min(R0 + AC_ROWS - 1, p.T * G - 1) / G - s0 + 1;
+        for (int i = threadIdx.x - 64; i < tokens * pairs; i += 128) {
+            float2 a;
+            wa_angle(p.freq_v[i % pairs], p.pos0 + s0 + i / pairs, a.x, a.y);
+            reinterpret_cast<float2*>(sm)[i] = a;
+        }
+    }
+    __device__ __forceinline__ void store(unsigned char* sm, int R0, int R, int d, const uint32_t (&r)[16], float inv) const {
+        const int s = R / G, pairs = p.vdim / 2;
+        __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.cat) + (size_t)s * p.cat_ld + (size_t)(kv * G + R % G) * p.vdim + d;
+        const float2* t = reinterpret_cast<const float2*>(sm) + (size_t)(s - R0 / G) * pairs + d / 2;
+        uint32_t o[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            float u = __uint_as_float(r[2 * j]) * inv, v = __uint_as_float(r[2 * j + 1]) * inv;
+            if (p.freq_v && d + 2 * j + 1 < p.vdim) { // a value pair turns back by its token's position
+                const float2 cs = t[j];
+                const float a = u * cs.x + v * cs.y;
+                v = v * cs.x - u * cs.y;
+                u = a;
+            }
+            const __nv_bfloat162 b = __floats2bfloat162_rn(u, v);
+            o[j] = *reinterpret_cast<const uint32_t*>(&b);
+        }
+        if (((p.vdim | p.cat_ld) & 7) == 0 && d + 16 <= p.vdim) {
+            reinterpret_cast<uint4*>(dst)[0] = make_uint4(o[0], o[1], o[2], o[3]);
+            reinterpret_cast<uint4*>(dst)[1] = make_uint4(o[4], o[5], o[6], o[7]);
+        } else {
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+                if (d + j < p.vdim) reinterpret_cast<uint16_t*>(dst)[j] = (uint16_t)(o[j >> 1] >> (16 * (j & 1)));
+        }
+    }
+};
+extern "C" __global__ void __launch_bounds__(LB_AC_THREADS, 1) wattn_chunk_tc(const __grid_constant__ lb_wattn_params p, const __grid_constant__ lb_ac_maps maps) {
+    extern __shared__ __align__(1024) unsigned char wt_sm[];
+    __shared__ ac_shared sh;
+    const int G = p.H / p.KV, n_rows = p.T * G, R0 = (int)(gridDim.x - 1 - blockIdx.x) * AC_ROWS;
+    const wa_chunk_rows c = {p, (int)blockIdx.y, G, p.qh, p.ql};
+    attn_chunk_tc(c, maps, sh, wt_sm, (int)blockIdx.y, R0, n_rows, c.low(R0), c.lim(min(R0 + AC_ROWS - 1, n_rows - 1)), p.dim_p, p.dim_p - p.tail_p, p.vdim_p, LB_AC_UNITS(p.dim_p),
+                  p.status);
+}
