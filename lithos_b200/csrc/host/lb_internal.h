@@ -102,6 +102,8 @@ int lb_driver_load(char* err, size_t errlen); /* LB_OK or LB_ERR_NO_DRIVER */
     X(decay_gate_beta)                \
     X(deltanet_step_bf16)             \
     X(deltanet_step_f32)              \
+    X(deltanet_step16_bf16)           \
+    X(deltanet_step16_f32)            \
     X(deltanet_one_bf16)              \
     X(deltanet_one_f32)               \
     X(deltanet_two_bf16)              \

@@ -367,10 +367,15 @@ LB_API int lb_deltanet_step(lb_ctx* c, uint64_t state, uint64_t q, uint64_t k, u
     p.HV = HV; p.HK = HK;
     void* params[] = {&p, &n_steps};
     /* two steps: the kernel of few steps while its CTAs are at most two per SM (fp32, two steps / run: 48 heads 3.74 / 3.96 us, 96 heads 4.99 / 4.66) */
-    const int kernel = n_steps == 1 ? (in_is_f32 ? LBK_deltanet_one_f32 : LBK_deltanet_one_bf16)
-                     : n_steps == 2 && 2 * HV <= c->sm_count ? (in_is_f32 ? LBK_deltanet_two_f32 : LBK_deltanet_two_bf16)
-                                    : (in_is_f32 ? LBK_deltanet_step_f32 : LBK_deltanet_step_bf16);
-    return lb_launch(c, kernel, (unsigned)HV, 4, 1, 128, 0, params, 1);
+    const int few = n_steps == 1 || (n_steps == 2 && 2 * HV <= c->sm_count);
+    /* More than eight steps: 16 columns per CTA instead of 32 where the fullest SM then has less than twice as many of them.  us, 32 / 16 columns: 48 heads (two
+     * CTAs / three) 8 steps 4.8 / 5.1, 16 7.3 / 7.1, 64 21.5 / 19.5, 256 78.4 / 68.9; 16 heads (one / one) 16 steps 5.0 / 4.5, 256 52.1 / 42.1; 24 and 32 heads
+     * (one / two) 24 steps 6.6 / 7.2, 256 52.1 / 53.5 */
+    const int narrow = !few && n_steps > 8 && (8 * HV + c->sm_count - 1) / c->sm_count < 2 * ((4 * HV + c->sm_count - 1) / c->sm_count);
+    const int kernel = few ? (n_steps == 1 ? (in_is_f32 ? LBK_deltanet_one_f32 : LBK_deltanet_one_bf16) : (in_is_f32 ? LBK_deltanet_two_f32 : LBK_deltanet_two_bf16))
+                     : narrow ? (in_is_f32 ? LBK_deltanet_step16_f32 : LBK_deltanet_step16_bf16)
+                              : (in_is_f32 ? LBK_deltanet_step_f32 : LBK_deltanet_step_bf16);
+    return lb_launch(c, kernel, (unsigned)HV, narrow ? 8 : 4, 1, 128, 0, params, 1);
 }
 
 LB_API int lb_decay_gate(lb_ctx* c, uint64_t a, uint64_t a_log, uint64_t dt_bias, uint64_t b, uint64_t g_out,

@@ -15,16 +15,18 @@
 // n_steps > 1 it stays on chip for the whole run of steps.
 #include "deltanet_core.cuh"
 
-// A warp owns 8 columns of a head, all 128 rows of them: lane (rg, cg) holds 16 rows (four neighbouring ones of every 32, so that the
-// lanes' 16-byte reads of a token's k or q are one conflict-free wavefront) of 2 columns, the rows in pairs for packed multiply-adds; cg is
-// the fast part of the lane number, so that a half-warp's 8-byte accesses to the state fill whole sectors.  A
+// A warp owns 4 CL columns of a head, all 128 rows of them: lane (rg, cg) holds 16 rows (four neighbouring ones of every 32, so that the
+// lanes' 16-byte reads of a token's k or q are free of conflicts) of CL columns, the rows in pairs for packed multiply-adds; cg is
+// the fast part of the lane number, so that neighbouring lanes' accesses to the state are neighbours.  A
 // step needs nothing from another warp: both sums over the rows end in three shuffles, and what the warps of a CTA share, the operands of
 // DN_RUN tokens in fp32, costs one block barrier per DN_RUN tokens.  A thread loads its piece of the run after next into registers and
 // stores it a run later, so the chain of a step (dot, three shuffles, update) meets no trip to L2.  The read-outs of four tokens are summed
-// together (seven shuffles instead of 24), in the order of a single one: the same bits for one step and for many.
-// 48 heads, bf16 (us before -> after; before: a column's rows in four lanes, 16 reads of k and q and a barrier a token): 5.0 -> 4.2 at 4 steps,
-// 38 -> 24 at 64, 144 -> 86 at 256.  Two warps per scheduler now take 620 cycles a token, of which 256 are the
-// multiply-adds' and 440 one warp's chain; reading the next token's k ahead moved it by 3 % either way.
+// together, in the order of a single one: the same bits for one step and for many.
+// DN_RUN whole tokens are one stretch of code without a branch, in which a token's read-out and decay and the next token's operands lie in the shadow of the
+// recall's shuffles.  What a step costs then is its instructions and that chain (140 instructions of a warp at CL = 2, 390 cycles alone on a scheduler) and,
+// with three CTAs on an SM, what shared memory delivers (16 bytes to every lane per read, 8 reads a token and warp).  CL = 1 has twice the warps to
+// balance and hide the chain with, CL = 2 half the start.  us a call, before -> CL = 2, CL = 1 (the rule stands at lb_deltanet_step): 256 steps of 16 heads 64.6 -> 52.1, 42.1;
+// 24 64.6 -> 52.1, 53.5; 32 64.8 -> 52.3, 53.6; 48 86.6 -> 78.4, 68.9; 8 steps of 48 heads 5.06 -> 4.77, 5.06.
 #define DN_RUN 8
 template <typename T> struct dn_in; // element type of q, k, v: 16 bytes of them, and how they go to shared memory as fp32
 template <> struct dn_in<float> {
@@ -63,80 +65,82 @@ __device__ __forceinline__ float dn_sum4(uint64_t a, uint64_t b) { // two runnin
     return (x.x + x.y) + (y.x + y.y);
 }
 
-// a lane's two columns of a state row: 8 bytes at once where the state's address allows it (PAIRS)
-template <bool PAIRS> __device__ __forceinline__ float2 dn_row(const float* r) {
-    if (!PAIRS) return make_float2(r[0], r[1]);
-    return *reinterpret_cast<const float2*>(r);
-}
-template <bool PAIRS> __device__ __forceinline__ void dn_load_rows(const float* S, uint64_t (&s)[4][2][2]) {
-    float2 x[4][2][2];
+// a lane's CL columns of a state row: 8 bytes at once where the state's address allows it (PAIRS)
+template <int CL, bool PAIRS> __device__ __forceinline__ void dn_load_rows(const float* S, uint64_t (&s)[4][2][CL]) {
+    __align__(8) float x[4][4][CL];
 #pragma unroll
-    for (int i = 0; i < 16; ++i) x[i >> 2][(i >> 1) & 1][i & 1] = dn_row<PAIRS>(S + (size_t)(32 * (i >> 2) + (i & 3)) * DN_D);
+    for (int i = 0; i < 16; ++i) {
+        const float* r = S + (size_t)(32 * (i >> 2) + (i & 3)) * DN_D;
+        if (PAIRS) *reinterpret_cast<float2*>(x[i >> 2][i & 3]) = *reinterpret_cast<const float2*>(r);
+        else
+#pragma unroll
+            for (int c = 0; c < CL; ++c) x[i >> 2][i & 3][c] = r[c];
+    }
 #pragma unroll
     for (int j = 0; j < 4; ++j)
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            s[j][e][0] = dn_pack(x[j][e][0].x, x[j][e][1].x);
-            s[j][e][1] = dn_pack(x[j][e][0].y, x[j][e][1].y);
-        }
+        for (int e = 0; e < 2; ++e)
+#pragma unroll
+            for (int c = 0; c < CL; ++c) s[j][e][c] = dn_pack(x[j][2 * e][c], x[j][2 * e + 1][c]);
 }
-__device__ __forceinline__ void dn_load_state(const float* S, bool pairs, uint64_t (&s)[4][2][2]) {
-    if (pairs) dn_load_rows<true>(S, s);
-    else dn_load_rows<false>(S, s);
+template <int CL> __device__ __forceinline__ void dn_load_state(const float* S, bool pairs, uint64_t (&s)[4][2][CL]) {
+    if (CL == 2 && pairs) dn_load_rows<CL, CL == 2>(S, s);
+    else dn_load_rows<CL, false>(S, s);
 }
-__device__ __forceinline__ void dn_store_state(float* S, bool pairs, const uint64_t (&s)[4][2][2]) {
+template <int CL> __device__ __forceinline__ void dn_store_state(float* S, bool pairs, const uint64_t (&s)[4][2][CL]) {
 #pragma unroll
     for (int j = 0; j < 4; ++j)
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
             float* r = S + (size_t)(32 * j + 2 * e) * DN_D;
-            const float2 x = dn_unpack(s[j][e][0]), y = dn_unpack(s[j][e][1]);
-            if (pairs) {
+            const float2 x = dn_unpack(s[j][e][0]), y = dn_unpack(s[j][e][CL - 1]);
+            if (CL == 2 && pairs) {
                 *reinterpret_cast<float2*>(r) = make_float2(x.x, y.x);
                 *reinterpret_cast<float2*>(r + DN_D) = make_float2(x.y, y.y);
             } else {
-                r[0] = x.x; r[1] = y.x;
-                r[DN_D] = x.y; r[DN_D + 1] = y.y;
+                r[0] = x.x; r[DN_D] = x.y;
+                if (CL == 2) { r[1] = y.x; r[DN_D + 1] = y.y; }
             }
         }
 }
-// r_j = sum_i k_i S_ij (pre-update state): four running sums per column
-__device__ __forceinline__ void dn_recall(const uint64_t (&k)[4][2], const uint64_t (&s)[4][2][2], uint64_t (&a)[2][2]) {
+// sum_i k_i S_ij over this lane's rows: four running sums per column
+template <int CL> __device__ __forceinline__ void dn_dot(const uint64_t (&k)[4][2], const uint64_t (&s)[4][2][CL], float (&r)[CL]) {
+    uint64_t a[CL][2];
 #pragma unroll
     for (int j = 0; j < 4; ++j)
 #pragma unroll
-        for (int c = 0; c < 2; ++c)
+        for (int c = 0; c < CL; ++c)
 #pragma unroll
             for (int e = 0; e < 2; ++e) a[c][e] = j ? dn_fma2(k[j][e], s[j][e][c], a[c][e]) : dn_mul2(k[j][e], s[j][e][c]);
+#pragma unroll
+    for (int c = 0; c < CL; ++c) r[c] = dn_sum4(a[c][0], a[c][1]);
 }
-__device__ __forceinline__ void dn_decay(float g, uint64_t (&s)[4][2][2]) {
+template <int CL> __device__ __forceinline__ void dn_decay(float g, uint64_t (&s)[4][2][CL]) {
     const uint64_t g2 = dn_pack(g, g);
 #pragma unroll
     for (int j = 0; j < 4; ++j)
 #pragma unroll
         for (int e = 0; e < 2; ++e)
 #pragma unroll
-            for (int c = 0; c < 2; ++c) s[j][e][c] = dn_mul2(g2, s[j][e][c]);
+            for (int c = 0; c < CL; ++c) s[j][e][c] = dn_mul2(g2, s[j][e][c]);
 }
-// S_ij += k_i d_j on the decayed state, o_j = sum_i S_ij q_i
-__device__ __forceinline__ void dn_update(const uint64_t (&k)[4][2], const uint64_t (&q)[4][2], float d0, float d1, uint64_t (&s)[4][2][2], uint64_t (&a)[2][2]) {
-    const uint64_t d[2] = {dn_pack(d0, d0), dn_pack(d1, d1)};
+// d_j = beta (v_j - r_j), S_ij += k_i d_j on the decayed state
+template <int CL> __device__ __forceinline__ void dn_write(const uint64_t (&k)[4][2], float beta, const float (&v)[CL], const float (&r)[CL], uint64_t (&s)[4][2][CL]) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
+    for (int c = 0; c < CL; ++c) {
+        const float dj = beta * (v[c] - r[c]);
+        const uint64_t d = dn_pack(dj, dj);
 #pragma unroll
-        for (int c = 0; c < 2; ++c)
+        for (int j = 0; j < 4; ++j)
 #pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                s[j][e][c] = dn_fma2(k[j][e], d[c], s[j][e][c]);
-                a[c][e] = j ? dn_fma2(q[j][e], s[j][e][c], a[c][e]) : dn_mul2(q[j][e], s[j][e][c]);
-            }
-}
-__device__ __forceinline__ void dn_reduce(float& x, float& y) { // over the eight row groups
-#pragma unroll
-    for (int m = 4; m < 32; m <<= 1) {
-        x += __shfl_xor_sync(0xffffffffu, x, m);
-        y += __shfl_xor_sync(0xffffffffu, y, m);
+            for (int e = 0; e < 2; ++e) s[j][e][c] = dn_fma2(k[j][e], d, s[j][e][c]);
     }
+}
+template <int CL> __device__ __forceinline__ void dn_reduce(float (&r)[CL]) { // over the eight row groups
+#pragma unroll
+    for (int m = 4; m < 32; m <<= 1)
+#pragma unroll
+        for (int c = 0; c < CL; ++c) r[c] += __shfl_xor_sync(0xffffffffu, r[c], m);
 }
 __device__ __forceinline__ void dn_read(const float* row, uint64_t (&r)[4][2]) { // a lane's rows of k or q, from shared memory
 #pragma unroll
@@ -225,16 +229,16 @@ __device__ __forceinline__ void deltanet_few(const lb_deltanet_params& p) {
 
 // n_steps consecutive tokens: q,k are [n_steps][HK][128], v (z, out) are
 // [n_steps][HV][128], g and beta are [n_steps][HV].
-template <typename T>
+template <typename T, int CL>
 __device__ __forceinline__ void deltanet_body(const lb_deltanet_params& p, int n_steps) {
-    constexpr int N = dn_in<T>::N, PIECES = DN_RUN * 2 * DN_D / N, PER = PIECES / DN_THREADS; // 16-byte pieces of a run's k and q
-    constexpr int VP = DN_RUN * DN_COLS / N;
-    __shared__ __align__(16) float kq[2][DN_RUN][2][DN_D], vs[2][DN_RUN][DN_COLS], gb[2][2][DN_RUN];
+    constexpr int THREADS = DN_THREADS, COLS = CL * THREADS / 8, N = dn_in<T>::N, PIECES = DN_RUN * 2 * DN_D / N, PER = PIECES / THREADS; // 16-byte pieces of a run's k and q
+    constexpr int VP = DN_RUN * COLS / N;
+    __shared__ __align__(16) float kq[2][DN_RUN][2][DN_D], vs[2][DN_RUN][COLS], gb[2][2][DN_RUN];
     const int h = blockIdx.x, jb = blockIdx.y;
     const int kh = h / (p.HV / p.HK);
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5, rg = lane >> 2, cg = lane & 3;
-    const int jl = warp * 8 + cg * 2; // this lane's first column of the slab
-    float* S = p.state + (size_t)h * DN_D * DN_D + (size_t)(4 * rg) * DN_D + jb * DN_COLS + jl;
+    const int jl = CL * (warp * 4 + cg); // this lane's first column of the CTA's
+    float* S = p.state + (size_t)h * DN_D * DN_D + (size_t)(4 * rg) * DN_D + jb * COLS + jl;
     const bool pairs = (reinterpret_cast<uintptr_t>(p.state) & 7) == 0;
 
     pdl_wait();
@@ -243,36 +247,121 @@ __device__ __forceinline__ void deltanet_body(const lb_deltanet_params& p, int n
     auto load = [&](int s0) { // this thread's pieces of tokens s0 .. s0 + DN_RUN - 1 (those that there are)
 #pragma unroll
         for (int i = 0; i < PER; ++i) {
-            const int e = i * DN_THREADS + t, tok = e / (2 * DN_D / N), which = (e / (DN_D / N)) & 1, c = e % (DN_D / N);
+            const int e = i * THREADS + t, tok = e / (2 * DN_D / N), which = (e / (DN_D / N)) & 1, c = e % (DN_D / N);
             if (s0 + tok < n_steps)
                 piece[i] = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(which ? p.q : p.k) + ((size_t)(s0 + tok) * p.HK + kh) * DN_D) + c);
         }
         if (t < VP) {
-            const int tok = t / (DN_COLS / N), c = t % (DN_COLS / N);
+            const int tok = t / (COLS / N), c = t % (COLS / N);
             if (s0 + tok < n_steps)
-                vpiece = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(p.v) + ((size_t)(s0 + tok) * p.HV + h) * DN_D + jb * DN_COLS) + c);
-        } else if (t >= DN_THREADS - 2 * DN_RUN) {
-            const int e = t - (DN_THREADS - 2 * DN_RUN), tok = e % DN_RUN;
+                vpiece = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(p.v) + ((size_t)(s0 + tok) * p.HV + h) * DN_D + jb * COLS) + c);
+        } else if (t >= THREADS - 2 * DN_RUN) {
+            const int e = t - (THREADS - 2 * DN_RUN), tok = e % DN_RUN;
             if (s0 + tok < n_steps) gpiece = __ldg((e < DN_RUN ? p.g : p.beta) + (size_t)(s0 + tok) * p.HV + h);
         }
     };
     auto store = [&](int st) {
 #pragma unroll
         for (int i = 0; i < PER; ++i) {
-            const int e = i * DN_THREADS + t;
+            const int e = i * THREADS + t;
             dn_in<T>::put(&kq[st][e / (2 * DN_D / N)][(e / (DN_D / N)) & 1][(e % (DN_D / N)) * N], piece[i]);
         }
-        if (t < VP) dn_in<T>::put(&vs[st][t / (DN_COLS / N)][(t % (DN_COLS / N)) * N], vpiece);
-        else if (t >= DN_THREADS - 2 * DN_RUN) gb[st][(t - (DN_THREADS - 2 * DN_RUN)) / DN_RUN][t % DN_RUN] = gpiece;
+        if (t < VP) dn_in<T>::put(&vs[st][t / (COLS / N)][(t % (COLS / N)) * N], vpiece);
+        else if (t >= THREADS - 2 * DN_RUN) gb[st][(t - (THREADS - 2 * DN_RUN)) / DN_RUN][t % DN_RUN] = gpiece;
     };
-    static_assert(VP <= DN_THREADS - 2 * DN_RUN && DN_THREADS % DN_RUN == 0, "threads for v, g and beta");
+    static_assert(VP <= THREADS - 2 * DN_RUN && THREADS % DN_RUN == 0, "threads for v, g and beta");
 #pragma unroll
     for (int i = 0; i < PER; ++i) piece[i] = make_uint4(0u, 0u, 0u, 0u);
     load(0);
-    uint64_t s[4][2][2]; // [run of 32 rows][rows 4 rg + (0, 1) / (2, 3) of it][column]
+    uint64_t s[4][2][CL]; // [run of 32 rows][rows 4 rg + (0, 1) / (2, 3) of it][column]
     dn_load_state(S, pairs, s);
     store(0);
     if (DN_RUN < n_steps) load(DN_RUN);
+
+    // sums of four tokens' read-outs over the eight row groups: lane rg is left with token (rg & 1) * 2 + (rg >> 1 & 1), column rg >> 2 of two (one: twice)
+    auto put_out = [&](float (&o)[4 * CL], int first) {
+#pragma unroll
+        for (int m = 1, len = 2 * CL; m < 8; m <<= 1, len >>= 1)
+#pragma unroll
+            for (int i = 0; i < 2 * CL; ++i) {
+                if (i < len) {
+                    const float give = rg & m ? o[i] : o[len + i], keep = rg & m ? o[len + i] : o[i];
+                    o[i] = keep + __shfl_xor_sync(0xffffffffu, give, 4 * m);
+                } else if (len == 0 && i == 0) o[0] += __shfl_xor_sync(0xffffffffu, o[0], 4 * m);
+            }
+        const int step = first + (rg & 1) * 2 + ((rg >> 1) & 1);
+        if (step < n_steps && (CL == 2 || rg < 4)) {
+            const size_t oi = ((size_t)step * p.HV + h) * DN_D + jb * COLS + jl + (CL == 2 ? rg >> 2 : 0);
+            float y = o[0];
+            if (p.z) y *= siluf_dev(p.z[oi]);
+            p.out[oi] = y;
+        }
+    };
+    auto values = [&](int st, int u, float (&v)[CL]) {
+        if (CL == 2) {
+            const float2 x = *reinterpret_cast<const float2*>(&vs[st][u][jl]);
+            v[0] = x.x;
+            v[CL - 1] = x.y;
+        } else v[0] = vs[st][u][jl];
+    };
+    auto run_full = [&](int st, int s0) {
+        uint64_t kk[4][2], qq[4][2];
+        dn_read(kq[st][0][0] + 4 * rg, kk);
+        float o[4 * CL], r[CL], v[CL], y[CL];
+#pragma unroll
+        for (int u = 0; u < DN_RUN; ++u) {
+            uint64_t kn[4][2];
+            dn_dot(kk, s, r); // recall from the old state
+            const float g = gb[st][0][u], beta = gb[st][1][u];
+            values(st, u, v);
+            if (u + 1 < DN_RUN) dn_read(kq[st][u + 1][0] + 4 * rg, kn);
+            if (u > 0) {
+                dn_dot(qq, s, y); // read-out of the token before
+#pragma unroll
+                for (int c = 0; c < CL; ++c) o[CL * ((u - 1) & 3) + c] = y[c];
+            }
+            dn_read(kq[st][u][1] + 4 * rg, qq);
+            dn_decay(g, s);
+            dn_reduce(r);
+            if (u == 4) put_out(o, s0);
+            dn_write(kk, beta, v, r, s);
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) kk[j][e] = kn[j][e];
+        }
+        dn_dot(qq, s, y);
+#pragma unroll
+        for (int c = 0; c < CL; ++c) o[CL * 3 + c] = y[c];
+        put_out(o, s0 + 4);
+    };
+    auto run_part = [&](int st, int s0) { // fewer than DN_RUN tokens
+#pragma unroll
+        for (int u0 = 0; u0 < DN_RUN; u0 += 4) {
+            if (s0 + u0 >= n_steps) break;
+            float o[4 * CL];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                float r[CL], v[CL], y[CL];
+#pragma unroll
+                for (int c = 0; c < CL; ++c) o[CL * u + c] = 0.f;
+                if (s0 + u0 + u >= n_steps) continue;
+                uint64_t kk[4][2], qq[4][2];
+                dn_read(kq[st][u0 + u][0] + 4 * rg, kk);
+                dn_read(kq[st][u0 + u][1] + 4 * rg, qq);
+                const float g = gb[st][0][u0 + u], beta = gb[st][1][u0 + u];
+                values(st, u0 + u, v);
+                dn_dot(kk, s, r);
+                dn_decay(g, s); // independent of the sum: in its shadow
+                dn_reduce(r);
+                dn_write(kk, beta, v, r, s);
+                dn_dot(qq, s, y);
+#pragma unroll
+                for (int c = 0; c < CL; ++c) o[CL * u + c] = y[c];
+            }
+            put_out(o, s0 + u0);
+        }
+    };
 
     for (int s0 = 0, st = 0; s0 < n_steps; s0 += DN_RUN, st ^= 1) {
         __syncthreads(); // the run's operands are visible, and everybody is done with the other stage
@@ -280,62 +369,24 @@ __device__ __forceinline__ void deltanet_body(const lb_deltanet_params& p, int n
             store(st ^ 1);
             if (s0 + 2 * DN_RUN < n_steps) load(s0 + 2 * DN_RUN);
         }
-#pragma unroll
-        for (int u0 = 0; u0 < DN_RUN; u0 += 4) {
-            if (s0 + u0 >= n_steps) break;
-            float o[8]; // read-outs of four tokens, two columns each: this lane's rows
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                o[2 * u] = o[2 * u + 1] = 0.f;
-                if (s0 + u0 + u >= n_steps) continue;
-                uint64_t kk[4][2], qq[4][2], a[2][2];
-                dn_read(kq[st][u0 + u][0] + 4 * rg, kk);
-                dn_read(kq[st][u0 + u][1] + 4 * rg, qq);
-                const float g = gb[st][0][u0 + u], beta = gb[st][1][u0 + u];
-                const float2 v = *reinterpret_cast<const float2*>(&vs[st][u0 + u][jl]);
-                dn_recall(kk, s, a);
-                float r0 = dn_sum4(a[0][0], a[0][1]), r1 = dn_sum4(a[1][0], a[1][1]);
-                dn_decay(g, s); // independent of the sums: in their shadow
-                dn_reduce(r0, r1);
-                dn_update(kk, qq, beta * (v.x - r0), beta * (v.y - r1), s, a);
-                o[2 * u] = dn_sum4(a[0][0], a[0][1]);
-                o[2 * u + 1] = dn_sum4(a[1][0], a[1][1]);
-            }
-            // sums over the eight row groups: lane rg is left with token (rg & 1) * 2 + (rg >> 1 & 1), column rg >> 2
-#pragma unroll
-            for (int m = 1, len = 4; m < 8; m <<= 1, len >>= 1)
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    if (i < len) {
-                        const float give = rg & m ? o[i] : o[len + i], keep = rg & m ? o[len + i] : o[i];
-                        o[i] = keep + __shfl_xor_sync(0xffffffffu, give, 4 * m);
-                    }
-            const int step = s0 + u0 + (rg & 1) * 2 + ((rg >> 1) & 1);
-            if (step < n_steps) {
-                const size_t oi = ((size_t)step * p.HV + h) * DN_D + jb * DN_COLS + jl + (rg >> 2);
-                float y = o[0];
-                if (p.z) y *= siluf_dev(p.z[oi]);
-                p.out[oi] = y;
-            }
-        }
+        if (s0 + DN_RUN <= n_steps) run_full(st, s0);
+        else run_part(st, s0);
     }
     pdl_launch_dependents();
     dn_store_state(S, pairs, s);
 }
 
-extern "C" __global__ void __launch_bounds__(DN_THREADS) deltanet_step_bf16(const __grid_constant__ lb_deltanet_params p,
-                                                                            int n_steps) {
-    deltanet_body<__nv_bfloat16>(p, n_steps);
-}
+// grid (HV, 4) / (HV, 8): 32 / 16 columns per CTA
+#define DN_RUNS(name, T, CL) \
+    extern "C" __global__ void __launch_bounds__(DN_THREADS) name(const __grid_constant__ lb_deltanet_params p, int n_steps) { deltanet_body<T, CL>(p, n_steps); }
+DN_RUNS(deltanet_step_bf16, __nv_bfloat16, 2)
+DN_RUNS(deltanet_step_f32, float, 2)
+DN_RUNS(deltanet_step16_bf16, __nv_bfloat16, 1)
+DN_RUNS(deltanet_step16_f32, float, 1)
 extern "C" __global__ void __launch_bounds__(DN_THREADS) deltanet_one_bf16(const __grid_constant__ lb_deltanet_params p) { deltanet_few<__nv_bfloat16, 1>(p); }
 extern "C" __global__ void __launch_bounds__(DN_THREADS) deltanet_one_f32(const __grid_constant__ lb_deltanet_params p) { deltanet_few<float, 1>(p); }
 extern "C" __global__ void __launch_bounds__(DN_THREADS) deltanet_two_bf16(const __grid_constant__ lb_deltanet_params p) { deltanet_few<__nv_bfloat16, 2>(p); }
 extern "C" __global__ void __launch_bounds__(DN_THREADS) deltanet_two_f32(const __grid_constant__ lb_deltanet_params p) { deltanet_few<float, 2>(p); }
-extern "C" __global__ void __launch_bounds__(DN_THREADS) deltanet_step_f32(const __grid_constant__ lb_deltanet_params p,
-                                                                           int n_steps) {
-    deltanet_body<float>(p, n_steps);
-}
-
 // g = exp(-exp(A_log) softplus(a + dt_bias)), beta = sigmoid(b); natural log
 // as in models/.../deltanet/unroll.ls (DecayGate: softplus = ln(1+e^x)).
 extern "C" __global__ void decay_gate_beta(const __grid_constant__ lb_decay_params p) {
