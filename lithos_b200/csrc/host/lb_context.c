@@ -127,7 +127,7 @@ static int load_cubin(lb_ctx* c, const char* dir, const char* file) {
     return LB_OK;
 }
 
-static const char* const k_cubins[] = {"gemv.cubin", "chain.cubin", "batched.cubin", "batched_tc.cubin", "deltanet.cubin", "attention.cubin", "attention_mma.cubin", "small.cubin", "comm.cubin", "prefill.cubin",
+static const char* const k_cubins[] = {"gemv.cubin", "chain.cubin", "batched.cubin", "batched_tc.cubin", "batched_ring.cubin", "deltanet.cubin", "attention.cubin", "attention_mma.cubin", "small.cubin", "comm.cubin", "prefill.cubin",
                                        "rows_gemv.cubin", "dense_gemm.cubin", "window_attention.cubin", "decay_attention.cubin",
                                        "latent_attention.cubin", "ssm.cubin"};
 

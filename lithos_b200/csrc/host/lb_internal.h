@@ -95,6 +95,8 @@ int lb_driver_load(char* err, size_t errlen); /* LB_OK or LB_ERR_NO_DRIVER */
     X(gemm_int4_tc_256)               \
     X(gemm_int4_tc_exact16)           \
     X(gemm_int4_tc_exact32)           \
+    X(gemm_int4_ring8)                \
+    X(gemm_int4_ring16)               \
     X(gptq_dequant_f32)               \
     X(gptq_unpack_u8)                 \
     X(dense_bf16_gemv)                \

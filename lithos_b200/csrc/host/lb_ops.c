@@ -264,6 +264,39 @@ static int exact_on_tc(lb_ctx* c, int B, int blocks, int groups) {
     return 1;
 }
 
+/* X [B, K] fp16, box = 64 k (128 bytes) x nt tokens, laid down with the 128-byte swizzle */
+static int map_tokens(lb_ctx* c, lb_bgemm_params* p, int nt) {
+    CUtensorMap tm;
+    cuuint64_t dims[2] = {(cuuint64_t)p->K, (cuuint64_t)p->B}, strides[1] = {(cuuint64_t)p->K * 2};
+    cuuint32_t box[2] = {64, (cuuint32_t)nt}, estr[2] = {1, 1};
+    LB_CU(c, lb_drv.TensorMapEncodeTiled(&tm, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, (void*)p->x, dims, strides, box, estr,
+                                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                                         CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE));
+    memcpy(p->tmap_x, &tm, sizeof tm);
+    return LB_OK;
+}
+
+/* gemm_int4_ring8 / 16 run 2 to 16 tokens at every size (us, the kernels before / ring: 5120 -> 17408 at 2 tokens 19.0 / 12.2, 12 24.4 / 15.2; 17408 -> 5120 28.2 / 15.4,
+ * 27.5 / 18.7; 1024 -> 1024 5.1 / 4.2, 5.7 / 4.8; 8192 -> 2048 9.6 / 6.7, 8.9 / 8.0), but for the sizes of 9 to 16 tokens whose rows keep the bits that
+ * LB_GEMM_MMA_SYNC gives: columns of at most 512, whole columns of at most 1024, and the long columns of which mma.sync makes more slices (8192 -> 7168 at 12
+ * tokens 19.6 / 14.1, 14336 -> 5888 31.8 / 21.1: slower, but the same rows as ever) */
+static int pinned_to_mma(lb_ctx* c, int B, int blocks, int groups) {
+    return B > 8 && !exact_on_tc(c, B, blocks, groups) && (2 * blocks <= c->sm_count || groups <= 8);
+}
+/* gemm_int4_ring8 / 16 */
+static int launch_ring(lb_ctx* c, lb_bgemm_params* p, int blocks, int groups) {
+    const int nt = p->B > 8 ? 16 : 8, ksplit = tc_slices(c, blocks, groups);
+    CUtensorMap tm; /* qweight as [N/32 column blocks][K/8 packed rows][32 columns] */
+    cuuint64_t dims[3] = {32, (cuuint64_t)(p->K / 8), (cuuint64_t)(p->N / 32)}, strides[2] = {(cuuint64_t)p->N * 4, 128};
+    cuuint32_t box[3] = {32, 16, 4}, estr[3] = {1, 1, 1};
+    LB_CU(c, lb_drv.TensorMapEncodeTiled(&tm, CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, (void*)p->qweight, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                         CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE));
+    memcpy(p->tmap_w, &tm, sizeof tm);
+    LB_TRY(map_tokens(c, p, nt));
+    void* params[] = {p};
+    return lb_launch_cluster(c, nt > 8 ? LBK_gemm_int4_ring16 : LBK_gemm_int4_ring8, (unsigned)blocks, (unsigned)ksplit, 1, LB_RING_THREADS, (unsigned)LB_RING_SMEM(nt), params, 1, (unsigned)ksplit);
+}
+
 LB_API int lb_gemm_int4(lb_ctx* c, uint64_t qweight, uint64_t scales, uint64_t qzeros, uint64_t x, uint64_t y, int K, int N,
                         int B, int flags) {
     if (!c || !qweight || !scales || !x || !y || K <= 0 || N <= 0 || K % 128 || N % 16 || B < 1 || B > LB_GEMM_MAX_BATCH ||
@@ -286,19 +319,13 @@ LB_API int lb_gemm_int4(lb_ctx* c, uint64_t qweight, uint64_t scales, uint64_t q
     if (x & 15) return lb_fail(c, LB_ERR_INVALID, "lb_gemm_int4: x must be 16-byte aligned");
     const int mma_ok = ((qweight & 7) | (scales & 3)) == 0; /* the mma.sync kernels load the words and scales of two columns at once */
     if ((flags & LB_GEMM_MMA_SYNC) && !mma_ok) return lb_fail(c, LB_ERR_INVALID, "lb_gemm_int4: LB_GEMM_MMA_SYNC wants qweight 8-byte and scales 4-byte aligned");
+    const int ring_ok = N % 32 == 0 && ((qweight | scales | qzeros) & 15) == 0; /* what its bulk copies want */
+    if (ring_ok && B > 1 && B <= 16 && !(flags & (LB_GEMM_MMA_SYNC | LB_GEMM_TCGEN05)) && !pinned_to_mma(c, B, blocks, groups)) return launch_ring(c, &p, blocks, groups);
     const int exact = B <= 32 && !(flags & (LB_GEMM_MMA_SYNC | LB_GEMM_TCGEN05)) && (!mma_ok || (B > 8 && exact_on_tc(c, B, blocks, groups)));
     if (exact || (B > 32 && !(flags & LB_GEMM_MMA_SYNC)) || (flags & LB_GEMM_TCGEN05)) {
         const int nt = exact ? (B > 16 ? 32 : 16) : LB_TC_NT(B), halves = nt > LB_TC_HALVES_FROM;
         const unsigned smem = halves ? (unsigned)(LB_TC_X_HALVES * nt * 128) : (unsigned)((exact ? 7 : LB_TC_STAGES(nt)) * nt * 256); /* activation stages; the partial tile [nt][132] fp32 fits over them */
-        CUtensorMap tm; /* X [B, K] fp16, box = 64 k (128 bytes) x NT tokens, laid down with the 128-byte swizzle */
-        cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)B};
-        cuuint64_t strides[1] = {(cuuint64_t)K * 2};
-        cuuint32_t box[2] = {64, (cuuint32_t)nt};
-        cuuint32_t estr[2] = {1, 1};
-        LB_CU(c, lb_drv.TensorMapEncodeTiled(&tm, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, (void*)x, dims, strides, box, estr,
-                                             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                                             CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE));
-        memcpy(p.tmap_x, &tm, sizeof tm);
+        LB_TRY(map_tokens(c, &p, nt));
         const int ksplit = tc_slices(c, blocks, groups);
         return lb_launch_cluster(c, exact ? (nt > 16 ? LBK_gemm_int4_tc_exact32 : LBK_gemm_int4_tc_exact16) : halves ? LBK_gemm_int4_tc_256 : LBK_gemm_int4_tc, (unsigned)blocks, (unsigned)ksplit, 1,
                                  exact ? (nt > 16 ? LB_TC_EXACT32_THREADS : LB_TC_EXACT16_THREADS) : LB_TC_THREADS, smem, params, 1, (unsigned)ksplit);

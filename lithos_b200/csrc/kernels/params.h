@@ -146,9 +146,14 @@ typedef struct {
 #define LB_TC_STAGES(nt) ((512 - ((nt) > 64 ? (nt) : 64)) / 64) /* weight stages of 64 columns beside the accumulator in tensor memory */
 #define LB_TC_HALVES_FROM 160           /* more tokens a product: gemm_int4_tc_256 (five whole stages of 160 tokens are 200 KB) */
 #define LB_TC_X_HALVES 7        /* gemm_int4_tc_256: 64-k halves of a K-group's activations in shared memory (32 KB each at 256 tokens) */
+#define LB_RING_THREADS 256     /* gemm_int4_ring*: eight warps */
+#define LB_RING_SLOTS(tok) ((tok) > 8 ? 17 : 21) /* K-groups in flight: 8 KB of words, 256 bytes per token, 320 of scales and zero-points */
+#define LB_RING_SMEM(tok) (LB_RING_SLOTS(tok) * (8192 + 256 * (tok) + 320))
 typedef struct {
     /* gemm_int4_tc: CUtensorMap over X [B, K] fp16, box 64 k x NT tokens, 128-byte swizzle */
     unsigned char tmap_x[128] __attribute__((aligned(64)));
+    /* gemm_int4_ring*: over qweight as [N/32 column blocks][K/8 packed rows][32 columns], box 4 x 16 x 32, 128-byte swizzle */
+    unsigned char tmap_w[128] __attribute__((aligned(64)));
     const uint32_t* qweight; /* [K/8, N] */
     const uint16_t* scales;  /* fp16 [K/128, N] */
     const uint32_t* qzeros;  /* [K/128, N/8] or NULL: zero-point 8 */
