@@ -692,8 +692,7 @@ static int hybrid_pf_layer(lb_model* m, pf_set* w, int l, int pos0, int T) {
         LB_TRY(lb_ac_fill(c, &maps, L->k_cache, kv_ld, 0, 0, 0, L->v_cache, kv_ld, 256, pos0 + T));
         void* params[] = {&p, &maps};
         LB_TRY(lb_launch(c, LBK_pf_attn_prepare, (unsigned)T, 1, 1, 256, 0, params, 1));
-        const int rows = T * (m->HQ / m->HKV);
-        LB_TRY(lb_launch(c, LBK_pf_attn_chunk, (unsigned)((rows + LB_AC_ROWS - 1) / LB_AC_ROWS), (unsigned)m->HKV, 1, LB_AC_THREADS, LB_AC_SMEM, params, 1));
+        LB_TRY(lb_ac_launch(c, LBK_pf_attn_chunk, LBK_pf_attn_merge, T * (m->HQ / m->HKV), m->HKV, pos0 + T, 256, w->hy.gu, (size_t)PF_CHUNK * 2 * m->inter_s * 4, &p, &maps));
     }
     LB_TRY(gemm(m, &L->w_out, w->hy.mix16, w->hy.y, T));
     /* MLP */

@@ -130,6 +130,7 @@ int lb_driver_load(char* err, size_t errlen); /* LB_OK or LB_ERR_NO_DRIVER */
     X(pf_add)                         \
     X(pf_attn_prepare)                \
     X(pf_attn_chunk)                  \
+    X(pf_attn_merge)                  \
     X(rows_gemv)                      \
     X(rows_gemv_rms)                  \
     X(rows_gemv_ln)                   \
@@ -158,6 +159,7 @@ int lb_driver_load(char* err, size_t errlen); /* LB_OK or LB_ERR_NO_DRIVER */
     X(wattn_chunk_128)                \
     X(wattn_chunk_256)                \
     X(wattn_chunk_tc)                 \
+    X(wattn_merge_tc)                 \
     X(da_step_64)                     \
     X(da_step_128)                    \
     X(da_step_256)                    \
@@ -265,6 +267,8 @@ int lb_launch_cluster(lb_ctx* c, int kernel, unsigned gx, unsigned gy, unsigned 
                       void** params, int pdl, unsigned cluster_y);
 /* tensor maps for the chunk attention on tcgen05: keys and values of rows 0..rows-1 */
 int lb_ac_fill(lb_ctx* c, lb_ac_maps* m, CUdeviceptr k, int k_ld, CUdeviceptr tail, int tail_w, int tail_ld, CUdeviceptr v, int v_ld, int vdim, int rows);
+/* its launch: rows query rows per KV head, keys the last of them sees; the parts' scratch of `bytes` bytes; params {kernel's own, maps}; + 1 entry for the split */
+int lb_ac_launch(lb_ctx* c, int kernel, int merge, int rows, int kv_heads, int keys, int vdim, CUdeviceptr scratch, size_t bytes, void* p, lb_ac_maps* maps);
 int lb_launch_pairs(lb_ctx* c, int kernel, unsigned pairs, unsigned bx, unsigned smem, void** params, int pdl);
 
 unsigned char* lb_map_file(const char* path, size_t* bytes); /* lb_safetensors.c: a whole file, read-only */

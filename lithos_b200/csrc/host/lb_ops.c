@@ -470,6 +470,25 @@ int lb_ac_fill(lb_ctx* c, lb_ac_maps* m, CUdeviceptr k, int k_ld, CUdeviceptr ta
     return ac_map(c, m->v, v, v_ld, v_ld, rows, 8192 / vdim);
 }
 
+/* Key blocks of a tile are dealt to several CTAs where the tiles of a launch leave half of the SMs idle or more: as many parts as make one wave, of two blocks at
+ * least (a part pays its queries' way in and its rows' way out). */
+int lb_ac_launch(lb_ctx* c, int kernel, int merge, int rows, int kv_heads, int keys, int vdim, CUdeviceptr scratch, size_t bytes, void* p, lb_ac_maps* maps) {
+    lb_ac_split sp;
+    memset(&sp, 0, sizeof sp);
+    sp.tiles = (rows + LB_AC_ROWS - 1) / LB_AC_ROWS;
+    sp.part = (float*)scratch;
+    const size_t one = (size_t)kv_heads * sp.tiles * LB_AC_ROWS * (vdim + 4) * 4;
+    int parts = c->sm_count / (sp.tiles * kv_heads);
+    if (parts > (keys + 127) / 256) parts = (keys + 127) / 256;
+    if (parts > 16) parts = 16;
+    if (one && (size_t)parts > bytes / one) parts = (int)(bytes / one);
+    sp.parts = parts > 1 ? parts : 1;
+    void* params[] = {p, maps, &sp};
+    LB_TRY(lb_launch(c, kernel, (unsigned)sp.tiles, (unsigned)kv_heads, (unsigned)sp.parts, LB_AC_THREADS, LB_AC_SMEM, params, 1));
+    if (sp.parts == 1) return LB_OK;
+    return lb_launch(c, merge, (unsigned)sp.tiles, (unsigned)kv_heads, (unsigned)(vdim / 32), 256, 0, params, 1);
+}
+
 LB_API int lb_rmsnorm(lb_ctx* c, uint64_t x, uint64_t res, uint64_t w, uint64_t y, uint64_t sum_out, int rows, int D,
                       float eps, int one_plus_w) {
     if (!c || !x || !w || !y || rows <= 0 || D <= 0) return lb_fail(c, LB_ERR_INVALID, "lb_rmsnorm: bad argument");

@@ -830,13 +830,13 @@ static void norm_adds(const lb_model* m, const pf_set* w, int i, lb_norm2_params
 static int has_experts(const stack_t* S, int i) { return i >= 0 && S->d.layer[i].ff && S->d.layer[i].ff_kind == LB_FF_EXPERTS; }
 
 /* a chunk's attention: on tcgen05 where heads are whole 64s of features, on mma.sync otherwise */
-static int launch_wattn_chunk(lb_ctx* c, lb_wattn_params* p) {
+static int launch_wattn_chunk(lb_ctx* c, lb_wattn_params* p, CUdeviceptr scratch, size_t bytes) { /* scratch: the projections' buffer, which nobody reads any more */
     const int rows = p->T * (p->H / p->KV), own = p->dim_p - p->tail_p;
     lb_ac_maps maps;
     void* params[] = {p, &maps};
     if (own % 64 == 0 && p->tail_p % 64 == 0 && p->dim_p <= 256 && (p->vdim_p == 64 || p->vdim_p == 128 || p->vdim_p == 256)) {
         LB_TRY(lb_ac_fill(c, &maps, (CUdeviceptr)p->k_cache, p->KV * own, (CUdeviceptr)p->k_tail, p->tail_p, p->tail_ld, (CUdeviceptr)p->v_cache, p->KV * p->vdim_p, p->vdim_p, p->pos0 + p->T));
-        return lb_launch(c, LBK_wattn_chunk_tc, (unsigned)((rows + LB_AC_ROWS - 1) / LB_AC_ROWS), (unsigned)p->KV, 1, LB_AC_THREADS, LB_AC_SMEM, params, 1);
+        return lb_ac_launch(c, LBK_wattn_chunk_tc, LBK_wattn_merge_tc, rows, p->KV, p->block > 0 && p->block < p->pos0 + p->T ? p->block : p->pos0 + p->T, p->vdim_p, scratch, bytes, p, &maps);
     }
     const unsigned smem = (unsigned)(2 * LB_WA_ROWS * (2 * p->dim_p + 16) + 2 * LB_WA_KV * (2 * p->dim_p + 2 * p->vdim_p + 32));
     return lb_launch(c, p->vdim_p <= 64 ? LBK_wattn_chunk_64 : p->vdim_p <= 128 ? LBK_wattn_chunk_128 : LBK_wattn_chunk_256,
@@ -872,7 +872,7 @@ static int pf_latent(lb_model* m, pf_set* w, int i, int pos0, int T) {
     a.sink = D->sink; a.sink_w = (const uint16_t*)L->sink; a.status = (uint32_t*)c->dev_status;
     a.H = a.KV = D->heads; a.dim = D->dim + D->rot_dim; a.dim_p = kd; a.vdim = D->vdim; a.vdim_p = L->vdim_p;
     a.pos0 = pos0; a.T = T; a.max_ctx = S->d.max_ctx; a.cat = (void*)w->st.cat; a.cat_ld = L->out.K;
-    return launch_wattn_chunk(c, &a);
+    return launch_wattn_chunk(c, &a, w->st.proj, (size_t)m->pf_chunk * S->max_in * 4);
 }
 
 static int pf_ssm(lb_model* m, pf_set* w, int i, int pos0, int T) {
@@ -966,7 +966,7 @@ static int stack_pf_layer(lb_model* m, pf_set* w, int i, int pos0, int T) {
         } else {
             p.qh = (uint16_t*)w->st.q; p.ql = (uint16_t*)w->st.k;
             LB_TRY(lb_launch(c, LBK_wattn_prepare_bf16, (unsigned)T, 1, 1, 256, 0, params, 1));
-            LB_TRY(launch_wattn_chunk(c, &p));
+            LB_TRY(launch_wattn_chunk(c, &p, w->st.proj, (size_t)m->pf_chunk * S->max_in * 4));
         }
     } else {
         lb_decay_params2 p;

@@ -8,6 +8,9 @@
 // tensor memory), so the scores of block i + 1 are made while block i is with the soft-max warps.
 // The maximum a row's probabilities refer to follows its running maximum only when that is more than 8 (in log2 units) ahead, and then the accumulator is
 // rescaled in tensor memory; sums of up to 256 x as large terms cost no precision in fp32, and almost no block rescales.
+// Few query rows behind many keys leave SMs idle: the key blocks of a tile are then dealt to `parts` CTAs (grid.z), which leave unnormalised rows, maxima and sums
+// in scratch, and attn_chunk_merge adds them in order (lb_ac_launch chooses; us: hybrid 75 tokens behind 2000 1625 -> 1545, 5 tokens 1102 -> 1003, Vobunex 100
+// behind 2000 930 -> 907, Nufalorn 150 behind 2000 1009 -> 984).
 // Every wait is bounded and reports through the status word; TMEM is freed on every path.
 // Bound by the products: 128 x 128 x 16 from shared memory takes about 107 cycles, 128 x 256 x 16 with P in tensor memory 138, so 128 keys of the hybrid's heads
 // (256 features) cost 5600 cycles and of 128-feature heads 2900; the soft-max warps need less.  Before (mma.sync, 16 query rows per warp, keys and values
@@ -53,9 +56,12 @@ struct ac_shared {
 // dim: features of a key, own of them at k[row][kv * own ..], the rest (shared by the KV heads) at tail[row][..]; multiples of 64.  vdim 64, 128 or 256.
 template <class C>
 __device__ __forceinline__ void attn_chunk_tc(const C& c, const lb_ac_maps& maps, ac_shared& sh, unsigned char* sm, int kv, int R0, int n_rows, int first_key, int last_key,
-                                              int dim, int own, int vdim, int units, uint32_t* status) {
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int n = (last_key - first_key) / AC_KEYS + 1, NB = vdim > 128 ? 2 : 3, kc = dim / 64, vu = vdim / 64, vr = 8192 / vdim;
+                                              int dim, int own, int vdim, int units, uint32_t* status, const lb_ac_split& sp) {
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, z = blockIdx.z;
+    const int blocks = (last_key - first_key) / AC_KEYS + 1, b0 = blocks * z / sp.parts, n = blocks * (z + 1) / sp.parts - b0; // n 0: a part without keys
+    first_key += b0 * AC_KEYS;
+    float* part = sp.parts > 1 ? sp.part + ((((size_t)kv * sp.tiles + R0 / AC_ROWS) * sp.parts + z) * AC_ROWS) * (vdim + 4) : nullptr; // [128][vdim | maximum, sum]
+    const int NB = vdim > 128 ? 2 : 3, kc = dim / 64, vu = vdim / 64, vr = 8192 / vdim;
     unsigned char* ring = sm + (size_t)2 * kc * AC_UNIT; // behind the queries: [2 terms][kc][128 rows][128 bytes], 128-byte swizzle
     if (tid == 0) {
         for (int s = 0; s < units; ++s) {
@@ -204,7 +210,7 @@ __device__ __forceinline__ void attn_chunk_tc(const C& c, const lb_ac_maps& maps
         const int quad = warp & 3, R = R0 + 32 * quad + lane, Rc = min(R, n_rows - 1);
         const uint32_t lanes = (uint32_t)(32 * quad) << 16;
         const int lim = c.lim(Rc), low = c.low(Rc);
-        float m = c.m0(Rc), l = c.l0();
+        float m = z == 0 ? c.m0(Rc) : -1e30f, l = z == 0 ? c.l0() : 0.f;
         bool ok = true;
         for (int i = 0; i < n; ++i) {
             const int b = i % NB, key0 = first_key + i * AC_KEYS;
@@ -267,20 +273,33 @@ __device__ __forceinline__ void attn_chunk_tc(const C& c, const lb_ac_maps& maps
             __syncwarp();
             if (lane == 0) mbar_arrive(&sh.p_ready[b]);
         }
-        if (ok) ok = __all_sync(0xffffffffu, tc_wait(&sh.pv_done[(n - 1) % NB], (uint32_t)((n - 1) / NB) & 1u));
+        if (ok && n > 0) ok = __all_sync(0xffffffffu, tc_wait(&sh.pv_done[(n - 1) % NB], (uint32_t)((n - 1) / NB) & 1u));
         tc_fence_after();
         pdl_launch_dependents();
         if (!ok && lane == 0 && status) atomicExch(status, AC_FAIL_SCORES);
         ok = __all_sync(0xffffffffu, ok);
-        c.table(sm, R0); // every product is done: queries and ring are free
-        asm volatile("bar.sync 2, 128;" ::: "memory");
+        float* mine = part ? part + (size_t)(32 * quad + lane) * (vdim + 4) : nullptr;
+        if (part) {
+            mine[vdim] = m;
+            mine[vdim + 1] = l;
+        } else {
+            c.table(sm, R0); // every product is done: queries and ring are free
+            asm volatile("bar.sync 2, 128;" ::: "memory");
+        }
         const float inv = 1.0f / l;
         for (int d = 0; d < vdim && ok; d += 16) {
             uint32_t r[16];
             __syncwarp(); // the stores before are some lanes' only
-            tmem_ld16(tmem_o + lanes + (uint32_t)d, r);
-            tmem_ld_wait();
-            if (R < n_rows) c.store(sm, R0, R, d, r, inv);
+            if (n > 0) {
+                tmem_ld16(tmem_o + lanes + (uint32_t)d, r);
+                tmem_ld_wait();
+            } else
+#pragma unroll
+                for (int j = 0; j < 16; ++j) r[j] = 0u;
+            if (part) {
+#pragma unroll
+                for (int j = 0; j < 16; j += 4) *reinterpret_cast<uint4*>(mine + d + j) = make_uint4(r[j], r[j + 1], r[j + 2], r[j + 3]);
+            } else if (R < n_rows) c.store(sm, R0, R, d, r, inv);
         }
         tc_fence_before();
     }
@@ -289,5 +308,33 @@ __device__ __forceinline__ void attn_chunk_tc(const C& c, const lb_ac_maps& maps
         __syncwarp();
         tc_fence_after();
         tmem_dealloc(tmem, 512);
+    }
+}
+
+// The parts of a tile, in order: grid (tiles, KV heads, 128 vdim / 4096), block 256, a thread 16 features of a row
+template <class C>
+__device__ __forceinline__ void attn_chunk_merge(const C& c, int kv, int n_rows, int vdim, const lb_ac_split& sp) {
+    pdl_wait();
+    const int per = vdim / 16, i = (int)blockIdx.z * 256 + threadIdx.x, row = i / per, d = 16 * (i - row * per), tile = (int)blockIdx.x, R = tile * AC_ROWS + row;
+    if (R < n_rows) {
+        const float* base = sp.part + ((((size_t)kv * sp.tiles + tile) * sp.parts) * AC_ROWS + row) * (vdim + 4);
+        const size_t step = (size_t)AC_ROWS * (vdim + 4);
+        float M = -INFINITY, L = 0.f, o[16];
+        for (int z = 0; z < sp.parts; ++z) M = fmaxf(M, base[z * step + vdim]);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) o[j] = 0.f;
+        for (int z = 0; z < sp.parts; ++z) {
+            const float w = exp2f(base[z * step + vdim] - M), l = base[z * step + vdim + 1];
+            L = fmaf(w, l, L);
+#pragma unroll
+            for (int j = 0; j < 16; j += 4) {
+                const float4 v = *reinterpret_cast<const float4*>(base + z * step + d + j);
+                o[j] = fmaf(w, v.x, o[j]); o[j + 1] = fmaf(w, v.y, o[j + 1]); o[j + 2] = fmaf(w, v.z, o[j + 2]); o[j + 3] = fmaf(w, v.w, o[j + 3]);
+            }
+        }
+        uint32_t r[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(o[j]);
+        c.store(nullptr, 0, R, d, r, 1.0f / L);
     }
 }

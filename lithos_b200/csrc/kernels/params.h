@@ -247,6 +247,10 @@ typedef struct {
     unsigned char tail[128] __attribute__((aligned(64))); /* ... the features that the KV heads share [rows, tail] ... */
     unsigned char v[128] __attribute__((aligned(64)));    /* ... and values [rows, KV heads * vdim], boxes of 64 features x 8192 / vdim rows */
 } lb_ac_maps;
+typedef struct {
+    float* part;    /* scratch [KV heads][tiles][parts][128][vdim + 4], unused with one part */
+    int32_t parts, tiles;
+} lb_ac_split;
 
 /* ---- GQA decode attention ------------------------------------------------- */
 typedef struct {

@@ -274,10 +274,14 @@ struct pf_chunk_rows {
         dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
     }
 };
-extern "C" __global__ void __launch_bounds__(LB_AC_THREADS, 1) pf_attn_chunk(const __grid_constant__ lb_pf_attn_params p, const __grid_constant__ lb_ac_maps maps) {
+extern "C" __global__ void __launch_bounds__(LB_AC_THREADS, 1) pf_attn_chunk(const __grid_constant__ lb_pf_attn_params p, const __grid_constant__ lb_ac_maps maps, const lb_ac_split sp) {
     extern __shared__ __align__(1024) unsigned char pa_sm[];
     __shared__ ac_shared sh;
     const int G = p.HQ / p.HKV, n_rows = p.T * G, R0 = (int)(gridDim.x - 1 - blockIdx.x) * AC_ROWS;
     const pf_chunk_rows c = {p, (int)blockIdx.y, G, p.qh, p.ql};
-    attn_chunk_tc(c, maps, sh, pa_sm, (int)blockIdx.y, R0, n_rows, 0, p.pos0 + min(R0 + AC_ROWS - 1, n_rows - 1) / G, AT_D, AT_D, AT_D, LB_AC_UNITS(AT_D), p.status);
+    attn_chunk_tc(c, maps, sh, pa_sm, (int)blockIdx.y, R0, n_rows, 0, p.pos0 + min(R0 + AC_ROWS - 1, n_rows - 1) / G, AT_D, AT_D, AT_D, LB_AC_UNITS(AT_D), p.status, sp);
+}
+extern "C" __global__ void __launch_bounds__(256) pf_attn_merge(const __grid_constant__ lb_pf_attn_params p, const __grid_constant__ lb_ac_maps, const lb_ac_split sp) {
+    const pf_chunk_rows c = {p, (int)blockIdx.y, p.HQ / p.HKV, p.qh, p.ql};
+    attn_chunk_merge(c, (int)blockIdx.y, p.T * c.G, AT_D, sp);
 }

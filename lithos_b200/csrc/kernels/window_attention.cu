@@ -530,7 +530,9 @@ struct wa_chunk_rows {
         for (int j = 0; j < 8; ++j) {
             float u = __uint_as_float(r[2 * j]) * inv, v = __uint_as_float(r[2 * j + 1]) * inv;
             if (p.freq_v && d + 2 * j + 1 < p.vdim) { // a value pair turns back by its token's position
-                const float2 cs = t[j];
+                float2 cs;
+                if (sm) cs = t[j];
+                else wa_angle(p.freq_v[d / 2 + j], p.pos0 + s, cs.x, cs.y);
                 const float a = u * cs.x + v * cs.y;
                 v = v * cs.x - u * cs.y;
                 u = a;
@@ -548,11 +550,15 @@ struct wa_chunk_rows {
         }
     }
 };
-extern "C" __global__ void __launch_bounds__(LB_AC_THREADS, 1) wattn_chunk_tc(const __grid_constant__ lb_wattn_params p, const __grid_constant__ lb_ac_maps maps) {
+extern "C" __global__ void __launch_bounds__(LB_AC_THREADS, 1) wattn_chunk_tc(const __grid_constant__ lb_wattn_params p, const __grid_constant__ lb_ac_maps maps, const lb_ac_split sp) {
     extern __shared__ __align__(1024) unsigned char wt_sm[];
     __shared__ ac_shared sh;
     const int G = p.H / p.KV, n_rows = p.T * G, R0 = (int)(gridDim.x - 1 - blockIdx.x) * AC_ROWS;
     const wa_chunk_rows c = {p, (int)blockIdx.y, G, p.qh, p.ql};
     attn_chunk_tc(c, maps, sh, wt_sm, (int)blockIdx.y, R0, n_rows, c.low(R0), c.lim(min(R0 + AC_ROWS - 1, n_rows - 1)), p.dim_p, p.dim_p - p.tail_p, p.vdim_p, LB_AC_UNITS(p.dim_p),
-                  p.status);
+                  p.status, sp);
+}
+extern "C" __global__ void __launch_bounds__(256) wattn_merge_tc(const __grid_constant__ lb_wattn_params p, const __grid_constant__ lb_ac_maps, const lb_ac_split sp) {
+    const wa_chunk_rows c = {p, (int)blockIdx.y, p.H / p.KV, p.qh, p.ql};
+    attn_chunk_merge(c, (int)blockIdx.y, p.T * c.G, p.vdim_p, sp);
 }

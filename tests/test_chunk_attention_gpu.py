@@ -40,3 +40,38 @@ def test_shared_key_part(ctx, lb, tmp_path, heads, dim, rot, vdim):
         TV.check(TV.feed(m, toks, cuts), want, "bfloat16", cuts)
     assert ctx.device_status() == 0
     m.close()
+
+
+@pytest.mark.parametrize("block", [700, 5000])
+def test_few_rows_behind_many_keys(ctx, lb, tmp_path, block):
+    """the keys of a tile of rows dealt to several CTAs: parts of unequal length, parts without visible keys (a window that begins far along)"""
+    c = TN.Case(tmp_path, ctx, C.config(96, 89, [C.att(4, 2, 128, 128, block, rot_dims=32), C.att(6, 2, 64, 64, block)]), 33)
+    n = 1500
+    toks = TN.tokens(c.cfg, n, 4)
+    want = c.want(toks)
+    m = c.open("bfloat16", n)
+    for cuts in ([1400, 2, 5, 33, 60], [695, 8, 300, 129, 368]):
+        m.reset_state()
+        TN.check(TN.feed(m, toks, cuts), want, "bfloat16", cuts)
+    assert ctx.device_status() == 0
+    m.close()
+
+
+def test_hybrid_few_rows_behind_many_keys(ctx, lb):
+    """the same for the int4 hybrid: portions of 1 to 40 tokens behind 900 give the logits of one prompt to the prompt's own tolerance (fp16 activations: 2e-3)"""
+    from lithos_b200 import model as M
+    cfg = M.tiny(max_ctx=1024)
+    m = M.Model(ctx, cfg)
+    m.fill_synthetic(9)
+    toks = np.random.default_rng(5).integers(0, cfg.vocab, 960).tolist()
+    want = m.forward(toks, 0, list(range(900, 960)))
+    m.reset_state()
+    m.forward(toks[:900], 0, [])
+    got, pos = [], 900
+    for n in (5, 2, 40, 13):
+        got.append(m.forward(toks[pos:pos + n], pos, list(range(n))))
+        pos += n
+    got = np.concatenate(got)
+    assert ctx.device_status() == 0
+    assert np.max(np.abs(got - want)) <= 4e-3 * np.max(np.abs(want))
+    m.close()
