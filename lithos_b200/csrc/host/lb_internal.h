@@ -265,6 +265,8 @@ int lb_launch(lb_ctx* c, int kernel, unsigned gx, unsigned gy, unsigned gz, unsi
               int pdl);
 int lb_launch_cluster(lb_ctx* c, int kernel, unsigned gx, unsigned gy, unsigned gz, unsigned bx, unsigned smem,
                       void** params, int pdl, unsigned cluster_y);
+/* lb_gemm_int4 of 33 tokens or more with an epilogue (LB_BG_*) */
+int lb_gemm_int4_epi(lb_ctx* c, uint64_t qweight, uint64_t scales, uint64_t qzeros, uint64_t x, uint64_t y, int K, int N, int B, int flags, int epi);
 /* tensor maps for the chunk attention on tcgen05: keys and values of rows 0..rows-1 */
 int lb_ac_fill(lb_ctx* c, lb_ac_maps* m, CUdeviceptr k, int k_ld, CUdeviceptr tail, int tail_w, int tail_ld, CUdeviceptr v, int v_ld, int vdim, int rows);
 /* its launch: rows query rows per KV head, keys the last of them sees; the parts' scratch of `bytes` bytes; params {kernel's own, maps}; + 1 entry for the split */

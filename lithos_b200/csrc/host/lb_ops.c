@@ -297,8 +297,7 @@ static int launch_ring(lb_ctx* c, lb_bgemm_params* p, int blocks, int groups) {
     return lb_launch_cluster(c, nt > 8 ? LBK_gemm_int4_ring16 : LBK_gemm_int4_ring8, (unsigned)blocks, (unsigned)ksplit, 1, LB_RING_THREADS, (unsigned)LB_RING_SMEM(nt), params, 1, (unsigned)ksplit);
 }
 
-LB_API int lb_gemm_int4(lb_ctx* c, uint64_t qweight, uint64_t scales, uint64_t qzeros, uint64_t x, uint64_t y, int K, int N,
-                        int B, int flags) {
+int lb_gemm_int4_epi(lb_ctx* c, uint64_t qweight, uint64_t scales, uint64_t qzeros, uint64_t x, uint64_t y, int K, int N, int B, int flags, int epi) {
     if (!c || !qweight || !scales || !x || !y || K <= 0 || N <= 0 || K % 128 || N % 16 || B < 1 || B > LB_GEMM_MAX_BATCH ||
         (flags & ~(LB_GEMV_Y_F32 | LB_GEMM_MMA_SYNC | LB_GEMM_TCGEN05)) ||
         ((flags & LB_GEMM_MMA_SYNC) && (flags & LB_GEMM_TCGEN05)) || ((flags & LB_GEMM_TCGEN05) && B <= 8) ||
@@ -309,7 +308,8 @@ LB_API int lb_gemm_int4(lb_ctx* c, uint64_t qweight, uint64_t scales, uint64_t q
     memset(&p, 0, sizeof p);
     p.qweight = (const uint32_t*)qweight; p.scales = (const uint16_t*)scales; p.qzeros = (const uint32_t*)qzeros;
     p.x = (const uint16_t*)x; p.y = (void*)y;
-    p.K = K; p.N = N; p.B = B; p.y_f32 = (flags & LB_GEMV_Y_F32) != 0;
+    p.K = K; p.N = N; p.B = B; p.y_f32 = (flags & LB_GEMV_Y_F32) != 0; p.epi = epi;
+    if (epi && (B <= 32 || (flags & ~LB_GEMV_Y_F32) || (epi == LB_BG_SWIGLU && N % 128))) return lb_fail(c, LB_ERR_INVALID, "lb_gemm_int4: an epilogue of the kernels of 33 tokens or more");
     p.status = (uint32_t*)c->dev_status;
     /* one token: the GEMV kernel (TMA-streamed, integer tensor-core products) is the faster path, with the same result type */
     if (B == 1 && !(flags & LB_GEMM_MMA_SYNC) && N % 32 == 0 && ((qweight | scales | qzeros | x | y) & 15ull) == 0)
@@ -324,9 +324,9 @@ LB_API int lb_gemm_int4(lb_ctx* c, uint64_t qweight, uint64_t scales, uint64_t q
     const int exact = B <= 32 && !(flags & (LB_GEMM_MMA_SYNC | LB_GEMM_TCGEN05)) && (!mma_ok || (B > 8 && exact_on_tc(c, B, blocks, groups)));
     if (exact || (B > 32 && !(flags & LB_GEMM_MMA_SYNC)) || (flags & LB_GEMM_TCGEN05)) {
         const int nt = exact ? (B > 16 ? 32 : 16) : LB_TC_NT(B), halves = nt > LB_TC_HALVES_FROM;
-        const unsigned smem = halves ? (unsigned)(LB_TC_X_HALVES * nt * 128) : (unsigned)((exact ? 7 : LB_TC_STAGES(nt)) * nt * 256); /* activation stages; the partial tile [nt][132] fp32 fits over them */
         LB_TRY(map_tokens(c, &p, nt));
         const int ksplit = tc_slices(c, blocks, groups);
+        const unsigned smem = halves ? (unsigned)(LB_TC_X_HALVES * nt * 128) : (unsigned)((exact ? 7 : LB_TC_STAGES(nt)) * nt * 256); /* activation stages; the partial tile [nt][132] fp32 fits over them */
         return lb_launch_cluster(c, exact ? (nt > 16 ? LBK_gemm_int4_tc_exact32 : LBK_gemm_int4_tc_exact16) : halves ? LBK_gemm_int4_tc_256 : LBK_gemm_int4_tc, (unsigned)blocks, (unsigned)ksplit, 1,
                                  exact ? (nt > 16 ? LB_TC_EXACT32_THREADS : LB_TC_EXACT16_THREADS) : LB_TC_THREADS, smem, params, 1, (unsigned)ksplit);
     }
@@ -335,6 +335,11 @@ LB_API int lb_gemm_int4(lb_ctx* c, uint64_t qweight, uint64_t scales, uint64_t q
     const unsigned smem = (unsigned)((B > 16 ? 3 : 4) * rows * 320); /* activation ring (the partial tile reuses it) */
     const int ksplit = mma_slices(c, blocks, groups);
     return lb_launch_cluster(c, kernel, (unsigned)blocks, (unsigned)ksplit, 1, 256, smem, params, 1, (unsigned)ksplit);
+}
+
+LB_API int lb_gemm_int4(lb_ctx* c, uint64_t qweight, uint64_t scales, uint64_t qzeros, uint64_t x, uint64_t y, int K, int N,
+                        int B, int flags) {
+    return lb_gemm_int4_epi(c, qweight, scales, qzeros, x, y, K, N, B, flags, LB_BG_STORE);
 }
 
 LB_API int lb_gptq_dequant(lb_ctx* c, uint64_t qweight, uint64_t scales, uint64_t qzeros, uint64_t w_out, int K, int N) {

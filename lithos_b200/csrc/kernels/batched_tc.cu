@@ -90,8 +90,19 @@ struct tc_group { // a thread's share of one K-group: the 16 packed words (8 k e
 #define TC_FAIL_FULL 0x1103u           // status: a stage was never filled
 
 __device__ __forceinline__ void tc_store_y(const lb_bgemm_params& p, size_t o, float v) {
-    if (p.y_f32) reinterpret_cast<float*>(p.y)[o] = v;
+    if (p.epi == LB_BG_ADD) reinterpret_cast<float*>(p.y)[o] += v;
+    else if (p.y_f32) reinterpret_cast<float*>(p.y)[o] = v;
     else reinterpret_cast<__half*>(p.y)[o] = __float2half_rn(v);
+}
+
+// a lane's four columns (lanes 0..15: gates, lanes 16..31: the ups that belong to them) of token b, SwiGLU: the whole warp together
+__device__ __forceinline__ void tc_store_glu(const lb_bgemm_params& p, int b, float4 v) {
+    const int lane = threadIdx.x & 31;
+    const float4 u = make_float4(__shfl_down_sync(0xffffffffu, v.x, 16), __shfl_down_sync(0xffffffffu, v.y, 16), __shfl_down_sync(0xffffffffu, v.z, 16), __shfl_down_sync(0xffffffffu, v.w, 16));
+    if (lane >= 16) return;
+    const __half2 lo = __floats2half2_rn(siluf_dev(v.x) * u.x, siluf_dev(v.y) * u.y), hi = __floats2half2_rn(siluf_dev(v.z) * u.z, siluf_dev(v.w) * u.w);
+    *reinterpret_cast<uint2*>(reinterpret_cast<__half*>(p.y) + (size_t)b * (p.N / 2) + (size_t)blockIdx.x * 64 + 4 * lane) =
+        make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
 }
 
 // SETS: converting sets of four warps (a set = the 128 columns); the exact kernels have fewer, their reading warps need the registers (spilling there cost
@@ -367,6 +378,7 @@ __device__ __forceinline__ void gemm_int4_tc_body(const lb_bgemm_params& p, unsi
             else if (live && j < p.B) tc_store_y(p, (size_t)j * p.N + n, sum[j]);
         }
     }
+    const bool glu = !EXACT && p.epi == LB_BG_SWIGLU, tiled = KS > 1 || glu; // through the tile in shared memory
     if (!failed && !EXACT && warp < CV_WARPS) {
         for (int c = warp >> 2; c < NT / 16; c += SETS) { // the sets share the tokens
             uint32_t r[16];
@@ -376,12 +388,17 @@ __device__ __forceinline__ void gemm_int4_tc_body(const lb_bgemm_params& p, unsi
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
                 const int b = c * 16 + j;
-                if (KS > 1) pt[b * TC_PSTRIDE + 32 * (warp & 3) + lane] = __uint_as_float(r[j]);
+                if (tiled) pt[b * TC_PSTRIDE + 32 * (warp & 3) + lane] = __uint_as_float(r[j]);
                 else if (live && b < p.B) tc_store_y(p, (size_t)b * p.N + n, __uint_as_float(r[j]));
             }
         }
     }
     tc_fence_before();
+    if (KS == 1 && glu) {
+        __syncthreads();
+        if (!failed)
+            for (int b = warp; b < p.B; b += (int)(blockDim.x >> 5)) tc_store_glu(p, b, *reinterpret_cast<const float4*>(pt + b * TC_PSTRIDE + 4 * lane));
+    }
     if (KS > 1) {
         tc_cluster_sync(); // every CTA of the cluster has its tile in place
         const int rank = (int)tc_cluster_rank();
@@ -395,7 +412,18 @@ __device__ __forceinline__ void gemm_int4_tc_body(const lb_bgemm_params& p, unsi
                     v.x += t.x; v.y += t.y; v.z += t.z; v.w += t.w;
                 }
                 const size_t o = (size_t)b * p.N + (size_t)blockIdx.x * TC_COLS + c;
-                if (wide) *reinterpret_cast<float4*>(reinterpret_cast<float*>(p.y) + o) = v;
+                if (glu) {
+                    tc_store_glu(p, b, v); // whole blocks of 128 columns: every lane is here
+                    continue;
+                }
+                if (wide) {
+                    float4* y = reinterpret_cast<float4*>(reinterpret_cast<float*>(p.y) + o);
+                    if (p.epi == LB_BG_ADD) {
+                        const float4 a = *y;
+                        v.x += a.x; v.y += a.y; v.z += a.z; v.w += a.w;
+                    }
+                    *y = v;
+                }
                 else {
                     tc_store_y(p, o, v.x); tc_store_y(p, o + 1, v.y); tc_store_y(p, o + 2, v.z); tc_store_y(p, o + 3, v.w);
                 }

@@ -162,8 +162,11 @@ typedef struct {
     int32_t K, N, B;
     int32_t y_f32;
     uint32_t* status; /* device status word for bounded waits (the host layer always passes the context's) */
-    int32_t reserved;
+    int32_t epi;      /* gemm_int4_tc, gemm_int4_tc_256: LB_BG_* */
 } lb_bgemm_params;
+enum { LB_BG_STORE = 0,
+       LB_BG_ADD = 1,      /* y (fp32) += */
+       LB_BG_SWIGLU = 2 }; /* columns in interleaved blocks of 64 gates and 64 ups (N % 128 == 0): fp16 y[B, N/2] = silu(gate) * up */
 
 /* ---- dense bf16 [N,K] x vector ------------------------------------------ */
 typedef struct {
