@@ -510,15 +510,21 @@ static int launch_rows(lb_model* m, lb_rows_gemv_params* p) {
 }
 
 /* Tokens per product tile, and what a product then costs in units of one wave of 256-token tiles: fewer tokens per tile make more tiles
- * for narrow matrices, at a lower rate per tile (measured: the operands' trip through shared memory bounds small tiles). */
+ * for narrow matrices, at a lower rate per tile (measured: the operands' trip through shared memory bounds small tiles); widths between the measured ones
+ * where they fit the tokens or the SMs better, by more than the costs are known to and more than the pairs of CTAs give that tiles of 256 run on (us, widths of
+ * powers of two only -> these: Nufalorn 1300 tokens 3483 -> 3389, 150 behind 2000 1036 -> 984, Vobunex 1500 behind 300 2325 -> 2228, 4001 5201 -> 5124). */
 static double product_cost(const lb_ctx* c, int row_tiles, int T, int* nt_out) {
-    static const struct { int nt; double cost; } k[] = {{256, 1.0}, {128, 0.55}, {64, 0.38}, {32, 0.34}, {16, 0.33}};
+    static const struct { int nt; double cost; } k[] = {{16, 0.33}, {32, 0.34}, {64, 0.38}, {128, 0.55}, {256, 1.0}};
     double best = 1e30;
-    for (int i = 0; i < 5; i++) {
-        const int tiles = row_tiles * ((T + k[i].nt - 1) / k[i].nt);
-        const double v = (double)((tiles + c->sm_count - 1) / c->sm_count) * k[i].cost;
-        if (v < best) { best = v; *nt_out = k[i].nt; }
-    }
+    for (int step = 0; step < 2; step++)
+        for (int i = 4, nt = 256; nt >= 16; nt -= step ? 16 : 1) {
+            while (i > 0 && nt < k[i].nt) i--;
+            if (!step && nt != k[i].nt) continue;
+            const double w = nt == k[i].nt ? k[i].cost : k[i].cost + (k[i + 1].cost - k[i].cost) * (nt - k[i].nt) / (k[i + 1].nt - k[i].nt);
+            const int tiles = row_tiles * ((T + nt - 1) / nt);
+            const double v = (double)((tiles + c->sm_count - 1) / c->sm_count) * w;
+            if (v < (step ? 0.94 : 1.0) * best) { best = v; *nt_out = nt; }
+        }
     return best;
 }
 
