@@ -123,8 +123,8 @@ int lb_driver_load(char* err, size_t errlen); /* LB_OK or LB_ERR_NO_DRIVER */
     X(pf_embed)                       \
     X(pf_rmsnorm_f16)                 \
     X(pf_dn_frontend)                 \
-    X(pf_dn_ring)                     \
     X(pf_ab_gate)                     \
+    X(pf_ab_gate_few)                 \
     X(pf_headnorm_gate_f16)           \
     X(pf_swiglu_f16)                  \
     X(pf_add)                         \

@@ -9,8 +9,17 @@
 // X[t, :] = float(E[token[t], :])                                   grid T, block 256
 extern "C" __global__ void pf_embed(const uint16_t* __restrict__ table, const int* __restrict__ tokens, float* __restrict__ X, int D) {
     pdl_wait(); // launched with programmatic stream serialization: nothing of the previous kernel is read before this
-    const size_t src = (size_t)tokens[blockIdx.x] * D, dst = (size_t)blockIdx.x * D;
-    for (int i = threadIdx.x; i < D; i += blockDim.x) X[dst + i] = bf16_bits_to_f32(table[src + i]);
+    const uint16_t* src = table + (size_t)tokens[blockIdx.x] * D;
+    float* dst = X + (size_t)blockIdx.x * D;
+    if ((D & 7) == 0 && (reinterpret_cast<uintptr_t>(table) & 15) == 0) { // whole 16-byte pieces
+        for (int i = threadIdx.x; i < D / 8; i += blockDim.x) {
+            const uint4 u = __ldg(reinterpret_cast<const uint4*>(src) + i);
+            reinterpret_cast<float4*>(dst)[2 * i] = make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u), __uint_as_float(u.y << 16), __uint_as_float(u.y & 0xffff0000u));
+            reinterpret_cast<float4*>(dst)[2 * i + 1] = make_float4(__uint_as_float(u.z << 16), __uint_as_float(u.z & 0xffff0000u), __uint_as_float(u.w << 16), __uint_as_float(u.w & 0xffff0000u));
+        }
+        return;
+    }
+    for (int i = threadIdx.x; i < D; i += blockDim.x) dst[i] = bf16_bits_to_f32(src[i]);
 }
 
 // [x[t, :] += add[t, :] when add is given;]  y16[t, :] = fp16( x[t, :] * rsqrt(mean x^2 + eps) * (1 + w) )
@@ -48,7 +57,7 @@ extern "C" __global__ void __launch_bounds__(256) pf_rmsnorm_f16(float* __restri
 // The DeltaNet front end of a chunk: causal 4-tap convolution over time, SiLU, per-head L2 norm of q and k, q / sqrt(128).
 // One block per (token, head of q, k or v): grid (T, 2*HK + HV), thread = channel.  The three earlier tokens of a channel are
 // rows of the same projection buffer, or, before the chunk's first token, slots of the ring history (slot = position & 3),
-// which this kernel only reads: pf_dn_ring records the chunk's last positions afterwards.
+// which this kernel only reads: pf_ab_gate records the chunk's last positions afterwards.
 // proj [T, ld]: q | k | v | z columns of the fused projection.  Writes q, k [T, HK, 128], v [T, HV, 128] (fp32).
 //                                                                        (inference/recur.ls:12-40, reduce.ls:153-207)
 extern "C" __global__ void __launch_bounds__(128) pf_dn_frontend(const float* __restrict__ proj, int ld, const uint16_t* __restrict__ conv_w,
@@ -77,70 +86,122 @@ extern "C" __global__ void __launch_bounds__(128) pf_dn_frontend(const float* __
     else k[((size_t)s * HK + head) * 128 + t] = y * rsqrtf(n2);
 }
 
-// ring[(pos0 + s) & 3][c] = proj[s][c] for the chunk's last (up to four) tokens: the history the next chunk, or the decode
-// step, continues from.  grid ceil(C / 256), block 256
-extern "C" __global__ void pf_dn_ring(const float* __restrict__ proj, int ld, float* __restrict__ ring, int C, int pos0, int T) {
-    pdl_wait(); // launched with programmatic stream serialization: nothing of the previous kernel is read before this
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= C) return;
-    for (int s = T > 4 ? T - 4 : 0; s < T; ++s) ring[(size_t)((pos0 + s) & 3) * C + c] = proj[(size_t)s * ld + c];
-}
-
 // decay and beta of a chunk: a = in_proj_a . xn, b = in_proj_b . xn per value head, then
-// g = exp(-exp(A_log) softplus(a + dt_bias)), beta = sigmoid(b).  A block owns one head and 8 consecutive tokens (the two
-// weight rows are read once per 8 tokens); its four warps take a quarter of the hidden dimension each and the quarters are
-// added in warp order.  grid (ceil(T/8), HV), block 128; H a multiple of 8.
-extern "C" __global__ void __launch_bounds__(128) pf_ab_gate(const __half* __restrict__ xn, const uint16_t* __restrict__ proj_a,
-                                                             const uint16_t* __restrict__ proj_b, const float* __restrict__ a_log,
-                                                             const uint16_t* __restrict__ dt_bias, float* __restrict__ g,
-                                                             float* __restrict__ beta, int HV, int H, int T) {
+// g = exp(-exp(A_log) softplus(a + dt_bias)), beta = sigmoid(b).  A block is 16 tokens x 8 NT of the 2 HV rows (a's, then b's), its eight warps take the hidden
+// dimension in turn, 32 at a time, U (even) of those in flight.  The products are mma.sync m16n8k8 tf32, in which fp16 activations and
+// bf16 weights are exact (sums fp32): a lane's 16-byte pieces of a token and of a row are its operands of four k-steps, the order of k being free.  The tensor core
+// truncates its sums, so chains of two products start from zero and are added pairwise: as far from 64 bits as the fp32 multiply-adds before (48 heads, 5120: g 2.1e-7
+// against 2.2e-7 rms, beta 1.2e-7 against 1.3e-7; one chain over all k was ten times as far off).
+// Bound by the loads' way in.  Before, one head x 8 tokens per block read the tokens 48 times.  NT = 3 reads them less often, NT = 1 makes three times the blocks and
+// keeps the SMs busy with a few tokens (the launch decides).  48 heads, hidden 5120, us, before -> after: 16 tokens 8.3 -> 8.3, 75 9.5 -> 8.3, 128 12.3 -> 8.3,
+// 256 17.0 -> 10.3; with the ring's launch gone, whole prompts: 4096 tokens 33 090 -> 32 350, 800 behind 500 7400 -> 7240, 75 behind 2000 1517 -> 1492.
+// Besides, the ring slots of the chunk's last (up to four) tokens, ring[(pos0 + s) & 3][c] = proj[s][c]: the history the next chunk, or the decode step, continues
+// from (pf_dn_frontend, the launch before, has read what was there).
+// grid (ceil(T / 16), ceil(2 HV / (8 NT))), block 256; H a multiple of 8
+__device__ __forceinline__ uint4 pf_ld16(const uint4* a) { // volatile: all loads of a stretch are issued before the first is used
+    uint4 v;
+    asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(a) : "memory");
+    return v;
+}
+template <int NT, int U>
+__device__ __forceinline__ void pf_ab_gate_body(const __half* __restrict__ xn, const uint16_t* __restrict__ proj_a, const uint16_t* __restrict__ proj_b, const float* __restrict__ a_log,
+                                                const uint16_t* __restrict__ dt_bias, float* __restrict__ g, float* __restrict__ beta, int HV, int H, int T,
+                                                const float* __restrict__ proj, int ld, float* __restrict__ ring, int C, int pos0) {
     pdl_wait(); // launched with programmatic stream serialization: nothing of the previous kernel is read before this
-    __shared__ float red[4][16];
-    const int s0 = blockIdx.x * 8, h = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint4* ra = reinterpret_cast<const uint4*>(proj_a + (size_t)h * H);
-    const uint4* rb = reinterpret_cast<const uint4*>(proj_b + (size_t)h * H);
-    float a[8], b[8];
+    __shared__ float red[8][16][8 * NT + 1];
+    const int s0 = blockIdx.x * 16, r0 = blockIdx.y * (8 * NT), t = threadIdx.x, warp = t >> 5, lane = t & 31, fg = lane >> 2, ft = lane & 3;
+    const uint4* x[2];
+    const uint4* w[NT];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) a[j] = b[j] = 0.f;
-    const int n8 = H / 8, per = (n8 + 3) / 4;
-    for (int i = warp * per + lane; i < min(n8, (warp + 1) * per); i += 32) {
-        const uint4 wa = __ldg(ra + i), wb = __ldg(rb + i);
-        const uint32_t aw[4] = {wa.x, wa.y, wa.z, wa.w}, bw[4] = {wb.x, wb.y, wb.z, wb.w};
+    for (int i = 0; i < 2; ++i) x[i] = reinterpret_cast<const uint4*>(xn + (size_t)min(s0 + fg + 8 * i, T - 1) * H) + ft; // tokens past the chunk repeat the last one
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int s = min(s0 + j, T - 1); // tokens past the chunk repeat the last one; they are not stored
-            const uint4 xx = *(reinterpret_cast<const uint4*>(xn + (size_t)s * H) + i);
-            const uint32_t xw[4] = {xx.x, xx.y, xx.z, xx.w};
+    for (int i = 0; i < NT; ++i) {
+        const int r = min(r0 + 8 * i + fg, 2 * HV - 1);
+        w[i] = reinterpret_cast<const uint4*>(r < HV ? proj_a + (size_t)r * H : proj_b + (size_t)(r - HV) * H) + ft;
+    }
+    float acc[NT][4];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const float2 xf = __half22float2(*reinterpret_cast<const __half2*>(&xw[q]));
-                a[j] = fmaf(__uint_as_float(aw[q] << 16), xf.x, a[j]);
-                a[j] = fmaf(__uint_as_float(aw[q] & 0xffff0000u), xf.y, a[j]);
-                b[j] = fmaf(__uint_as_float(bw[q] << 16), xf.x, b[j]);
-                b[j] = fmaf(__uint_as_float(bw[q] & 0xffff0000u), xf.y, b[j]);
-            }
+    for (int i = 0; i < NT; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+    const int pieces = H / 8;
+    for (int j0 = 4 * warp; j0 < pieces; j0 += 32 * U) {
+        uint4 xv[U][2], wv[U][NT];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int j = j0 + 32 * u;
+            const bool in = j + ft < pieces;
+#pragma unroll
+            for (int i = 0; i < 2; ++i) xv[u][i] = pf_ld16(x[i] + (in ? j : -ft));
+#pragma unroll
+            for (int i = 0; i < NT; ++i) wv[u][i] = pf_ld16(w[i] + (in ? j : -ft));
         }
+#pragma unroll
+        for (int u = 0; u < U; ++u) // past the end: zeros
+            if (j0 + 32 * u + ft >= pieces) {
+                xv[u][0] = xv[u][1] = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+                for (int i = 0; i < NT; ++i) wv[u][i] = make_uint4(0u, 0u, 0u, 0u);
+            }
+        float sum[NT][4], pair[NT][4], part[NT][4], stretch[NT][4]; // chains of two products, added pairwise
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int s = 0; s < 4; ++s) { // a k-step: two of the lane's eight k
+                float2 a[2];
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const uint32_t h = s == 0 ? xv[u][i].x : s == 1 ? xv[u][i].y : s == 2 ? xv[u][i].z : xv[u][i].w;
+                    a[i] = __half22float2(*reinterpret_cast<const __half2*>(&h));
+                }
+#pragma unroll
+                for (int i = 0; i < NT; ++i) {
+                    const uint32_t b = s == 0 ? wv[u][i].x : s == 1 ? wv[u][i].y : s == 2 ? wv[u][i].z : wv[u][i].w;
+                    if (s % 2 == 0) part[i][0] = part[i][1] = part[i][2] = part[i][3] = 0.f;
+                    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                        : "+f"(part[i][0]), "+f"(part[i][1]), "+f"(part[i][2]), "+f"(part[i][3])
+                        : "r"(__float_as_uint(a[0].x)), "r"(__float_as_uint(a[1].x)), "r"(__float_as_uint(a[0].y)), "r"(__float_as_uint(a[1].y)), "r"(b << 16), "r"(b & 0xffff0000u));
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        if (s == 1) pair[i][e] = part[i][e];
+                        if (s != 3) continue;
+                        const float v = pair[i][e] + part[i][e];
+                        if (u % 2 == 0) stretch[i][e] = v;
+                        else sum[i][e] = u == 1 ? stretch[i][e] + v : sum[i][e] + (stretch[i][e] + v);
+                        if (u == U - 1) acc[i][e] += sum[i][e];
+                    }
+                }
+            }
     }
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        a[j] = warp_sum(a[j]);
-        b[j] = warp_sum(b[j]);
-        if (lane == 0) {
-            red[warp][j] = a[j];
-            red[warp][8 + j] = b[j];
-        }
+    for (int i = 0; i < NT; ++i) {
+        red[warp][fg][8 * i + 2 * ft] = acc[i][0];
+        red[warp][fg][8 * i + 2 * ft + 1] = acc[i][1];
+        red[warp][fg + 8][8 * i + 2 * ft] = acc[i][2];
+        red[warp][fg + 8][8 * i + 2 * ft + 1] = acc[i][3];
     }
     __syncthreads();
-    const int j = threadIdx.x;
-    if (j < 8 && s0 + j < T) {
-        const float av = (red[0][j] + red[1][j]) + (red[2][j] + red[3][j]);
-        const float bv = (red[0][8 + j] + red[1][8 + j]) + (red[2][8 + j] + red[3][8 + j]);
-        const float tt = av + bf16_bits_to_f32(dt_bias[h]);
-        const float sp = tt > 20.f ? tt : log1pf(expf(tt));
-        g[(size_t)(s0 + j) * HV + h] = expf(-expf(a_log[h]) * sp);
-        beta[(size_t)(s0 + j) * HV + h] = 1.0f / (1.0f + expf(-bv));
+    for (int e = t; e < 16 * 8 * NT; e += 256) {
+        const int s = e / (8 * NT), c = e - 8 * NT * s, r = r0 + c;
+        if (s0 + s >= T || r >= 2 * HV) continue;
+        const float v = ((red[0][s][c] + red[1][s][c]) + (red[2][s][c] + red[3][s][c])) + ((red[4][s][c] + red[5][s][c]) + (red[6][s][c] + red[7][s][c]));
+        if (r < HV) {
+            const float tt = v + bf16_bits_to_f32(dt_bias[r]);
+            const float sp = tt > 20.f ? tt : log1pf(expf(tt));
+            g[(size_t)(s0 + s) * HV + r] = expf(-expf(a_log[r]) * sp);
+        } else beta[(size_t)(s0 + s) * HV + r - HV] = 1.0f / (1.0f + expf(-v));
+    }
+    const int last = T > 4 ? T - 4 : 0, blocks = gridDim.x * gridDim.y;
+    for (int i = (blockIdx.y * gridDim.x + blockIdx.x) * 256 + t; i < (T - last) * C; i += blocks * 256) {
+        const int s = last + i / C, c = i % C;
+        ring[(size_t)((pos0 + s) & 3) * C + c] = proj[(size_t)s * ld + c];
     }
 }
+#define PF_AB_GATE(name, NT, U)                                                                                                                                            \
+    extern "C" __global__ void __launch_bounds__(256) name(const __half* xn, const uint16_t* proj_a, const uint16_t* proj_b, const float* a_log, const uint16_t* dt_bias,     \
+                                                           float* g, float* beta, int HV, int H, int T, const float* proj, int ld, float* ring, int C, int pos0) {          \
+        pf_ab_gate_body<NT, U>(xn, proj_a, proj_b, a_log, dt_bias, g, beta, HV, H, T, proj, ld, ring, C, pos0);                                                           \
+    }
+PF_AB_GATE(pf_ab_gate, 3, 4)
+PF_AB_GATE(pf_ab_gate_few, 1, 10)
 
 // y16[t, h, :] = fp16( o * rsqrt(mean_head o^2 + eps) * w * silu(z) ): the out projection's input.  One warp per (token, head).
 // o [T, HV, 128]; z = proj + z_off with row stride ld.            grid (T, ceil(HV/4)), block 128
