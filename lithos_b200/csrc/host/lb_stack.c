@@ -28,7 +28,7 @@
 #define ST_LAT_ABSORB 16 /* latent attention: portions of fewer tokens do not make keys and values of every cached position */
 #define ST_MOE_TILE 64 /* token tile of the fp32 expert products */
 #define ST_SSM_SEGS 8  /* most segments of a chunk through a state-space recurrence */
-#define ST_SEG 128     /* tokens of a chunk a recurrence walks one after the other; segments run side by side */
+#define ST_SEG 128     /* a chunk's segments through a recurrence that run side by side: one per so many tokens of the largest chunk at most */
 
 typedef struct {
     CUdeviceptr w;
@@ -984,9 +984,18 @@ static int stack_pf_layer(lb_model* m, pf_set* w, int i, int pos0, int T) {
         const int part = L->dk_p / 16, tok = 3 * 16 * (part == 4 ? 4 : part + 4) + 64; /* floats a token's operands take in a stage */
         const int dki = L->dk_p == 64 ? 0 : L->dk_p == 128 ? 1 : 2;
         static const int k_scan[3] = {LBK_da_scan_64, LBK_da_scan_128, LBK_da_scan_256}, k_local[3] = {LBK_da_local_64, LBK_da_local_128, LBK_da_local_256};
-        const unsigned slabs = (unsigned)((D->vdim + 63) / 64), threads = dki == 2 ? 256 : 128, smem = (unsigned)(3 * 4 * tok * 4), segs = (unsigned)((T + ST_SEG - 1) / ST_SEG);
-        p.seg = ST_SEG; p.seg_state = (float*)w->st.seg_state; p.seg_decay = (float*)w->st.seg_decay;
-        if (segs > 1) LB_TRY(lb_launch(c, k_local[dki], (unsigned)D->heads, slabs, segs, threads, smem, params, 1));
+        const unsigned slabs = (unsigned)((D->vdim + 63) / 64), threads = dki == 2 ? 256 : 128, smem = (unsigned)(3 * 4 * tok * 4);
+        /* As many segments side by side as CTAs fit on the SMs at a time (registers: three, or one of 256 rows), of 16 tokens at least.  Nufalorn prompts, us with 1 / 2 / 4 / 6 / 8
+         * segments a chunk: 3000 tokens 7120 / 6870 / 6600 / 6605 / 6650, 300 tokens 1197 / 1141 / 1112 / 1105 / 1115, 150 tokens 922 / 917 / 871 / 862 / 873 (segments of 128
+         * tokens, a ninth of them in a second wave: 6930, 1210, 1000) */
+        int P = c->sm_count * (dki == 2 ? 1 : 3) / (int)((unsigned)D->heads * slabs);
+        if (P > (T + 15) / 16) P = (T + 15) / 16;
+        if (P > (m->pf_chunk + ST_SEG - 1) / ST_SEG) P = (m->pf_chunk + ST_SEG - 1) / ST_SEG; /* the workspace */
+        if (P < 1) P = 1;
+        p.seg = pad_to((T + P - 1) / P, 4); /* whole stages: what the last one reads past the chunk is less than a stage */
+        const unsigned segs = (unsigned)((T + p.seg - 1) / p.seg);
+        p.seg_state = (float*)w->st.seg_state; p.seg_decay = (float*)w->st.seg_decay;
+        if (segs > 1) LB_TRY(lb_launch(c, k_local[dki], (unsigned)D->heads, slabs, segs - 1, threads, smem, params, 1));
         LB_TRY(lb_launch(c, k_scan[dki], (unsigned)D->heads, slabs, segs, threads, smem, params, 1));
         LB_TRY(lb_launch(c, LBK_da_finish, (unsigned)T, (unsigned)((D->heads + 3) / 4), 1, 128, 0, params, 1));
     }
@@ -1183,7 +1192,7 @@ static int stack_build(lb_model* m, const lb_stack_desc* d, lb_weight_source* sr
             MAX(groups_max, groups);
         } else {
             MAX(S->max_dk, D->heads * L->dk_p);
-            MAX(S->max_state, state_bytes(D));
+            MAX(S->max_state, (size_t)D->heads * ((D->vdim + 63) / 64) * 64 * L->dk_p * 4); /* whole tiles */
             MAX(S->max_o, D->heads * D->vdim);
         }
 #undef MAX

@@ -169,9 +169,10 @@ __device__ __forceinline__ da_f2 da_mul2(da_f2 a, da_f2 b) {
 struct __align__(16) da_quad { da_f2 lo, hi; }; // four consecutive rows
 
 // Segments (gridDim.z = P > 1; segment g is tokens g * seg .. of the chunk).  The state after a segment is diag(b) S_in + L, b the product
-// of its decays and L what it makes of a zero state.  LOCAL (first launch): every segment leaves L and b in the workspace; segment 0 starts
-// from the sequence's state, so its L is a true state.  Second launch: segment g makes its S_in from the L and b of those before it, then runs
-// with read-outs; segment 0, the only one that touches the sequence's state, replaces it by the state after the last segment.
+// of its decays and L what it makes of a zero state.  LOCAL (first launch, P - 1 segments): every segment leaves L and b in the workspace; segment 0 starts
+// from the sequence's state, so its L is a true state, and keeps the sequence's state in the workspace's last place.  Second launch: segment g makes its S_in
+// from the L and b of those before it, then runs with read-outs; the last one leaves the sequence's state.
+// A workspace in the state's own layout took 64 loads of 4 bytes a thread and segment, 32 sectors each.
 template <int R, int C, bool LOCAL>
 __device__ __forceinline__ void da_scan_body(const lb_decay_params2& p) {
     constexpr int DA_SCAN_THREADS = 16 * DA_SLAB / C;
@@ -180,9 +181,9 @@ __device__ __forceinline__ void da_scan_body(const lb_decay_params2& p) {
     constexpr int NI = (DA_U * PIECES + DA_SCAN_THREADS - 1) / DA_SCAN_THREADS;
     extern __shared__ __align__(16) float da_sm[]; // [DA_AHEAD][DA_U][TOK]
     const int h = blockIdx.x, t = threadIdx.x, e = t & 15, cg = t >> 4, j = blockIdx.y * DA_SLAB + C * cg;
-    const int g = blockIdx.z, P = gridDim.z, tok0 = g * p.seg, n_tok = min(p.seg, p.T - tok0), n_st = (n_tok + DA_U - 1) / DA_U;
+    const int g = blockIdx.z, P = LOCAL ? gridDim.z + 1 : gridDim.z, tok0 = g * p.seg, n_tok = min(p.seg, p.T - tok0), n_st = (n_tok + DA_U - 1) / DA_U;
     const int rows = min(R, p.dk - e * R), cols = min(C, p.dv - j); // what of this thread's tile exists
-    const size_t head_off = ((size_t)h * p.dk + (size_t)e * R) * p.dv + j, all = (size_t)p.H * p.dk * p.dv; // this thread's corner of a state
+    const size_t head_off = ((size_t)h * p.dk + (size_t)e * R) * p.dv + j; // this thread's corner of a state
     pdl_wait();
     // operands: a thread copies the same pieces of every stage, so only the source moves on.  A last stage reads past the chunk's tokens
     // (the buffers hold a whole number of stages); what it reads there is not used.
@@ -218,43 +219,97 @@ __device__ __forceinline__ void da_scan_body(const lb_decay_params2& p) {
     }
     // the tile as pairs of rows (2r, 2r + 1), column by column
     da_f2 s[C][R / 2];
-    auto load = [&](const float* S) {
+    const bool quads = cols == C && (p.dv & 3) == 0 && (reinterpret_cast<uintptr_t>(p.state) & 15) == 0; // rows of whole 16-byte pieces
+    auto load = [&](const float* S) { // from the sequence's state
 #pragma unroll
         for (int r = 0; r < R; r += 2)
 #pragma unroll
-            for (int c = 0; c < C; ++c)
-                s[c][r / 2] = da_pack(c < cols && r < rows ? S[(size_t)r * p.dv + c] : 0.f, c < cols && r + 1 < rows ? S[(size_t)(r + 1) * p.dv + c] : 0.f);
+            for (int c = 0; c < C; c += 4) {
+                float x[2][4];
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const float* row = S + (size_t)(r + i) * p.dv + c;
+                    if (quads && r + i < rows) {
+                        const float4 v = *reinterpret_cast<const float4*>(row);
+                        x[i][0] = v.x; x[i][1] = v.y; x[i][2] = v.z; x[i][3] = v.w;
+                    } else {
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) x[i][u] = !quads && c + u < cols && r + i < rows ? row[u] : 0.f;
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u) s[c + u][r / 2] = da_pack(x[0][u], x[1][u]);
+            }
     };
-    auto store = [&](float* S) {
+    auto store = [&](float* S) { // to the sequence's state
 #pragma unroll
         for (int r = 0; r < R; r += 2)
 #pragma unroll
-            for (int c = 0; c < C; ++c) {
-                const float2 x = da_unpack(s[c][r / 2]);
-                if (c < cols && r < rows) S[(size_t)r * p.dv + c] = x.x;
-                if (c < cols && r + 1 < rows) S[(size_t)(r + 1) * p.dv + c] = x.y;
+            for (int c = 0; c < C; c += 4) {
+                float2 x[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) x[u] = da_unpack(s[c + u][r / 2]);
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    if (r + i >= rows) continue;
+                    float* row = S + (size_t)(r + i) * p.dv + c;
+                    if (quads) *reinterpret_cast<float4*>(row) = i ? make_float4(x[0].y, x[1].y, x[2].y, x[3].y) : make_float4(x[0].x, x[1].x, x[2].x, x[3].x);
+                    else {
+#pragma unroll
+                        for (int u = 0; u < 4; ++u)
+                            if (c + u < cols) row[u] = i ? x[u].y : x[u].x;
+                    }
+                }
+            }
+    };
+    // the workspace holds a tile in the order of the threads: 16 bytes of each beside those of the next
+    const size_t tile = (size_t)16 * R * DA_SLAB, tiles = (size_t)gridDim.x * gridDim.y;
+    float4* ws = reinterpret_cast<float4*>(p.seg_state + ((size_t)h * gridDim.y + blockIdx.y) * tile) + t;
+    auto ws_at = [&](int seg, int c, int r) { return ws + (size_t)seg * (tiles * tile / 4) + (c * (R / 4) + r / 2) * DA_SCAN_THREADS; };
+    auto put = [&](int seg) {
+#pragma unroll
+        for (int c = 0; c < C; ++c)
+#pragma unroll
+            for (int r = 0; r < R / 2; r += 2) {
+                const float2 x = da_unpack(s[c][r]), y = da_unpack(s[c][r + 1]);
+                *ws_at(seg, c, r) = make_float4(x.x, x.y, y.x, y.y);
+            }
+    };
+    auto get = [&](int seg) {
+#pragma unroll
+        for (int c = 0; c < C; ++c)
+#pragma unroll
+            for (int r = 0; r < R / 2; r += 2) {
+                const float4 x = *ws_at(seg, c, r);
+                s[c][r] = da_pack(x.x, x.y);
+                s[c][r + 1] = da_pack(x.z, x.w);
             }
     };
     auto advance = [&](int seg) { // the state through a whole segment: S <- diag(b) S + L
-        const float* L = p.seg_state + (size_t)seg * all + head_off;
-        const float* b = p.seg_decay + ((size_t)seg * p.H + h) * (16 * R) + e * R;
+        const float4* b = reinterpret_cast<const float4*>(p.seg_decay + ((size_t)seg * p.H + h) * (16 * R) + e * R);
 #pragma unroll
-        for (int r = 0; r < R; r += 2) {
-            const da_f2 bb = da_pack(b[r], b[r + 1]);
+        for (int r = 0; r < R / 2; r += 2) {
+            const float4 bb = b[r / 2];
 #pragma unroll
-            for (int c = 0; c < C; ++c)
-                s[c][r / 2] = da_fma2(bb, s[c][r / 2], da_pack(c < cols && r < rows ? L[(size_t)r * p.dv + c] : 0.f, c < cols && r + 1 < rows ? L[(size_t)(r + 1) * p.dv + c] : 0.f));
+            for (int c = 0; c < C; ++c) {
+                const float4 x = *ws_at(seg, c, r);
+                s[c][r] = da_fma2(da_pack(bb.x, bb.y), s[c][r], da_pack(x.x, x.y));
+                s[c][r + 1] = da_fma2(da_pack(bb.z, bb.w), s[c][r + 1], da_pack(x.z, x.w));
+            }
         }
     };
-    if (LOCAL ? g > 0 : false) {
+    if (LOCAL && g > 0) {
 #pragma unroll
         for (int c = 0; c < C; ++c)
 #pragma unroll
             for (int r = 0; r < R / 2; ++r) s[c][r] = 0ull;
-    } else if (LOCAL || g == 0) {
+    } else if (LOCAL || P == 1) {
         load(p.state + head_off);
+        if (LOCAL) put(P - 1);
+    } else if (g == 0) {
+        get(P - 1);
     } else {
-        load(p.seg_state + head_off);
+        get(0);
         for (int q = 1; q < g; ++q) advance(q);
     }
     da_f2 dec[R / 2]; // LOCAL: product of the segment's decays
@@ -330,7 +385,7 @@ __device__ __forceinline__ void da_scan_body(const lb_decay_params2& p) {
     }
     pdl_launch_dependents();
     if (LOCAL) {
-        store(p.seg_state + (size_t)g * all + head_off);
+        put(g);
         if (blockIdx.y == 0 && t < 16) {
             float* b = p.seg_decay + ((size_t)g * p.H + h) * (16 * R) + e * R;
 #pragma unroll
@@ -340,11 +395,7 @@ __device__ __forceinline__ void da_scan_body(const lb_decay_params2& p) {
                 b[2 * r + 1] = x.y;
             }
         }
-    } else if (P == 1) {
-        store(p.state + head_off);
-    } else if (g == 0) {
-        load(p.seg_state + head_off);
-        for (int q = 1; q < P; ++q) advance(q);
+    } else if (g == P - 1) {
         store(p.state + head_off);
     }
 }

@@ -445,7 +445,7 @@ typedef struct {
     float* a;
     float* o;             /* fp32 [T, H * dv] */
     void* cat;            /* prompt: bf16 / fp32 rows [T, cat_ld] */
-    float* seg_state;     /* prompt in segments: fp32 [segments, H, dk, dv] and ... */
+    float* seg_state;     /* prompt in segments: fp32 [segments, H, tiles of 64 columns in the order of the threads] and ... */
     float* seg_decay;     /* ... [segments, H, dk_p] */
     int32_t kind, ld, q_off, k_off, v_off, g_off; /* k_off: HGRN2 the gate's section; g_off < 0: no output gate */
     int32_t a1_off, rank; /* GLA: section of the low-rank pre-activation */
