@@ -193,6 +193,8 @@ int lb_driver_load(char* err, size_t errlen); /* LB_OK or LB_ERR_NO_DRIVER */
     X(ssm_scan_f32_64)                \
     X(ssm_scan_f32_128)               \
     X(ssm_scan_f32_256)               \
+    X(ssm_tc)                         \
+    X(ssm_tc_local)                   \
     X(ssm_finish)                     \
     X(l2_flush)
 

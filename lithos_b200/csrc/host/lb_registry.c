@@ -64,7 +64,7 @@ static int open_hybrid(lb_ctx* c, const lb_json* cfg, const char* dir, int max_c
 
 static const struct { const char* architecture; open_fn open; const char* images; } k_registry[] = {
     {"Nufalorn", open_nufalorn, "small prefill rows_gemv dense_gemm window_attention decay_attention"},
-    {"Vobunex", open_vobunex, "small prefill rows_gemv dense_gemm window_attention latent_attention ssm"},
+    {"Vobunex", open_vobunex, "small prefill rows_gemv dense_gemm window_attention latent_attention ssm ssm_tc"},
     {"Qwen3.5-hybrid", open_hybrid, "gemv chain batched batched_tc batched_ring deltanet attention attention_mma small comm prefill"},
 };
 

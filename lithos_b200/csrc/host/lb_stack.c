@@ -896,7 +896,21 @@ static int pf_ssm(lb_model* m, pf_set* w, int i, int pos0, int T) {
     static const int k_local[3] = {LBK_ssm_local_64, LBK_ssm_local_128, LBK_ssm_local_256};
     const unsigned slabs = (unsigned)(L->V_p / LB_SSM_COLS), heads = (unsigned)D->heads;
     if (S->esz == 4) LB_TRY(lb_launch(c, k_f32[state_size(D)], heads, slabs, 1, 128, 0, params, 1));
-    else {
+    else if (L->N_p == 128 && L->V_p == 64 && T > LB_SSM_SEG) { /* up to one block of the other kernel's, two CTAs a head on it are faster: Vobunex, 64 tokens 823 against 845 us */
+        /* segments as below; a CTA has an SM for itself */
+        const int blocks = (T + LB_SSM_TC_TOKENS - 1) / LB_SSM_TC_TOKENS, fit = c->sm_count / (int)heads;
+        int P = fit < blocks / 2 ? fit : blocks / 2;
+        if (P > ST_SSM_SEGS) P = ST_SSM_SEGS;
+        if (P < 1) P = 1;
+        p.seg = (blocks + P - 1) / P * LB_SSM_TC_TOKENS;
+        P = (T + p.seg - 1) / p.seg;
+        p.seg_state = (float*)w->st.seg_state; p.seg_decay = (float*)w->st.seg_decay; p.status = (uint32_t*)c->dev_status;
+        lb_ac_maps maps;
+        LB_TRY(lb_ac_fill(c, &maps, w->st.xbc, p.ld_xbc, 0, 0, 0, w->st.xbc, p.ld_xbc, 64, T));
+        void* tp[] = {&p, &maps};
+        if (P > 1) LB_TRY(lb_launch(c, LBK_ssm_tc_local, heads, 1, (unsigned)P - 1, 256, LB_SSM_TC_SMEM, tp, 1));
+        LB_TRY(lb_launch(c, LBK_ssm_tc, heads, 1, (unsigned)P, 256, LB_SSM_TC_SMEM, tp, 1));
+    } else {
         /* as many segments side by side as CTAs fit on the SMs, four blocks of tokens each at least */
         const int blocks = (T + LB_SSM_SEG - 1) / LB_SSM_SEG, fit = c->sm_count * (L->N_p <= 128 ? 3 : 1) / (int)(heads * slabs);
         int P = fit < blocks / 4 ? fit : blocks / 4;
@@ -1176,7 +1190,7 @@ static int stack_build(lb_model* m, const lb_stack_desc* d, lb_weight_source* sr
                 MAX(S->max_q, D->heads * kd); MAX(S->max_kx, D->heads * L->dim_p); MAX(S->max_vx, D->heads * L->vdim_p);
             }
         } else if (D->mixer == LB_MIX_SSM) {
-            MAX(S->max_state, state_bytes(D));
+            MAX(S->max_state, (size_t)D->heads * L->N_p * L->V_p * 4);
             MAX(S->max_heads, D->heads); MAX(S->max_dk, D->heads); MAX(S->max_xbc, D->heads * L->V_p + 2 * D->groups * L->N_p); MAX(S->max_o, D->heads * D->vdim);
         } else if (D->mixer == LB_MIX_ATTENTION) {
             MAX(S->max_q, D->heads * L->dim_p);

@@ -4,7 +4,7 @@
 // A column of a head's state needs only that column of x, so a CTA owns LB_SSM_COLS columns of one head.
 //   ssm_step_*     one token (decode): convolution, state read and written once, read-out
 //   ssm_conv       a prompt chunk's convolved channels and step sizes
-//   ssm_chunk_*    a prompt chunk on the tensor cores, block by block of LB_SSM_SEG tokens, the state on chip between blocks; where the heads
+//   ssm_chunk_*    a prompt chunk on the tensor cores (states of 128 rows with heads of 64 columns from 65 tokens on: ssm_tc.cu), block by block of LB_SSM_SEG tokens, the state on chip between blocks; where the heads
 //                  are few, in segments side by side: ssm_local_* carries each from a zero state, ssm_chunk_* starts each from its true state
 //   ssm_scan_f32_* the same token by token in fp32
 //   ssm_finish     gate, norm in parts, and the convolution's last inputs into the ring
