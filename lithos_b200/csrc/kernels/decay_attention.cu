@@ -17,20 +17,21 @@
 __device__ __forceinline__ float da_sigmoid(float z) { return 1.0f / (1.0f + expf(-z)); }
 __device__ __forceinline__ float da_log_sigmoid(float z) { return fminf(z, 0.f) - log1pf(expf(-fabsf(z))); }
 
-// q, k, a of channel ch (= head * dk + i); row: the token's projections, z2: GLA's second low-rank product
-__device__ __forceinline__ void da_channel(const lb_decay_params2& p, const float* row, int ch, float z2, float& q, float& k, float& a) {
-    const float zq = row[p.q_off + ch];
-    const float b = bf16_bits_to_f32(p.bias[ch]);
+// q, k, a of a channel: its projections zq, zk, bias b, lower bound lo, and z2, GLA's second low-rank product
+__device__ __forceinline__ void da_values(const lb_decay_params2& p, float zq, float zk, float b, float lo, float z2, float& q, float& k, float& a) {
     if (p.kind == LB_DA_HGRN2) {
-        const float z = row[p.k_off + ch] + b, lo = bf16_bits_to_f32(p.lower[ch]);
+        const float z = zk + b;
         q = zq * da_sigmoid(zq);
         a = fmaf(1.0f - lo, da_sigmoid(z), lo);
         k = (1.0f - lo) * da_sigmoid(-z); // 1 - a without cancellation
     } else {
         q = zq * p.q_scale;
-        k = row[p.k_off + ch];
+        k = zk;
         a = expf(da_log_sigmoid(z2 + b) * p.inv_tau);
     }
+}
+__device__ __forceinline__ void da_channel(const lb_decay_params2& p, const float* row, int ch, float z2, float& q, float& k, float& a) { // ch = head * dk + i; row: the token's projections
+    da_values(p, row[p.q_off + ch], row[p.k_off + ch], bf16_bits_to_f32(p.bias[ch]), p.kind == LB_DA_HGRN2 ? bf16_bits_to_f32(p.lower[ch]) : 0.f, z2, q, k, a);
 }
 __device__ __forceinline__ float da_dot_rank(const uint16_t* w, const float* x, int rank) {
     float s = 0.f;
@@ -94,8 +95,9 @@ extern "C" __global__ void __launch_bounds__(DA_THREADS) da_step_64(const __grid
 extern "C" __global__ void __launch_bounds__(DA_THREADS) da_step_128(const __grid_constant__ lb_decay_params2 p) { da_step_body<32>(p); }
 extern "C" __global__ void __launch_bounds__(DA_THREADS) da_step_256(const __grid_constant__ lb_decay_params2 p) { da_step_body<64>(p); }
 
-// q, k, a of a chunk, [T, H, dk_p] with zero padding.  grid (ceil(H dk_p / 256), ceil(T / 8)), block 256: a thread makes one channel of
-// eight tokens, so a row of W2 is read once per eight tokens.  dynamic shared memory: [8][rank] fp32
+// q, k, a of a chunk, [T, H, dk_p] with zero padding.  Bound by the trip to memory: a thread's 16 projections are on their way before the first is used (one token
+// after the other, with da_finish's rows in pieces of 4 bytes: Nufalorn prompts of 60 / 150 / 1000 tokens 748 / 870 / 2401 us; now 734 / 862 / 2381).
+// grid (ceil(H dk_p / 256), ceil(T / 8)), block 256: a thread makes one channel of eight tokens, so a row of W2 is read once per eight tokens.  dynamic shared memory: [8][rank] fp32
 extern "C" __global__ void __launch_bounds__(256) da_inputs(const __grid_constant__ lb_decay_params2 p) {
     extern __shared__ float a1_s[];
     pdl_wait();
@@ -110,6 +112,14 @@ extern "C" __global__ void __launch_bounds__(256) da_inputs(const __grid_constan
     if (c < p.H * p.dk_p) {
         const int h = c / p.dk_p, i = c - h * p.dk_p, ch = h * p.dk + i;
         const bool live = i < p.dk;
+        float zq[8], zk[8]; // all on their way before the first is used
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const float* row = p.proj + (size_t)min(t0 + u, p.T - 1) * p.ld;
+            zq[u] = live ? row[p.q_off + ch] : 0.f;
+            zk[u] = live ? row[p.k_off + ch] : 0.f;
+        }
+        const float b = live ? bf16_bits_to_f32(p.bias[ch]) : 0.f, lo = live && p.kind == LB_DA_HGRN2 ? bf16_bits_to_f32(p.lower[ch]) : 0.f;
         float z2[8] = {};
         if (live && p.kind == LB_DA_GLA)
             for (int r = 0; r < p.rank; ++r) {
@@ -121,7 +131,7 @@ extern "C" __global__ void __launch_bounds__(256) da_inputs(const __grid_constan
         for (int u = 0; u < 8; ++u) {
             if (u >= nt) break;
             float q = 0.f, k = 0.f, a = 0.f;
-            if (live) da_channel(p, p.proj + (size_t)(t0 + u) * p.ld, ch, z2[u], q, k, a);
+            if (live) da_values(p, zq[u], zk[u], b, lo, z2[u], q, k, a);
             const size_t o = (size_t)(t0 + u) * p.H * p.dk_p + c;
             p.q[o] = q;
             p.k[o] = k;
@@ -412,16 +422,47 @@ extern "C" __global__ void __launch_bounds__(128) da_finish(const __grid_constan
     const int s = blockIdx.x, h = blockIdx.y * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (h < p.H) {
         const float* o = p.o + ((size_t)s * p.H + h) * p.dv;
+        const float* gate = p.g_off >= 0 ? p.proj + (size_t)s * p.ld + p.g_off + (size_t)h * p.dv : nullptr;
+        const size_t d0 = (size_t)s * p.cat_ld + (size_t)h * p.dv;
+        if (((p.dv | p.cat_ld | (gate ? p.ld | p.g_off : 0)) & 3) == 0 && p.dv <= 256 &&
+            ((reinterpret_cast<uintptr_t>(p.o) | reinterpret_cast<uintptr_t>(p.proj) | reinterpret_cast<uintptr_t>(p.cat) | (reinterpret_cast<uintptr_t>(p.head_w) << 1)) & 15) == 0) {
+            float4 x[2], g[2]; // rows of whole 16-byte pieces stay in registers
+            float ss = 0.f;
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int i = 4 * (lane + 32 * u);
+                x[u] = i < p.dv ? *reinterpret_cast<const float4*>(o + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+                g[u] = gate && i < p.dv ? *reinterpret_cast<const float4*>(gate + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+#pragma unroll
+            for (int u = 0; u < 2; ++u) ss += (x[u].x * x[u].x + x[u].y * x[u].y) + (x[u].z * x[u].z + x[u].w * x[u].w);
+            const float r = 1.0f / sqrtf(warp_sum(ss) / (float)p.dv + p.eps);
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int i = 4 * (lane + 32 * u);
+                if (i >= p.dv) break;
+                const uint2 w = __ldg(reinterpret_cast<const uint2*>(p.head_w + i));
+                float4 v = make_float4(x[u].x * r * __uint_as_float(w.x << 16), x[u].y * r * __uint_as_float(w.x & 0xffff0000u), x[u].z * r * __uint_as_float(w.y << 16),
+                                       x[u].w * r * __uint_as_float(w.y & 0xffff0000u));
+                if (gate) {
+                    v.x *= g[u].x * da_sigmoid(g[u].x); v.y *= g[u].y * da_sigmoid(g[u].y); v.z *= g[u].z * da_sigmoid(g[u].z); v.w *= g[u].w * da_sigmoid(g[u].w);
+                }
+                if (p.cat_f32) *reinterpret_cast<float4*>(reinterpret_cast<float*>(p.cat) + d0 + i) = v;
+                else {
+                    const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+                    *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p.cat) + d0 + i) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+                }
+            }
+            pdl_launch_dependents();
+            return;
+        }
         float ss = 0.f;
         for (int i = lane; i < p.dv; i += 32) ss += o[i] * o[i];
         const float r = 1.0f / sqrtf(warp_sum(ss) / (float)p.dv + p.eps);
         for (int i = lane; i < p.dv; i += 32) {
             float v = o[i] * r * bf16_bits_to_f32(p.head_w[i]);
-            if (p.g_off >= 0) {
-                const float g = p.proj[(size_t)s * p.ld + p.g_off + (size_t)h * p.dv + i];
-                v *= g * da_sigmoid(g);
-            }
-            const size_t d = (size_t)s * p.cat_ld + (size_t)h * p.dv + i;
+            if (gate) v *= gate[i] * da_sigmoid(gate[i]);
+            const size_t d = d0 + i;
             if (p.cat_f32) reinterpret_cast<float*>(p.cat)[d] = v;
             else reinterpret_cast<__nv_bfloat16*>(p.cat)[d] = __float2bfloat16_rn(v);
         }
