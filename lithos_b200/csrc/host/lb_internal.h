@@ -237,7 +237,7 @@ struct lb_ctx {
     /* strip-packed copies made by lb_gemv_pack and still alive: lb_gemv_int4 runs the strip-packed kernel for these matrices */
     struct { uint64_t qweight, packed; int K, N, swiglu; } packed_reg[LB_PACKED_REG_MAX];
     int n_packed_reg;
-    int tc_clusters[9], mma_clusters[9]; /* [k]: clusters of k CTAs of the batched int4 kernels that run at once, tcgen05 / mma.sync (0: not asked yet) */
+    int tc_clusters[9], mma_clusters[9], gemv_clusters[9]; /* [k]: clusters of k CTAs that run at once of the batched int4 kernels, tcgen05 / mma.sync, and of the GEMV (0: not asked yet) */
     int product_pairs;      /* lb_set_product_pairs */
     uint64_t n_product_pairs;
     int chain_mailbox;      /* hand vectors from a GEMV to the next one through the mailbox (1, default) or a grid barrier (0) */

@@ -13,11 +13,12 @@
  *  - All CTAs of a launch should be co-resident and carry equal work, so that the HBM pipe and
  *    not a tail of late CTAs ends the kernel: ksplit is chosen so that tiles*ksplit comes close
  *    to (and not above) two CTAs per SM.
- *  - A CTA's shared memory (ring of 16 KB stages + its activation slice) is kept under a quarter
- *    of an SM where possible, so that the CTAs of the NEXT kernel fit beside it and prefetch
- *    their weights while this one computes (programmatic dependent launch). */
-typedef struct { int tiles, ksplit, gps, stages; unsigned smem; } gemv_geom;
+ *  - A CTA's shared memory (ring of 16 KB stages + its activation slice) is kept under half
+ *    of an SM where possible; the CTAs of the NEXT kernel follow those that are done and prefetch
+ *    their weights while the others compute (programmatic dependent launch). */
+typedef struct { int tiles, ksplit, gps, stages, early; unsigned smem; } gemv_geom;
 
+static int clusters_at_once(lb_ctx* c, int kernel, int k, unsigned threads, unsigned smem, int per_sm, int* slot);
 static int gemv_plan(lb_ctx* c, int K, int N, gemv_geom* g) {
     if (K <= 0 || N <= 0 || K % LB_GEMV_GROUP != 0 || N % 32 != 0)
         return lb_fail(c, LB_ERR_INVALID, "int4 GEMV needs K %% 128 == 0 and N %% 32 == 0 (K=%d, N=%d)", K, N);
@@ -28,6 +29,10 @@ static int gemv_plan(lb_ctx* c, int K, int N, gemv_geom* g) {
     if (ks < 1) ks = 1;
     if (ks > LB_GEMV_MAX_SPLITS) ks = LB_GEMV_MAX_SPLITS;
     if (ks > groups) ks = groups;
+    /* Two CTAs an SM with a deep ring where all clusters run at once like that (5120 x 10240 as 40 clusters of 7, one too many: 15.6 us), otherwise shared memory
+     * for four, which leaves the clusters room (that shape 11.0 us; with fewer slices 11.4) */
+    if (ks > 1 && !c->gemv_clusters[ks]) LB_CU(c, lb_drv.CtxSetCurrent(c->cu_ctx));
+    const int two = clusters_at_once(c, LBK_gemv_int4_w256, ks, GEMV_THREADS, (unsigned)(c->max_smem_optin / 2 - 2048), 2, &c->gemv_clusters[ks]) >= g->tiles;
     g->gps = (groups + ks - 1) / ks;
     g->ksplit = (groups + g->gps - 1) / g->gps;
     /* shared memory: 1 KB alignment slack, ring of 16 KB stages (one group each), the digit
@@ -40,15 +45,19 @@ static int gemv_plan(lb_ctx* c, int K, int N, gemv_geom* g) {
     size_t per_stage = LB_GEMV_STAGE_BYTES + 16; /* stage + its two mbarriers */
     size_t sm_total = (size_t)c->max_smem_optin + 1024; /* shared memory of one SM */
     int st = 0;
-    for (int per_sm = 4; per_sm >= 1 && st < 2; per_sm >>= 1) {
+    for (int per_sm = two ? 2 : 4; per_sm >= 1 && st < 2; per_sm >>= 1) {
         size_t budget = sm_total / per_sm - 1024;
         if (budget > (size_t)c->max_smem_optin) budget = (size_t)c->max_smem_optin;
         st = budget > fixed ? (int)((budget - fixed) / per_stage) : 0;
     }
     if (st < 1) return lb_fail(c, LB_ERR_INVALID, "int4 GEMV: K slice of %d groups does not fit shared memory", g->gps);
+    /* the whole slice where six stages hold it, four otherwise (us with 3 / 4 / 6: 5120 x 17408 15.5 / 12.7 / 13.5, 4096 x 11008 with slices of six 10.3 / 10.4 / 9.6; with
+     * shared memory for four CTAs an SM, as before, two stages: 15.2 and 10.4) */
     if (st > 6) st = 6;
+    if (two && g->gps > 6 && st > 4) st = 4;
     if (st > g->gps) st = g->gps;
     g->stages = st;
+    g->early = two;
     g->smem = (unsigned)((fixed + (size_t)st * per_stage + 127) & ~(size_t)127);
     return LB_OK;
 }
@@ -121,6 +130,7 @@ LB_API int lb_gemv_int4_fused(lb_ctx* c, uint64_t qweight, uint64_t scales, uint
     p.x_mode = x_mode; p.y_mode = y_mode;
     p.eps = eps;
     p.stages = g.stages;
+    p.early = g.early;
     LB_TRY(lb_gemv_tensor_maps(c, qweight, scales, qzeros, K, N, g.gps, p.tmap, p.tmap_sc, p.tmap_zr));
     void* params[] = {&p};
     return lb_launch_cluster(c, LBK_gemv_int4_w256, (unsigned)g.tiles, (unsigned)g.ksplit, 1, GEMV_THREADS, g.smem, params, 1,

@@ -27,10 +27,11 @@
 //     the real-number dot product than an fp32 FMA loop.
 //     (mma.sync rather than tcgen05: M is 1 here; tcgen05's 64/128-row tiles belong to the
 //     batched path.  The int4 mma shape is emulated on this part: 152 cycles measured.)
-//   * A CTA needs about 55 KB of shared memory, so the CTAs of TWO consecutive kernels
-//     fit on an SM: griddepcontrol.launch_dependents is issued at once and the next kernel
-//     streams its first stages while this one computes; its consumers wait in
-//     griddepcontrol.wait for the activations.
+//   * Two CTAs share an SM, with four stages of 16 KB each (six where they hold the whole slice).  When a CTA's last request is
+//     out (slices longer than the ring; otherwise after its loop) it lets the next kernel in, whose CTAs then take the place of
+//     the first that are done and stream their first stages beside the others; its consumers wait in griddepcontrol.wait for the
+//     activations.  us, two stages and shared memory for four CTAs an SM -> this: 5120 x 17408 15.2 -> 12.7, 5120 x 34816 23.6 ->
+//     21.4, 6144 x 5120 8.9 -> 8.1, 4096 x 11008 10.4 -> 8.9.  (Let in at kernel start its requests get between this one's.)
 //   * Split-K is ordered and stays on chip: the CTAs that split one column tile form a
 //     thread-block cluster and rank 0 adds their partial sums in rank order out of
 //     distributed shared memory, so results are bit-identical run to run; the reference's
@@ -115,6 +116,7 @@ extern "C" __global__ void __launch_bounds__(GEMV_CONSUMERS + 32, 4) gemv_int4_w
                 mbar_arrive_expect_tx(&full[s], GEMV_STAGE_BYTES); // out-of-range parts of the box are zero-filled
                 tma_load_stage(smem_base + (uint32_t)s * GEMV_STAGE_BYTES, p.tmap, n0 >> 5, (g0 + u) * LB_GEMV_ROWS, &full[s], pol);
             }
+            if (p.early && n_groups > S) pdl_launch_dependents(); // the last request is out: the next kernel may become resident
         }
         // consumers wait for every stage, so no copy is in flight past their loop; the warp
         // stays for the cluster barriers below
@@ -294,7 +296,7 @@ extern "C" __global__ void __launch_bounds__(GEMV_CONSUMERS + 32, 4) gemv_int4_w
                 }
             }
         }
-        pdl_launch_dependents(); // the next kernel may become resident while this one reduces
+        if (!p.early || n_groups <= S) pdl_launch_dependents(); // the next kernel may become resident while this one reduces
         // add the digit planes held by the four ft lanes (fixed order), scale back to x units
 #pragma unroll
         for (int i = 0; i < 8; ++i) {

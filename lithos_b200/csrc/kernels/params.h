@@ -55,6 +55,7 @@ typedef struct {
     int32_t stages;           /* TMA ring depth */
     int32_t x_mode, y_mode;
     float eps;
+    int32_t early;            /* the next kernel is let in when a CTA's last request is out */
 } lb_gemv_params;
 
 /* ---- chain of int4 GEMVs in ONE persistent launch (chain.cu) ------------------------------
