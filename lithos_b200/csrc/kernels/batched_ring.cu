@@ -1,10 +1,10 @@
-// Batched int4 projection of 9 to 32 tokens on sm_100a (HBM-bound: the packed words once): Y[b][n] = sum_k W(k,n) X[b][k], operands as in batched.cu.
+// Batched int4 projection of 2 to 16 tokens on sm_100a (HBM-bound: the packed words once): Y[b][n] = sum_k W(k,n) X[b][k], operands as in batched.cu.
 // No weight is rounded: A = the exact integers q - z, the fp16 group scale multiplies a K-group's fp32 sum.
 //
 // One CTA per SM = 128 columns x a K slice, eight warps.  What bounds the other kernels of these sizes is not the words' way
 // from HBM but what a K-group costs beside it: hand-overs between converting, issuing and reading warps (gemm_int4_tc_exact*, 0.5 us a K-group), or loads
 // through registers that cannot be kept far enough ahead (gemm_int4_mma_*).  Here
-//   * a ring of K-groups (17 of 12.6 KB at 16 tokens, 13 of 16.7 KB at 32) is filled by bulk copies: packed words by one tiled TMA
+//   * a ring of K-groups (21 of 10.6 KB up to 8 tokens, 17 of 12.6 KB up to 16) is filled by bulk copies: packed words by one tiled TMA
 //     (16 packed rows x 128 columns as four boxes of 32 columns, 128-byte swizzle), the tokens' activations by two, scales and zero-points as plain runs;
 //   * a warp takes a K-group WHOLE (warp w: groups w, w + 8, ...): all 128 columns and all tokens, from its slot straight into
 //     mma.sync.m16n8k16 operands, and asks for the K-group that follows in the slot when it has read it.  It meets nobody until the end: one wait per 8 KB
