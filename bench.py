@@ -1032,10 +1032,10 @@ def bench_batched(args, local):
         for B, flag in [(B, f) for B in batches for f in ((0, lb.GEMM_MMA_SYNC) if B == 1 else (0,) if B <= 8 or B > 64 else (0, lb.GEMM_TCGEN05, lb.GEMM_MMA_SYNC))]:
             if flag or B == 1:
                 path = "gemv_int4" if not flag else "gemm_int4_tc" if flag == lb.GEMM_TCGEN05 else "gemm_int4_mma"
-            elif B <= 8 or (B <= 32 and np.array_equal(bits(B, 0), bits(B, lb.GEMM_MMA_SYNC))):
+            elif B <= 32 and np.array_equal(bits(B, 0), bits(B, lb.GEMM_MMA_SYNC)):
                 path = "gemm_int4_mma"
-            else:  # up to 32 tokens the two ways differ in the last bits
-                path = "gemm_int4_tc_exact%d" % (16 if B <= 16 else 32) if B <= 32 else "gemm_int4_tc" if B <= 128 else "gemm_int4_tc_256"
+            else:  # up to 32 tokens the ways differ in the last bits
+                path = "gemm_int4_ring%d" % (8 if B <= 8 else 16) if B <= 16 else "gemm_int4_tc_exact32" if B <= 32 else "gemm_int4_tc" if B <= 160 else "gemm_int4_tc_256"
             ctx.begin_capture()
             for j in range(reps):
                 w = dev[j % sets]
@@ -1063,7 +1063,7 @@ def bench_batched(args, local):
     ctx.close()
     return {"metric": "batched int4 projection sweep (config 4)", "unit": "us per launch", "n_gpus": 1, "data": "synthetic",
             "higher_is_better": False, "dtype": "int4 weights, fp16 activations, fp32 accumulation", "peak": peak, "peak_source": which,
-            "kernels": "gemm_int4_tc, gemm_int4_tc_256, gemm_int4_tc_exact16/32 (tcgen05.mma 128 x NT x 16, accumulator and converted weights in TMEM), gemm_int4_mma_b8/b16/b32/b64 (mma.sync m16n8k16), gemv_int4", "l2": "weight sets of a shape rotate, together > L2", "sweep": sweep}
+            "kernels": "gemm_int4_tc, gemm_int4_tc_256, gemm_int4_tc_exact32 (tcgen05.mma 128 x NT x 16, accumulator and converted weights in TMEM), gemm_int4_ring8/16 (mma.sync from a ring of bulk copies), gemm_int4_mma_b8/b16/b32/b64 (mma.sync m16n8k16), gemv_int4", "l2": "weight sets of a shape rotate, together > L2", "sweep": sweep}
 
 
 def reference_decode(args, rank):

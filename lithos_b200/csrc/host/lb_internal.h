@@ -93,6 +93,8 @@ int lb_driver_load(char* err, size_t errlen); /* LB_OK or LB_ERR_NO_DRIVER */
     X(gemm_int4_mma_b64)              \
     X(gemm_int4_tc)                   \
     X(gemm_int4_tc_256)               \
+    X(gemm_int4_tc_epi)               \
+    X(gemm_int4_tc_256_epi)           \
     X(gemm_int4_tc_exact16)           \
     X(gemm_int4_tc_exact32)           \
     X(gemm_int4_ring8)                \

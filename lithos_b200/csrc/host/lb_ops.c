@@ -337,7 +337,7 @@ int lb_gemm_int4_epi(lb_ctx* c, uint64_t qweight, uint64_t scales, uint64_t qzer
         LB_TRY(map_tokens(c, &p, nt));
         const int ksplit = tc_slices(c, blocks, groups);
         const unsigned smem = halves ? (unsigned)(LB_TC_X_HALVES * nt * 128) : (unsigned)((exact ? 7 : LB_TC_STAGES(nt)) * nt * 256); /* activation stages; the partial tile [nt][132] fp32 fits over them */
-        return lb_launch_cluster(c, exact ? (nt > 16 ? LBK_gemm_int4_tc_exact32 : LBK_gemm_int4_tc_exact16) : halves ? LBK_gemm_int4_tc_256 : LBK_gemm_int4_tc, (unsigned)blocks, (unsigned)ksplit, 1,
+        return lb_launch_cluster(c, exact ? (nt > 16 ? LBK_gemm_int4_tc_exact32 : LBK_gemm_int4_tc_exact16) : halves ? (epi ? LBK_gemm_int4_tc_256_epi : LBK_gemm_int4_tc_256) : epi ? LBK_gemm_int4_tc_epi : LBK_gemm_int4_tc, (unsigned)blocks, (unsigned)ksplit, 1,
                                  exact ? (nt > 16 ? LB_TC_EXACT32_THREADS : LB_TC_EXACT16_THREADS) : LB_TC_THREADS, smem, params, 1, (unsigned)ksplit);
     }
     const int rows = B > 32 ? 64 : B > 16 ? 32 : B > 8 ? 16 : 8; /* token rows the CTA stages */

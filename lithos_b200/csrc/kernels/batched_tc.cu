@@ -89,8 +89,9 @@ struct tc_group { // a thread's share of one K-group: the 16 packed words (8 k e
 #define TC_FAIL_DONE 0x1102u           // status: the last products never completed
 #define TC_FAIL_FULL 0x1103u           // status: a stage was never filled
 
+template <bool EPI>
 __device__ __forceinline__ void tc_store_y(const lb_bgemm_params& p, size_t o, float v) {
-    if (p.epi == LB_BG_ADD) reinterpret_cast<float*>(p.y)[o] += v;
+    if (EPI && p.epi == LB_BG_ADD) reinterpret_cast<float*>(p.y)[o] += v;
     else if (p.y_f32) reinterpret_cast<float*>(p.y)[o] = v;
     else reinterpret_cast<__half*>(p.y)[o] = __float2half_rn(v);
 }
@@ -108,7 +109,9 @@ __device__ __forceinline__ void tc_store_glu(const lb_bgemm_params& p, int b, fl
 // SETS: converting sets of four warps (a set = the 128 columns); the exact kernels have fewer, their reading warps need the registers (spilling there cost
 // 20 %: 17408 -> 5120 at 32 tokens 38.2 us with three sets, 31.3 with two; at 16 tokens 31.0 with registers for 32 tokens, 27.1 with those for 16).
 // HALVES (161..256 tokens): a K-group of activations is 64 KB, so they have a ring of their own of 64-k halves, seven of which fit beside four weight stages.
-template <int EXACT, int SETS, bool HALVES> // EXACT: 0, or the tokens the product carries (16, 32)
+// EPI: p.epi counts.  Kernels of their own, since its branches beside each store cost every call without one 0.4 to 0.7 us (24 tokens, 4096 -> 4096 9.1 -> 9.6, 2048 -> 17408
+// at 28 12.1 -> 12.8).
+template <int EXACT, int SETS, bool HALVES, bool EPI> // EXACT: 0, or the tokens the product carries (16, 32)
 __device__ __forceinline__ void gemm_int4_tc_body(const lb_bgemm_params& p, unsigned char* tc_smem) {
     __shared__ __align__(8) uint64_t bar_free[TC_STAGES]; // a stage's products are done (tcgen05.commit)
     __shared__ __align__(8) uint64_t bar_full[TC_STAGES]; // a stage's weights are in place (one arrival per warp of the set) and its activations have landed (transaction bytes)
@@ -375,10 +378,10 @@ __device__ __forceinline__ void gemm_int4_tc_body(const lb_bgemm_params& p, unsi
 #pragma unroll
         for (int j = 0; j < EXACT; ++j) {
             if (KS > 1) pt[j * TC_PSTRIDE + 32 * (warp & 3) + lane] = sum[j];
-            else if (live && j < p.B) tc_store_y(p, (size_t)j * p.N + n, sum[j]);
+            else if (live && j < p.B) tc_store_y<EPI>(p, (size_t)j * p.N + n, sum[j]);
         }
     }
-    const bool glu = !EXACT && p.epi == LB_BG_SWIGLU, tiled = KS > 1 || glu; // through the tile in shared memory
+    const bool glu = EPI && p.epi == LB_BG_SWIGLU, tiled = KS > 1 || glu; // through the tile in shared memory
     if (!failed && !EXACT && warp < CV_WARPS) {
         for (int c = warp >> 2; c < NT / 16; c += SETS) { // the sets share the tokens
             uint32_t r[16];
@@ -389,7 +392,7 @@ __device__ __forceinline__ void gemm_int4_tc_body(const lb_bgemm_params& p, unsi
             for (int j = 0; j < 16; ++j) {
                 const int b = c * 16 + j;
                 if (tiled) pt[b * TC_PSTRIDE + 32 * (warp & 3) + lane] = __uint_as_float(r[j]);
-                else if (live && b < p.B) tc_store_y(p, (size_t)b * p.N + n, __uint_as_float(r[j]));
+                else if (live && b < p.B) tc_store_y<EPI>(p, (size_t)b * p.N + n, __uint_as_float(r[j]));
             }
         }
     }
@@ -418,14 +421,14 @@ __device__ __forceinline__ void gemm_int4_tc_body(const lb_bgemm_params& p, unsi
                 }
                 if (wide) {
                     float4* y = reinterpret_cast<float4*>(reinterpret_cast<float*>(p.y) + o);
-                    if (p.epi == LB_BG_ADD) {
+                    if (EPI && p.epi == LB_BG_ADD) {
                         const float4 a = *y;
                         v.x += a.x; v.y += a.y; v.z += a.z; v.w += a.w;
                     }
                     *y = v;
                 }
                 else {
-                    tc_store_y(p, o, v.x); tc_store_y(p, o + 1, v.y); tc_store_y(p, o + 2, v.z); tc_store_y(p, o + 3, v.w);
+                    tc_store_y<EPI>(p, o, v.x); tc_store_y<EPI>(p, o + 1, v.y); tc_store_y<EPI>(p, o + 2, v.z); tc_store_y<EPI>(p, o + 3, v.w);
                 }
             }
         }
@@ -440,17 +443,25 @@ __device__ __forceinline__ void gemm_int4_tc_body(const lb_bgemm_params& p, unsi
 
 extern "C" __global__ void __launch_bounds__(LB_TC_THREADS, 1) gemm_int4_tc(const __grid_constant__ lb_bgemm_params p) { // 9..160 tokens
     extern __shared__ __align__(1024) unsigned char tc_smem[];
-    gemm_int4_tc_body<0, 4, false>(p, tc_smem);
+    gemm_int4_tc_body<0, 4, false, false>(p, tc_smem);
 }
 extern "C" __global__ void __launch_bounds__(LB_TC_THREADS, 1) gemm_int4_tc_256(const __grid_constant__ lb_bgemm_params p) { // 161..256 tokens
     extern __shared__ __align__(1024) unsigned char tc_smem[];
-    gemm_int4_tc_body<0, 4, true>(p, tc_smem);
+    gemm_int4_tc_body<0, 4, true, false>(p, tc_smem);
+}
+extern "C" __global__ void __launch_bounds__(LB_TC_THREADS, 1) gemm_int4_tc_epi(const __grid_constant__ lb_bgemm_params p) { // 33..160 tokens
+    extern __shared__ __align__(1024) unsigned char tc_smem[];
+    gemm_int4_tc_body<0, 4, false, true>(p, tc_smem);
+}
+extern "C" __global__ void __launch_bounds__(LB_TC_THREADS, 1) gemm_int4_tc_256_epi(const __grid_constant__ lb_bgemm_params p) { // 161..256 tokens
+    extern __shared__ __align__(1024) unsigned char tc_smem[];
+    gemm_int4_tc_body<0, 4, true, true>(p, tc_smem);
 }
 extern "C" __global__ void __launch_bounds__(LB_TC_EXACT16_THREADS, 1) gemm_int4_tc_exact16(const __grid_constant__ lb_bgemm_params p) { // 1..16 tokens
     extern __shared__ __align__(1024) unsigned char tc_smem[];
-    gemm_int4_tc_body<16, 3, false>(p, tc_smem);
+    gemm_int4_tc_body<16, 3, false, false>(p, tc_smem);
 }
 extern "C" __global__ void __launch_bounds__(LB_TC_EXACT32_THREADS, 1) gemm_int4_tc_exact32(const __grid_constant__ lb_bgemm_params p) { // 17..32 tokens
     extern __shared__ __align__(1024) unsigned char tc_smem[];
-    gemm_int4_tc_body<32, 2, false>(p, tc_smem);
+    gemm_int4_tc_body<32, 2, false, false>(p, tc_smem);
 }
