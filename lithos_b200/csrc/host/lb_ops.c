@@ -415,8 +415,9 @@ LB_API int lb_deltanet_step(lb_ctx* c, uint64_t state, uint64_t q, uint64_t k, u
     const int few = n_steps == 1 || (n_steps == 2 && 2 * HV <= c->sm_count);
     /* More than eight steps: 16 columns per CTA instead of 32 where the fullest SM then has less than twice as many of them.  us, 32 / 16 columns: 48 heads (two
      * CTAs / three) 8 steps 4.8 / 5.1, 16 7.3 / 7.1, 64 21.5 / 19.5, 256 78.4 / 68.9; 16 heads (one / one) 16 steps 5.0 / 4.5, 256 52.1 / 42.1; 24 and 32 heads
-     * (one / two) 24 steps 6.6 / 7.2, 256 52.1 / 53.5 */
-    const int narrow = !few && n_steps > 8 && (8 * HV + c->sm_count - 1) / c->sm_count < 2 * ((4 * HV + c->sm_count - 1) / c->sm_count);
+     * (one / two) 24 steps 6.6 / 7.2, 256 52.1 / 53.5.  fp32 operands, whose pieces want twice the registers, always (24 and 32 heads, 32 / 16 columns:
+     * 15 steps 5.8 / 5.6, 24 7.3 / 7.2, 63 16.5 / 14.8, 256 60.3 / 51.7) */
+    const int narrow = !few && n_steps > 8 && (in_is_f32 || (8 * HV + c->sm_count - 1) / c->sm_count < 2 * ((4 * HV + c->sm_count - 1) / c->sm_count));
     const int kernel = few ? (n_steps == 1 ? (in_is_f32 ? LBK_deltanet_one_f32 : LBK_deltanet_one_bf16) : (in_is_f32 ? LBK_deltanet_two_f32 : LBK_deltanet_two_bf16))
                      : narrow ? (in_is_f32 ? LBK_deltanet_step16_f32 : LBK_deltanet_step16_bf16)
                               : (in_is_f32 ? LBK_deltanet_step_f32 : LBK_deltanet_step_bf16);
