@@ -27,7 +27,7 @@
 //     the real-number dot product than an fp32 FMA loop.
 //     (mma.sync rather than tcgen05: M is 1 here; tcgen05's 64/128-row tiles belong to the
 //     batched path.  The int4 mma shape is emulated on this part: 152 cycles measured.)
-//   * Two CTAs share an SM, with four stages of 16 KB each (six where they hold the whole slice).  When a CTA's last request is
+//   * Two CTAs share an SM, with four stages of 16 KB each (six where they hold the whole slice; gemv_plan has the shapes that keep two).  When a CTA's last request is
 //     out (slices longer than the ring; otherwise after its loop) it lets the next kernel in, whose CTAs then take the place of
 //     the first that are done and stream their first stages beside the others; its consumers wait in griddepcontrol.wait for the
 //     activations.  us, two stages and shared memory for four CTAs an SM -> this: 5120 x 17408 15.2 -> 12.7, 5120 x 34816 23.6 ->
