@@ -413,11 +413,14 @@ LB_API int lb_deltanet_step(lb_ctx* c, uint64_t state, uint64_t q, uint64_t k, u
     void* params[] = {&p, &n_steps};
     /* two steps: the kernel of few steps while its CTAs are at most two per SM (fp32, two steps / run: 48 heads 3.74 / 3.96 us, 96 heads 4.99 / 4.66) */
     const int few = n_steps == 1 || (n_steps == 2 && 2 * HV <= c->sm_count);
-    /* More than eight steps: 16 columns per CTA instead of 32 where the fullest SM then has less than twice as many of them.  us, 32 / 16 columns: 48 heads (two
+    /* More than twelve steps: 16 columns per CTA instead of 32 where the fullest SM then has less than twice as many of them and holds them
+     * at a time (four).  us, 32 / 16 columns, bf16: 48 heads (two
      * CTAs / three) 8 steps 4.8 / 5.1, 16 7.3 / 7.1, 64 21.5 / 19.5, 256 78.4 / 68.9; 16 heads (one / one) 16 steps 5.0 / 4.5, 256 52.1 / 42.1; 24 and 32 heads
-     * (one / two) 24 steps 6.6 / 7.2, 256 52.1 / 53.5.  fp32 operands, whose pieces want twice the registers, always (24 and 32 heads, 32 / 16 columns:
-     * 15 steps 5.8 / 5.6, 24 7.3 / 7.2, 63 16.5 / 14.8, 256 60.3 / 51.7) */
-    const int narrow = !few && n_steps > 8 && (in_is_f32 || (8 * HV + c->sm_count - 1) / c->sm_count < 2 * ((4 * HV + c->sm_count - 1) / c->sm_count));
+     * (one / two) 24 steps 6.6 / 7.2, 256 52.1 / 53.5.  fp32: 48 heads 9 steps 5.5 / 5.7, 12 6.2 / 6.3, 15 7.0 / 7.0, 24 9.4 / 9.1, 256 77.5 / 67.0; 16 heads 15 steps
+     * 5.3 / 4.7, 256 50.9 / 41.4; 24 heads 24 steps 6.5 / 7.2, 256 51.0 / 51.8; 64 (two / four) 9 steps 5.5 / 7.0, 256 77.3 / 84.8; 96 (three / six, of which four fit at
+     * a time) 9 steps 6.9 / 10.1, 256 108 / 127 */
+    const int ctas32 = (4 * HV + c->sm_count - 1) / c->sm_count, ctas16 = (8 * HV + c->sm_count - 1) / c->sm_count; /* on the fullest SM */
+    const int narrow = !few && n_steps > 12 && ctas16 < 2 * ctas32 && ctas16 <= 4;
     const int kernel = few ? (n_steps == 1 ? (in_is_f32 ? LBK_deltanet_one_f32 : LBK_deltanet_one_bf16) : (in_is_f32 ? LBK_deltanet_two_f32 : LBK_deltanet_two_bf16))
                      : narrow ? (in_is_f32 ? LBK_deltanet_step16_f32 : LBK_deltanet_step16_bf16)
                               : (in_is_f32 ? LBK_deltanet_step_f32 : LBK_deltanet_step_bf16);

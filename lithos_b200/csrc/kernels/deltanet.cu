@@ -376,13 +376,14 @@ __device__ __forceinline__ void deltanet_body(const lb_deltanet_params& p, int n
     dn_store_state(S, pairs, s);
 }
 
-// grid (HV, 4) / (HV, 8): 32 / 16 columns per CTA
-#define DN_RUNS(name, T, CL) \
-    extern "C" __global__ void __launch_bounds__(DN_THREADS) name(const __grid_constant__ lb_deltanet_params p, int n_steps) { deltanet_body<T, CL>(p, n_steps); }
-DN_RUNS(deltanet_step_bf16, __nv_bfloat16, 2)
-DN_RUNS(deltanet_step_f32, float, 2)
-DN_RUNS(deltanet_step16_bf16, __nv_bfloat16, 1)
-DN_RUNS(deltanet_step16_f32, float, 1)
+// grid (HV, 4) / (HV, 8): 32 / 16 columns per CTA.  At CL = 2 the registers of three CTAs an SM: left to itself the compiler stops at 128 for fp32 and spills (us,
+// 128 -> 168 registers: 24 heads 24 steps 7.3 -> 6.5, 256 60.3 -> 51.0; 96 heads 256 steps 108, the loop without straight runs 109)
+#define DN_RUNS(name, T, CL, ...) \
+    extern "C" __global__ void __launch_bounds__(__VA_ARGS__) name(const __grid_constant__ lb_deltanet_params p, int n_steps) { deltanet_body<T, CL>(p, n_steps); }
+DN_RUNS(deltanet_step_bf16, __nv_bfloat16, 2, DN_THREADS, 3)
+DN_RUNS(deltanet_step_f32, float, 2, DN_THREADS, 3)
+DN_RUNS(deltanet_step16_bf16, __nv_bfloat16, 1, DN_THREADS)
+DN_RUNS(deltanet_step16_f32, float, 1, DN_THREADS)
 extern "C" __global__ void __launch_bounds__(DN_THREADS) deltanet_one_bf16(const __grid_constant__ lb_deltanet_params p) { deltanet_few<__nv_bfloat16, 1>(p); }
 extern "C" __global__ void __launch_bounds__(DN_THREADS) deltanet_one_f32(const __grid_constant__ lb_deltanet_params p) { deltanet_few<float, 1>(p); }
 extern "C" __global__ void __launch_bounds__(DN_THREADS) deltanet_two_bf16(const __grid_constant__ lb_deltanet_params p) { deltanet_few<__nv_bfloat16, 2>(p); }

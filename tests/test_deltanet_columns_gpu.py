@@ -13,8 +13,8 @@ class View:
         self.ptr = b.ptr + off
 
 
-@pytest.mark.parametrize("HV,HK", [(16, 8), (24, 8), (32, 16), (48, 16)])
-@pytest.mark.parametrize("T", [9, 16, 21, 40])
+@pytest.mark.parametrize("HV,HK", [(16, 8), (24, 8), (32, 16), (48, 16), (64, 16), (96, 32)])
+@pytest.mark.parametrize("T", [9, 13, 16, 21, 40])
 @pytest.mark.parametrize("f32", [False, True])
 def test_runs(ctx, lb, oracle, HV, HK, T, f32):
     c = deltanet_case(3 + T, HV, HK, steps=T)
