@@ -210,7 +210,7 @@ __device__ __forceinline__ void attn_chunk_tc(const C& c, const lb_ac_maps& maps
         const int quad = warp & 3, R = R0 + 32 * quad + lane, Rc = min(R, n_rows - 1);
         const uint32_t lanes = (uint32_t)(32 * quad) << 16;
         const int lim = c.lim(Rc), low = c.low(Rc);
-        float m = z == 0 ? c.m0(Rc) : -1e30f, l = z == 0 ? c.l0() : 0.f;
+        float m = z == 0 ? c.m0(Rc) : -INFINITY, l = z == 0 ? c.l0() : 0.f;
         bool ok = true;
         for (int i = 0; i < n; ++i) {
             const int b = i % NB, key0 = first_key + i * AC_KEYS;
@@ -251,13 +251,14 @@ __device__ __forceinline__ void attn_chunk_tc(const C& c, const lb_ac_maps& maps
                     }
                 }
             }
+            const float mu = m == -INFINITY ? 0.f : m; // nothing seen so far: every score of the block is -infinity, every probability 0
             float ps[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
             for (int j = 0; j < 4; ++j) { // 32 keys: 16 pairs
                 uint32_t h[16], r[16];
 #pragma unroll
                 for (int e = 0; e < 16; ++e) {
-                    const float p0 = ac_exp2(__uint_as_float(s[2 * j + (e >> 3)][2 * (e & 7)]) - m), p1 = ac_exp2(__uint_as_float(s[2 * j + (e >> 3)][2 * (e & 7) + 1]) - m);
+                    const float p0 = ac_exp2(__uint_as_float(s[2 * j + (e >> 3)][2 * (e & 7)]) - mu), p1 = ac_exp2(__uint_as_float(s[2 * j + (e >> 3)][2 * (e & 7) + 1]) - mu);
                     ps[(2 * e) & 3] += p0;
                     ps[(2 * e + 1) & 3] += p1;
                     ac_split(p0, p1, h[e], r[e]);

@@ -314,7 +314,7 @@ struct pf_chunk_rows {
     __device__ __forceinline__ size_t q_at(int R) const { return ((size_t)(R / G) * p.HQ + kv * G + R % G) * AT_D; }
     __device__ __forceinline__ int lim(int R) const { return p.pos0 + R / G; }
     __device__ __forceinline__ int low(int) const { return 0; }
-    __device__ __forceinline__ float m0(int) const { return -1e30f; }
+    __device__ __forceinline__ float m0(int) const { return -INFINITY; }
     __device__ __forceinline__ float l0() const { return 0.f; }
     __device__ __forceinline__ void table(unsigned char*, int) const {}
     // out[s][hq][d..d+15] = fp16( O / l * sigmoid(gate) )
