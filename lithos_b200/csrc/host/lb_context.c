@@ -282,6 +282,7 @@ LB_API int lb_set_wait_limit(lb_ctx* c, uint64_t ns) {
     LB_CU(c, lb_drv.CtxSetCurrent(c->cu_ctx));
     LB_CU(c, lb_drv.MemsetD32Async(c->dev_status + 8, (unsigned)(ns & 0xffffffffu), 1, c->stream));
     LB_CU(c, lb_drv.MemsetD32Async(c->dev_status + 12, (unsigned)(ns >> 32), 1, c->stream));
+    c->wait_limit_ns = ns;
     return LB_OK;
 }
 

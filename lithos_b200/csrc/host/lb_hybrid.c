@@ -539,6 +539,7 @@ static int launch_attention(lb_model* m, const layer_t* L, CUdeviceptr proj_row,
     p.splits = lb_attn_mma_splits(c, splits_for, m->HKV);
     p.status = (uint32_t*)c->dev_status;
     p.max_ctx = cfg->max_ctx;
+    p.stay = lb_attn_stay(c);
     p.in_dtype = 1; p.gate_stride = 512; p.q_stride = 512;
     p.rot_dims = cfg->rot_dims; p.rope_theta = cfg->rope_theta; p.eps = cfg->eps;
     for (int i = 0; i < cfg->rot_dims / 2; i++)

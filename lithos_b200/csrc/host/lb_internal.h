@@ -242,6 +242,7 @@ struct lb_ctx {
     int tc_clusters[9], mma_clusters[9], gemv_clusters[9]; /* [k]: clusters of k CTAs that run at once of the batched int4 kernels, tcgen05 / mma.sync, and of the GEMV (0: not asked yet) */
     int product_pairs;      /* lb_set_product_pairs */
     uint64_t n_product_pairs;
+    uint64_t wait_limit_ns; /* lb_set_wait_limit (0: the built-in one) */
     int chain_mailbox;      /* hand vectors from a GEMV to the next one through the mailbox (1, default) or a grid barrier (0) */
     int capturing;     /* stream capture in progress */
     uint64_t capture_launches0;
@@ -275,6 +276,7 @@ int lb_gemm_int4_epi(lb_ctx* c, uint64_t qweight, uint64_t scales, uint64_t qzer
 int lb_ac_fill(lb_ctx* c, lb_ac_maps* m, CUdeviceptr k, int k_ld, CUdeviceptr tail, int tail_w, int tail_ld, CUdeviceptr v, int v_ld, int vdim, int rows);
 /* its launch: rows query rows per KV head, keys the last of them sees; the parts' scratch of `bytes` bytes; params {kernel's own, maps}; + 1 entry for the split */
 int lb_ac_launch(lb_ctx* c, int kernel, int merge, int rows, int kv_heads, int keys, int vdim, CUdeviceptr scratch, size_t bytes, void* p, lb_ac_maps* maps);
+int lb_attn_stay(const lb_ctx* c); /* lb_attn_params.stay */
 int lb_launch_pairs(lb_ctx* c, int kernel, unsigned pairs, unsigned bx, unsigned smem, void** params, int pdl);
 
 unsigned char* lb_map_file(const char* path, size_t* bytes); /* lb_safetensors.c: a whole file, read-only */

@@ -444,6 +444,9 @@ int lb_attn_mma_splits(lb_ctx* c, int pos, int HKV) {
     return s > cap ? (cap < 1 ? 1 : cap) : s < 1 ? 1 : s;
 }
 
+/* a context with a shorter limit for its waits: one look */
+int lb_attn_stay(const lb_ctx* c) { return c->wait_limit_ns && c->wait_limit_ns < 200 * LB_ATTN_STAY ? 0 : LB_ATTN_STAY; }
+
 unsigned lb_attn_mma_smem(int G) { /* as attn_mma_body lays it out */
     return (unsigned)(16 * 576 + 8 * G * 260 * 4 + 2 * 256 * 2 + 2 * 64 * 4 + 2 * 8 * 8 * 4);
 }
@@ -466,6 +469,7 @@ LB_API int lb_attention_decode(lb_ctx* c, uint64_t q, uint64_t k_new, uint64_t v
     p.scratch = (float*)c->attn_scratch; p.counters = (uint32_t*)(c->gemv_counters + 2048 * 4);
     p.pos = pos; p.HQ = HQ; p.HKV = HKV;
     p.splits = lb_attn_mma_splits(c, pos, HKV);
+    p.stay = lb_attn_stay(c);
     p.status = (uint32_t*)c->dev_status;
     p.in_dtype = in_is_f32 ? 1 : 0;
     p.gate_stride = 256; p.q_stride = 256;

@@ -13,7 +13,9 @@
 //   * O^T = V^T P^T: the probabilities come out of the first product in exactly the B-fragment layout (head g, rows 2t and 2t+1) and go in
 //     as two bf16 terms as well.
 //   * Online soft-max per head over the warp's blocks, warps merged through shared memory in warp order, slices by all CTAs of a KV
-//     head together, each its share of the outputs, in slice order: run-to-run identical.
+//     head together, each its share of the outputs, in slice order: run-to-run identical.  A launch has no more CTAs than the GPU has SMs, but
+//     nothing promises it all of them: a CTA that has waited for the others some 50 us leaves its share to those that come later, the last of which waits for nobody.
+//     (A cooperative launch, which does promise them, takes 4 us longer.)
 // mma.sync rather than tcgen05: M is the 1..6 query heads of a KV head.
 // HBM-bound at long contexts (K and V rows once), a chain of latencies at short ones.  24 / 4 heads, us a call, before -> after (before: rows staged in
 // shared memory by 512-byte bulk copies, one block per warp in flight, up to 64 slices per KV head = two waves beyond 4736 rows, and there a single CTA
@@ -37,6 +39,18 @@ __device__ __forceinline__ void split_bf16x2(float x, float y, uint32_t& hi, uin
     const __nv_bfloat162 l = __floats2bfloat162_rn(x - hf.x, y - hf.y);
     hi = *reinterpret_cast<const uint32_t*>(&h);
     lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+__device__ __forceinline__ uint32_t am_add(uint32_t* a, uint32_t v) {
+    uint32_t old;
+    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], %2;" : "=r"(old) : "l"(a), "r"(v) : "memory");
+    return old;
+}
+// the last CTA to be done with a KV head's records puts the words back to zero (the flags are)
+__device__ __forceinline__ void am_done(const lb_attn_params& p, uint32_t* word, uint32_t* finished) {
+    if (atomicAdd(finished, 1u) == (uint32_t)p.splits - 1u) {
+        *word = 0u;
+        *finished = 0u;
+    }
 }
 // 16 bytes of a cache row, read once: not kept in L1, first to leave L2
 __device__ __forceinline__ uint4 ld_row16(const unsigned char* a, uint64_t pol) {
@@ -147,15 +161,23 @@ __device__ __forceinline__ void am_norm_rope(float (&v)[8], const uint16_t* w, c
     for (int j = 0; j < 8; ++j) v[j] *= scale;
 }
 
-// One output of a KV head from the records of all its slices, GR slice groups (group `sub`: slices sub, sub + GR, ...) of 256 / GR threads; the groups'
-// results are combined in group order.  red: [3][GR][256 / GR] floats.
+// the gate of this thread's first output of a share
+template <int G>
+__device__ __forceinline__ float am_gate(const lb_attn_params& p, int kv, int share) {
+    if (!p.gate) return 0.f;
+    const int per = (G * AT_D + p.splits - 1) / p.splits, ol = p.splits > 16 ? threadIdx.x & 63 : threadIdx.x, o = share * per + ol;
+    return ol < per && o < G * AT_D ? ld_in(p.gate, (size_t)(kv * G + o / AT_D) * p.gate_stride + o % AT_D, p.in_dtype) : 0.f;
+}
+
+// A share of a KV head's outputs (as many shares as slices) from the records of all its slices, GR slice groups (group `sub`: slices sub, sub + GR, ...) of
+// 256 / GR threads; the groups' results are combined in group order.  gate0: am_gate.  red: [3][GR][256 / GR] floats.
 template <int G, int GR>
-__device__ __forceinline__ void am_finish(const lb_attn_params& p, int kv, int split, float gate0, float* red) {
+__device__ __forceinline__ void am_finish(const lb_attn_params& p, int kv, int share, float gate0, float* red) {
     constexpr int W = 256 / GR;
-    const int t = threadIdx.x, sub = t / W, ol = t % W, per = (G * AT_D + p.splits - 1) / p.splits; // this CTA's outputs: [split * per, (split + 1) * per)
+    const int t = threadIdx.x, sub = t / W, ol = t % W, per = (G * AT_D + p.splits - 1) / p.splits; // the share: outputs [share * per, (share + 1) * per)
     const float* kvrec = p.scratch + (size_t)kv * p.splits * G * AT_REC;
     for (int ob = 0; ob < per; ob += W) {
-        const int o = split * per + ob + ol;
+        const int o = share * per + ob + ol;
         const bool live = ob + ol < per && o < G * AT_D;
         const int g = live ? o / AT_D : 0, dim = live ? o % AT_D : 0;
         float M = -INFINITY, L = 0.f, A = 0.f;
@@ -207,6 +229,25 @@ __device__ __forceinline__ void am_finish(const lb_attn_params& p, int kv, int s
             if (p.gate) out *= sigmoidf_dev(ob == 0 ? gate0 : ld_in(p.gate, (size_t)hq * p.gate_stride + dim, p.in_dtype));
             p.out[(size_t)hq * AT_D + dim] = out;
         }
+    }
+}
+
+// the shares that other CTAs have left; apart, so that the ordinary way does not carry its registers
+template <int G>
+__device__ __noinline__ void am_take_over(const lb_attn_params& p, int kv, uint32_t* flags, float* red) {
+    __shared__ int s_next;
+    for (int share = 0;; ++share) {
+        __syncthreads(); // everybody is done with the share before
+        if (threadIdx.x == 0) {
+            while (share < p.splits && atomicExch(flags + share, 0u) == 0u) ++share;
+            s_next = share;
+        }
+        __syncthreads();
+        share = s_next;
+        if (share >= p.splits) return;
+        const float gate0 = am_gate<G>(p, kv, share);
+        if (p.splits > 16) am_finish<G, 4>(p, kv, share, gate0, red);
+        else am_finish<G, 1>(p, kv, share, gate0, red);
     }
 }
 
@@ -394,8 +435,10 @@ __device__ __forceinline__ void attn_mma_body(const lb_attn_params& p, unsigned 
         return;
     }
 
-    // ---- merge the position slices.  Every CTA of the launch is resident (the host starts no more than one per SM): the CTAs of a KV
-    // head wait for each other and each finishes its own share of the (head, feature) outputs ----
+    // ---- merge the position slices: every CTA of a KV head leaves its record, and each finishes its own share of the (head, feature) outputs when all
+    // of them are there.  The arrivals are the low half of a word; a CTA that does not want to wait any longer puts a flag on its share, adds to the high half and
+    // leaves, unless that addition finds everybody arrived.  So whoever finds everybody there, the last arrival at least, also sees whether shares were left, and
+    // does those whose flags it takes off: each share is done once. ----
     float* rec = p.scratch + ((size_t)(kv * p.splits + split) * G) * AT_REC;
 #pragma unroll
     for (int g = 0; g < G; ++g) __stcg(rec + g * AT_REC + t, Ag[g]);
@@ -404,35 +447,37 @@ __device__ __forceinline__ void attn_mma_body(const lb_attn_params& p, unsigned 
         __stcg(rec + t * AT_REC + 257, L);
     }
     const bool groups = p.splits > 16;
-    float gate0 = 0.f; // the gate of this thread's first output, on its way during the wait
-    if (p.gate) {
-        const int per = (G * AT_D + p.splits - 1) / p.splits, ol = groups ? t & 63 : t, o = split * per + ol;
-        if (ol < per && o < G * AT_D) gate0 = ld_in(p.gate, (size_t)(kv * G + o / AT_D) * p.gate_stride + o % AT_D, p.in_dtype);
-    }
+    const float gate0 = am_gate<G>(p, kv, split); // on its way during the wait
     __syncthreads(); // the whole record is written
+    uint32_t *word = p.counters + kv, *finished = p.counters + 8 + kv, *flags = p.counters + 16 + kv * p.splits;
+    bool left = false; // of thread 0: others have left their shares
+    int leave = 0;
     if (t == 0) {
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p.counters + kv) : "memory");
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(word) : "memory");
         const uint64_t w0 = globaltimer_ns();
+        const uint32_t mask = (uint32_t)p.stay; // the timer is read once per mask + 1 polls
+        uint32_t v;
         bool ok = false;
-        for (unsigned it = 0; it < LB_WAIT_SPINS; ++it) {
-            unsigned v;
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p.counters + kv) : "memory");
-            if (v >= (unsigned)p.splits) { ok = true; break; }
-            if ((it & 255u) == 255u && globaltimer_ns() - w0 > LB_WAIT_NS) break;
+        for (uint32_t it = 0; it < LB_WAIT_SPINS; ++it) {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(word) : "memory");
+            if ((v & 0xffffu) == (uint32_t)p.splits) { ok = true; break; }
+            if ((it & mask) == mask && globaltimer_ns() - w0 >= 200ull * mask) break;
         }
-        if (!ok && p.status) atomicExch(p.status, LB_DEV_TIMEOUT_COUNTER);
+        if (!ok) {
+            atomicExch(flags + split, 1u);
+            v = am_add(word, 0x10000u);
+            if ((v & 0xffffu) != (uint32_t)p.splits || atomicExch(flags + split, 0u) == 0u) leave = 1;
+        }
+        left = v >> 16;
     }
-    __syncthreads();
+    if (__syncthreads_or(leave)) {
+        if (t == 0) am_done(p, word, finished);
+        return;
+    }
     if (groups) am_finish<G, 4>(p, kv, split, gate0, part);
     else am_finish<G, 1>(p, kv, split, gate0, part);
-    __syncthreads();
-    if (t == 0) { // the last CTA to finish reading puts both counters back to zero
-        const unsigned old = atomicAdd(p.counters + 8 + kv, 1u);
-        if (old == (unsigned)p.splits - 1u) {
-            p.counters[kv] = 0u;
-            p.counters[8 + kv] = 0u;
-        }
-    }
+    if (__syncthreads_or(left)) am_take_over<G>(p, kv, flags, part);
+    if (t == 0) am_done(p, word, finished);
 }
 
 extern "C" __global__ void __launch_bounds__(AT_THREADS, 1) attn_decode_mma(const __grid_constant__ lb_attn_params p) {

@@ -268,7 +268,7 @@ typedef struct {
     uint16_t* v_cache;
     float* out;           /* fp32 [HQ,256] */
     float* scratch;       /* split partials: [HKV][splits][G][(256 acc) + m + l] */
-    uint32_t* counters;   /* zero between launches: one per kv head; attn_decode_mma: arrivals [kv], finished [8 + kv] */
+    uint32_t* counters;   /* zero between launches: one per kv head; attn_decode_mma: arrivals [kv], finished [8 + kv], shares left [16 + kv * splits + slice] */
     const int* pos_ptr;   /* when non-NULL the position is read from device memory (graph replay) */
     int32_t pos;          /* position of the new token; rows [0,pos] are attended */
     int32_t HQ, HKV;
@@ -283,7 +283,9 @@ typedef struct {
     uint32_t* status;     /* device status word for bounded waits (attn_decode_mma); may be NULL */
     int32_t max_ctx;      /* rows the caches hold (0 = not checked): a position outside [0, max_ctx) sets status
                              LB_DEV_POS_RANGE and the kernel returns without reading or writing a cache row */
+    int32_t stay;         /* attn_decode_mma: 200 ns units a CTA waits for the other slices before it leaves its share to them; 2^n - 1 (0: one look) */
 } lb_attn_params;
+#define LB_ATTN_STAY 255  /* 51 us: the slices of a launch that has the GPU for itself end well within that of each other */
 
 /* ---- dense bf16 rows x one fp32 vector with fused prologue and epilogue (rows_gemv) ------------------------
  * One or two row-major bf16 matrices [rows, K] against vectors built in shared memory.  Rows are taken two at a time (a

@@ -34,3 +34,25 @@ def test_slices(ctx, lb, oracle, HQ, HKV, pos):
     assert np.array_equal(v, vc) and np.array_equal(np.delete(k, pos, 0), np.delete(kc, pos, 0))  # the new row and nothing else
     for x in d.values():
         x.free()
+
+
+@pytest.mark.parametrize("HQ,HKV,pos", [(24, 4, 300), (24, 4, 4096), (8, 4, 2049), (48, 8, 5003), (6, 1, 9000), (4, 2, 9472)])
+def test_shares_left_to_the_last_arrival(ctx, lb, HQ, HKV, pos):
+    """No CTA waits for others that may not be resident: one that has waited for its limit leaves its share to the last to arrive, the result is the same and
+    nothing is reported.  With a limit of a nanosecond nearly every CTA leaves, with the built-in one hardly any does; calls alternate, since the words reset themselves."""
+    c = attention_case(HQ + pos, pos + 2, HQ, HKV)
+    d = {n: ctx.to_device(c[n]) for n in c}
+    got = []
+    for limit in (0, 1, 1, 0, 1):
+        ctx.set_wait_limit(limit)
+        for _ in range(4):
+            o = ctx.to_device(np.full(HQ * 256, np.nan, np.float32))
+            ctx.attention_decode(d["q"], d["k_new"], d["v_new"], d["gate"], d["q_norm_w"], d["k_norm_w"], d["kc"], d["vc"], o, pos, HQ, HKV)
+            got.append(o.download(np.float32, HQ * 256))
+            o.free()
+    ctx.set_wait_limit(0)
+    assert ctx.device_status() == 0 and np.isfinite(got[0]).all()
+    for g in got[1:]:
+        assert np.array_equal(g, got[0])
+    for x in d.values():
+        x.free()
