@@ -56,3 +56,31 @@ def test_shares_left_to_the_last_arrival(ctx, lb, HQ, HKV, pos):
         assert np.array_equal(g, got[0])
     for x in d.values():
         x.free()
+
+
+@pytest.mark.parametrize("HQ,HKV", [(4, 1), (6, 2)])
+@pytest.mark.parametrize("pos", [8193, 9473, 20000])
+@pytest.mark.parametrize("late", [False, True])
+def test_more_slices_than_one_trip(ctx, lb, oracle, HQ, HKV, pos, late):
+    """one or two KV heads have more than 64 slices, which are added in two trips or three: a head's largest score in the first slice or in the last one, about as
+    heavy as all other rows together, so that what was summed before, or what comes after, is brought to another maximum (features that do not rotate).  The bound
+    above, with a largest score of 16 in place of 8: 4e-4."""
+    c = attention_case(HQ + pos, pos + 3, HQ, HKV)
+    f = oracle.bf16_to_f32
+    q, kc = f(c["q"]).reshape(HQ, 256), c["kc"]
+    row = pos - 3 if late else 5
+    for kv in range(HKV):
+        k = np.zeros(256, np.float32)
+        h = q[kv * (HQ // HKV)]
+        k[64:] = h[64:] * (10.0 * 16.0 / np.sum(h[64:] ** 2))
+        kc[row, kv] = lb.f32_to_bf16(k)
+    kw, vw = kc.copy(), c["vc"].copy()
+    want = oracle.attention_step(f(c["q"]), f(c["k_new"]), f(c["v_new"]), f(c["gate"]), f(c["q_norm_w"]), f(c["k_norm_w"]), kw, vw, pos, HQ, HKV)
+    d = {n: ctx.to_device(c[n]) for n in c}
+    o = ctx.to_device(np.full(HQ * 256, np.nan, np.float32))
+    ctx.attention_decode(d["q"], d["k_new"], d["v_new"], d["gate"], d["q_norm_w"], d["k_norm_w"], d["kc"], d["vc"], o, pos, HQ, HKV)
+    got = o.download(np.float32, HQ * 256)
+    assert ctx.device_status() == 0
+    assert rel_err_max(got, want.ravel()) <= 4e-4
+    for x in (*d.values(), o):
+        x.free()
