@@ -35,9 +35,10 @@ static int gemv_plan(lb_ctx* c, int K, int N, gemv_geom* g) {
      * clusters in beside them.  us, four / two, with the CTAs of room: none 6016 x 8384 10.4 / 11.5, five 8320 x 13984 18.6 / 20.2, six 8576 x 11232 17.3 / 15.2, eight
      * 17408 x 8192 24.1 / 19.7, twelve 5120 x 17408 15.1 / 12.6; not enough for all 5120 x 10240 11.0 / 15.6.  Slices of up to four K-groups stay with four (3840 x 2048 5.8 /
      * 6.3, 4096 x 4096 6.4 / 6.7), those of 7 to 9 want room for twelve (eight 8192 x 8192 12.6 / 12.7, ten 5120 x 13824 12.7 / 12.8). */
-    if (ks > 1 && !c->gemv_clusters[ks]) LB_CU(c, lb_drv.CtxSetCurrent(c->cu_ctx));
-    const int at_once = clusters_at_once(c, LBK_gemv_int4_w256, ks, GEMV_THREADS, (unsigned)(c->max_smem_optin / 2 - 2048), 2, &c->gemv_clusters[ks]);
-    const int two = g->gps > 4 && (at_once - g->tiles) * ks >= (g->gps >= 7 && g->gps <= 9 ? 12 : 6);
+    const int k = g->ksplit; /* the cluster that is launched: less than ks where whole slices make fewer of them */
+    if (k > 1 && !c->gemv_clusters[k]) LB_CU(c, lb_drv.CtxSetCurrent(c->cu_ctx));
+    const int at_once = clusters_at_once(c, LBK_gemv_int4_w256, k, GEMV_THREADS, (unsigned)(c->max_smem_optin / 2 - 2048), 2, &c->gemv_clusters[k]);
+    const int two = g->gps > 4 && (at_once - g->tiles) * k >= (g->gps >= 7 && g->gps <= 9 ? 12 : 6);
     /* shared memory: 1 KB alignment slack, ring of 16 KB stages (one group each), the digit
      * table of the K slice (26 bytes per packed row), per-group sums, result buffer, mbarriers */
     int rows = g->gps * LB_GEMV_ROWS;
