@@ -23,9 +23,6 @@
 #define AC_ROWS LB_AC_ROWS
 #define AC_KEYS 128
 #define AC_UNIT LB_AC_UNIT
-#define AC_FAIL_EMPTY 0x1301u // status: a ring unit's products never completed
-#define AC_FAIL_FULL 0x1302u  // status: a ring unit never landed
-#define AC_FAIL_SCORES 0x1303u // status: scores, probabilities or read-outs never completed
 
 __device__ __forceinline__ void ac_tma(uint32_t dst_smem, const void* tmap, int x, int row, uint64_t* bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst_smem),

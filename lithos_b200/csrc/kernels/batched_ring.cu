@@ -17,7 +17,6 @@
 #include "common.cuh"
 #include "params.h"
 
-#define RG_FAIL_FULL 0x1401u  // status: a slot was never filled
 #define RG_WARPS 8
 #define RG_COLS 128
 #define RG_PS 132 // floats per token of a partial tile

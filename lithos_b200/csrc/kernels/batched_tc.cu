@@ -85,9 +85,6 @@ struct tc_group { // a thread's share of one K-group: the 16 packed words (8 k e
 };
 
 #define TC_SBO 1024                    // bytes between groups of 8 rows: 8 rows of 128 bytes (one 128-byte swizzle atom)
-#define TC_FAIL_FREE 0x1101u           // status: a stage's products never completed
-#define TC_FAIL_DONE 0x1102u           // status: the last products never completed
-#define TC_FAIL_FULL 0x1103u           // status: a stage was never filled
 
 template <bool EPI>
 __device__ __forceinline__ void tc_store_y(const lb_bgemm_params& p, size_t o, float v) {

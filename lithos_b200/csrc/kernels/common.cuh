@@ -13,6 +13,22 @@
 #define LB_DEV_TIMEOUT_PEER 0x1003u    // gave up waiting for a peer GPU's flag
 #define LB_DEV_TIMEOUT_COUNTER 0x1004u // gave up waiting on a split counter
 #define LB_DEV_POS_RANGE 0x1005u       // the decode position lies outside the KV cache: nothing was read or written
+// batched_tc.cu: a stage's products never completed; the last products never completed; a stage was never filled
+#define TC_FAIL_FREE 0x1101u
+#define TC_FAIL_DONE 0x1102u
+#define TC_FAIL_FULL 0x1103u
+// dense_gemm.cu: a stage's products never completed; a stage's operands never landed; an accumulator was never completed / never freed
+#define DG_FAIL_EMPTY 0x1201u
+#define DG_FAIL_FULL 0x1202u
+#define DG_FAIL_ACC 0x1203u
+// attention_tc.cuh: a ring unit's products never completed; a ring unit never landed; scores, probabilities or read-outs never completed
+#define AC_FAIL_EMPTY 0x1301u
+#define AC_FAIL_FULL 0x1302u
+#define AC_FAIL_SCORES 0x1303u
+// batched_ring.cu: a slot was never filled
+#define RG_FAIL_FULL 0x1401u
+// ssm_tc.cu: a copy or a product never completed
+#define ST_FAIL 0x1501u
 
 #define LB_WAIT_SPINS (1u << 22)
 #define LB_WAIT_NS 2000000000ull // 2 s wall-clock cap on any single wait

@@ -11,9 +11,6 @@
 #include "tcgen05.cuh"
 #include "params.h"
 
-#define DG_FAIL_EMPTY 0x1201u // status: a stage's products never completed
-#define DG_FAIL_FULL 0x1202u  // status: a stage's operands never landed
-#define DG_FAIL_ACC 0x1203u   // status: an accumulator was never completed / never freed
 
 __device__ __forceinline__ void dg_tma(uint32_t dst_smem, const void* tmap, int k, int row, uint64_t* bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst_smem),

@@ -20,7 +20,6 @@
 #include "params.h"
 
 #define ST_UNIT 16384 /* 128 rows of 64 bf16 columns, 128-byte swizzle */
-#define ST_FAIL 0x1401u // status: a copy or a product never completed
 // tensor memory: G | M's three terms | Y1 | Y2 | D
 #define ST_G 0u
 #define ST_M 128u
