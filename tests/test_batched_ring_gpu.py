@@ -1,5 +1,5 @@
 """GPU: int4 projections of 2 to 16 tokens on the ring kernels: fewer K-groups than warps, as many as slots and one more, K slices of unequal length, column
-blocks of 32, 96 and 128, with and without zero-points, both result types, a result beside a 16-byte boundary; a row's bits do not depend on how many
+blocks of 32, 96 and 128, more of them than SMs, with and without zero-points, both result types, a result beside a 16-byte boundary; a row's bits do not depend on how many
 travel with it (2 to 16), nor on the run.
 
 No weight is rounded: a K-group's 128 products (an fp16 activation and a small integer, exact) are summed in fp32, its scaled sum joins at most 16 others of its
@@ -21,7 +21,7 @@ class View:
         self.ptr = b.ptr + off
 
 
-@pytest.mark.parametrize("groups,N", [(g, n) for g in (1, 3, 8, 9, 16, 17, 18, 21, 22, 45) for n in (32, 1184)] + [(5, 96), (45, 96), (9, 9600)])
+@pytest.mark.parametrize("groups,N", [(g, n) for g in (1, 3, 8, 9, 16, 17, 18, 21, 22, 45) for n in (32, 1184)] + [(5, 96), (45, 96), (9, 9600), (2, 18976)])
 @pytest.mark.parametrize("zeros", [True, False])
 def test_ring(ctx, lb, groups, N, zeros):
     K = 128 * groups
