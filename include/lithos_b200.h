@@ -199,14 +199,18 @@ int lb_gemv_chain_supports(lb_ctx* ctx, int K, int N, int swiglu);
  * also wants qweight 8-byte and scales 4-byte aligned).
  * One token is handed to the GEMV kernel of lb_gemv_int4.
  * 2..32 tokens round no weight: q - z stays exact and the group scale multiplies the group's fp32 sum, so row b of Y
- * equals lb_gemv_int4 on row b of X to fp32 rounding.  2..16 tokens run on mma.sync from a ring of bulk copies (N % 32 == 0, weight
- * buffers 16-byte aligned; some sizes of 9..16 and all others: on the mma.sync kernels of LB_GEMM_MMA_SYNC), 17..32 on those or on the
- * 5th-generation tensor cores (tcgen05.mma, accumulators in tensor memory), whichever is faster for K, N and B.
+ * equals lb_gemv_int4 on row b of X to fp32 rounding.  2..16 tokens run on mma.sync from a ring of bulk copies where N % 32 == 0 and the
+ * weight buffers are 16-byte aligned.  Exempt are sizes of 9..16 tokens that have always had the bits of LB_GEMM_MMA_SYNC and keep its
+ * kernel for that: K <= 512; K <= 1024 with more column blocks of 128 than half the SMs; and, with fewer, columns of 6144 (13 tokens or more: 8192)
+ * and longer where twice as many slices run at once there (29..32 and 56..70 blocks on 148 SMs), of 14336 and longer also at 46..49 blocks.
+ * What the ring does not take, and 17..32 tokens, run on the mma.sync kernels of LB_GEMM_MMA_SYNC or on the 5th-generation tensor
+ * cores (tcgen05.mma, accumulators in tensor memory), 9..32 tokens on whichever is faster for K, N and B, weight buffers that the
+ * mma.sync kernels cannot read always on the latter.
  * 33..256 tokens run on tcgen05 with the weights dequantised to fp16 - (q - z) * s, q - z exact, one fp16 rounding for
  * the scale - and handed to the tensor cores through tensor memory (one product of 128 columns x all tokens per k
  * step, the weights converted once for all of them).
  * A row's bits do not depend on its place or on the rows that travel with it, but on the kernel, and so on how many rows
- * there are: they are the same within the sizes of 2..16 that run on the ring, within those of 2..32 that run on the mma.sync
+ * there are (at the exempt sizes they change between 8 and 9): they are the same within the sizes of 2..16 that run on the ring, within those of 2..32 that run on the mma.sync
  * kernels of LB_GEMM_MMA_SYNC, within those of 9..32 that run on tcgen05, and within 33..256.
  * LB_GEMM_MMA_SYNC forces the mma.sync kernels for every size up to 64 tokens (the same bits up to 32),
  * LB_GEMM_TCGEN05 the kernel that rounds the weights to fp16 for 9 tokens or more (the same bits from 9 to 256).

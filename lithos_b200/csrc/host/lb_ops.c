@@ -32,9 +32,10 @@ static int gemv_plan(lb_ctx* c, int K, int N, gemv_geom* g) {
     g->gps = (groups + ks - 1) / ks;
     g->ksplit = (groups + g->gps - 1) / g->gps;
     /* Two CTAs an SM with a deep ring where all clusters run at once like that and leave room for six CTAs, otherwise shared memory for four, which lets the next launch's
-     * clusters in beside them.  us, four / two, with the CTAs of room: none 6016 x 8384 10.4 / 11.5, five 8320 x 13984 18.6 / 20.2, six 8576 x 11232 17.3 / 15.2, eight
+     * clusters in beside them.   us, four / two, with the CTAs of room: none 6016 x 8384 10.4 / 11.5, five 8320 x 13984 18.6 / 20.2, six 8576 x 11232 17.3 / 15.2, eight
      * 17408 x 8192 24.1 / 19.7, twelve 5120 x 17408 15.1 / 12.6; not enough for all 5120 x 10240 11.0 / 15.6.  Slices of up to four K-groups stay with four (3840 x 2048 5.8 /
-     * 6.3, 4096 x 4096 6.4 / 6.7), those of 7 to 9 want room for twelve (eight 8192 x 8192 12.6 / 12.7, ten 5120 x 13824 12.7 / 12.8). */
+     * 6.3, 4096 x 4096 6.4 / 6.7), those of 7 to 9, whose ring of four stages is a small part of them, want room for twelve (less: 5760 x 13824 14.4 / 15.0, 5120 x 13824 12.6 / 12.8, 2048 x 36864 12.4 / 12.7, 8192 x
+     * 8192 12.7 / 12.8; the exception found 2304 x 37120 14.2 / 12.3). */
     const int k = g->ksplit; /* the cluster that is launched: less than ks where whole slices make fewer of them */
     if (k > 1 && !c->gemv_clusters[k]) LB_CU(c, lb_drv.CtxSetCurrent(c->cu_ctx));
     const int at_once = clusters_at_once(c, LBK_gemv_int4_w256, k, GEMV_THREADS, (unsigned)(c->max_smem_optin / 2 - 2048), 2, &c->gemv_clusters[k]);
@@ -260,7 +261,7 @@ static int mma_slices(const lb_ctx* c, int blocks, int groups) {
     return k;
 }
 
-/* 9..32 tokens without a flag: gemm_int4_tc_exact16 / 32 (1) or the mma.sync kernels (0); neither rounds a weight.  us, mma.sync / tcgen05:
+/* 17..32 tokens without a flag, and 9..16 where launch_ring does not apply: gemm_int4_tc_exact16 / 32 (1) or the mma.sync kernels (0); neither rounds a weight.  us, mma.sync / tcgen05:
  * matrices split along K: 17408 -> 5120 at 12 tokens 33.9 / 27.1, at 32 47.5 / 31.1; 1024 -> 1024 6.9 / 5.3, 11.4 / 6.3
  * short columns, where the start counts: K = 512 at 9 tokens 4.8 / 4.9, 640 5.5 / 5.3; K = 256 at 17 tokens 5.0 / 5.2, 384 5.7 / 5.5
  * whole columns up to 16 tokens (two CTAs per SM against one): 5120 -> 17408 at 12 tokens 23.9 / 24.5; up to 32 tokens 34.6 / 28.0, 5120 -> 34816 54.7 / 57
@@ -290,10 +291,13 @@ static int map_tokens(lb_ctx* c, lb_bgemm_params* p, int nt) {
     return LB_OK;
 }
 
-/* gemm_int4_ring8 / 16 run 2 to 16 tokens at every size (us, the kernels before / ring: 5120 -> 17408 at 2 tokens 19.0 / 12.2, 12 24.4 / 15.2; 17408 -> 5120 28.2 / 15.4,
- * 27.5 / 18.7; 1024 -> 1024 5.1 / 4.2, 5.7 / 4.8; 8192 -> 2048 9.6 / 6.7, 8.9 / 8.0), but for the sizes of 9 to 16 tokens whose rows keep the bits that
- * LB_GEMM_MMA_SYNC gives: columns of at most 512, whole columns of at most 1024, and the long columns of which mma.sync makes more slices (8192 -> 7168 at 12
- * tokens 19.6 / 14.1, 14336 -> 5888 31.8 / 21.1: slower, but the same rows as ever) */
+/* gemm_int4_ring8 / 16 run 2 to 16 tokens at every size, more column blocks than SMs too (us, the kernels before / ring: 5120 -> 17408 at 2 tokens 19.0 / 12.2, 12 24.4 /
+ * 15.2; 17408 -> 5120 28.2 / 15.4, 27.5 / 18.7; 1024 -> 1024 5.1 / 4.2, 5.7 / 4.8; 8192 -> 2048 9.6 / 6.7, 8.9 / 8.0; one block more than SMs, 5120 -> 19072, at 2 29.6 /
+ * 22.0, 16 40.1 / 28.2; 5120 -> 34816 32.4 / 24.3, 39.9 / 29.8; 2048 -> 24576 15.0 / 11.4, 22.8 / 14.1; 4096 -> 37888 26.4 / 21.7, 33.1 / 26.0), but for those of 9 to 16
+ * tokens that ran on the kernels of LB_GEMM_MMA_SYNC before there was a ring: their callers may compare rows with and without the flag, and keep the kernel for that
+ * alone.  It is the slower one (8192 -> 7168 at 12 tokens 19.6 / 14.1, 14336 -> 5888 31.8 / 21.1), and such a matrix's rows of 2 to 8 tokens, which are the ring's,
+ * differ from these in the last bits; the header says which sizes they are.  Whole columns of more than 1024, which the same rule would keep, are the decode batches
+ * that the ring is for (5120 -> 17408). */
 static int pinned_to_mma(lb_ctx* c, int B, int blocks, int groups) {
     return B > 8 && !exact_on_tc(c, B, blocks, groups) && (2 * blocks <= c->sm_count || groups <= 8);
 }
@@ -438,7 +442,8 @@ LB_API int lb_decay_gate(lb_ctx* c, uint64_t a, uint64_t a_log, uint64_t dt_bias
 }
 
 /* attn_decode_mma: slices of 128 rows (a block of 16 per warp), and no more of them than make one wave of one CTA per SM: the CTAs of a KV head wait for
- * each other.  24 / 4 heads at 100 000 rows: 69 us as 37 slices a head, 102 with the 64 (two waves) of the kernel before */
+ * each other.  24 / 4 heads at 100 000 rows: 69 us as 37 slices a head, 102 with the 64 (two waves) of the kernel before; 48 / 8 heads, 18 slices / 64: 2400 rows 13.6 / 25.2, 8192 20.9 / 54.5,
+ * 100 000 129 / 188; 8 / 8 heads 8192 rows 18.6 / 39.7 */
 int lb_attn_mma_splits(lb_ctx* c, int pos, int HKV) {
     const int cap = (c->sm_count < 512 ? c->sm_count : 512) / HKV; /* the scratch holds 512 records of 8 heads */
     const int s = (pos + 127) / 128;

@@ -24,8 +24,8 @@
 //     every CTA leaves its partial tile in shared memory and the ranks add them in rank order through
 //     distributed shared memory, each rank the token rows b = rank (mod cluster size): a fixed order, so
 //     the result does not depend on timing.
-// This is the legacy tensor path (mma.sync): it serves 2..8 tokens, and up to 32 where its two CTAs per SM beat the tcgen05 kernels
-// of batched_tc.cu (the rule and both sides' times stand at lb_gemm_int4).
+// This is the legacy tensor path (mma.sync): it serves what the ring kernels of batched_ring.cu leave of 2..16 tokens, and up to 32 where its two CTAs per SM beat
+// the tcgen05 kernels of batched_tc.cu (the rules and both sides' times stand at lb_gemm_int4).
 #include "common.cuh"
 #include "params.h"
 

@@ -454,7 +454,7 @@ extern "C" __global__ void __launch_bounds__(LB_TC_THREADS, 1) gemm_int4_tc_256_
     extern __shared__ __align__(1024) unsigned char tc_smem[];
     gemm_int4_tc_body<0, 4, true, true>(p, tc_smem);
 }
-extern "C" __global__ void __launch_bounds__(LB_TC_EXACT16_THREADS, 1) gemm_int4_tc_exact16(const __grid_constant__ lb_bgemm_params p) { // 1..16 tokens
+extern "C" __global__ void __launch_bounds__(LB_TC_EXACT16_THREADS, 1) gemm_int4_tc_exact16(const __grid_constant__ lb_bgemm_params p) { // up to 16 tokens where neither the ring nor mma.sync takes them
     extern __shared__ __align__(1024) unsigned char tc_smem[];
     gemm_int4_tc_body<16, 3, false, false>(p, tc_smem);
 }

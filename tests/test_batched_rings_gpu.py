@@ -59,9 +59,13 @@ def test_rings(ctx, lb, groups, N, zeros, f32):
     (512, 1024, 16, False), (640, 1024, 16, True), (256, 1024, 17, False), (384, 1024, 17, True),                # short columns
     (8192, 7168, 12, False), (8192, 8832, 16, False), (8192, 9216, 9, True), (5120, 7168, 12, True),             # twice the slices, and all of them at once
     (14336, 5888, 12, False), (11008, 5888, 12, True),                                                           # four times, and idle SMs
-    (1024, 9472, 16, True), (1024, 9600, 16, False), (1024, 9600, 17, True), (1024, 18944, 32, True), (1024, 18960, 32, False)])
+    (1024, 9472, 16, True), (1024, 9600, 16, False), (1024, 9600, 17, True), (1024, 18944, 32, True), (1024, 18960, 32, False),
+    # up to 16 tokens at widths that the ring kernels do not take, as many blocks of columns as above: what is not mma.sync here is tensor memory
+    (512, 1008, 16, False), (640, 1008, 16, True), (8192, 7152, 12, False), (8192, 8816, 16, False), (8192, 9200, 9, True), (5120, 7152, 12, True),
+    (14336, 5872, 12, False), (11008, 5872, 12, True), (1024, 9456, 16, True), (1024, 9584, 16, False)])
 def test_which_kernel(ctx, lb, K, N, B, tc):
-    """9 to 32 tokens run on tensor memory where that is the faster way (148 SMs); both ways are exact, so their results differ in the last bits only"""
+    """which sizes of 9 to 32 tokens have the bits of LB_GEMM_MMA_SYNC (148 SMs).  The others run on tensor memory, or, up to 16 tokens at widths in whole 32s, on the
+    ring kernels; all ways are exact, so their results differ in the last bits only"""
     if ctx.sm_count != 148:
         pytest.skip("the sizes are those of 148 SMs")
     qw, sc, qz, _ = gptq_case(K, N, seed=K + N)
