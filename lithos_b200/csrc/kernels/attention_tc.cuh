@@ -7,14 +7,14 @@
 // probabilities.  P overwrites the scores it came from; there are three such buffers (two at 256 value features, where the accumulator takes half of the
 // tensor memory), so the scores of block i + 1 are made while block i is with the soft-max warps.
 // The maximum a row's probabilities refer to follows its running maximum only when that is more than 8 (in log2 units) ahead, and then the accumulator is
-// rescaled in tensor memory; sums of up to 256 x as large terms cost no precision in fp32, and almost no block rescales.
+// rescaled in tensor memory (the conditional rescaling of FlashAttention-4); sums of up to 256 x as large terms cost no precision in fp32, and almost no block rescales.
 // Few query rows behind many keys leave SMs idle: the key blocks of a tile are then dealt to `parts` CTAs (grid.z), which leave unnormalised rows, maxima and sums
 // in scratch, and attn_chunk_merge adds them in order (lb_ac_launch chooses; us: hybrid 75 tokens behind 2000 1625 -> 1545, 5 tokens 1102 -> 1003, Vobunex 100
 // behind 2000 930 -> 907, Nufalorn 150 behind 2000 1009 -> 984).
 // Every wait is bounded and reports through the status word; TMEM is freed on every path.
-// Bound by the products: 128 x 128 x 16 from shared memory takes about 107 cycles, 128 x 256 x 16 with P in tensor memory 138, so 128 keys of the hybrid's heads
-// (256 features) cost 5600 cycles and of 128-feature heads 2900; the soft-max warps need less.  Before (mma.sync, 16 query rows per warp, keys and values
-// re-read from shared memory through ldmatrix for every 16 rows, the reason it stood at a tenth of the tensor cores' rate), whole prompts, us: int4 hybrid 75 tokens
+// Bound by the products where a CTA has many keys, and by its start and end where it has few: the tensor pipe is busy for 42 % of the active cycles of the SM with most
+// blocks at 1536 tokens of 128-feature heads, for 37 % where 256 tokens of the hybrid's heads (256 features) behind 1536 are dealt to three CTAs a
+// tile (ncu).  Before (mma.sync, 16 query rows per warp, keys and values re-read from shared memory through ldmatrix for every 16 rows, the reason it stood at a tenth of the tensor cores' rate), whole prompts, us: int4 hybrid 75 tokens
 // behind 2000 1837 -> 1648, Nufalorn 3000 7185 -> 6869 and 40 behind 1500 861 -> 746, Vobunex 4001 6120 -> 5194 and 100 behind 2000 1168 -> 929.
 #pragma once
 #include "tcgen05.cuh"

@@ -12,8 +12,8 @@
 // from those before it, and the last leaves the sequence's state.  The workspace holds a state in the order of the threads.
 // Tokens past the chunk are zero-filled by the copy engine, their step size is 0 and they are not stored.
 // Every wait is bounded and reports through the status word; TMEM is freed on every path.
-// Bound by the chain of a block: products of about 5500 cycles (128 x 128 x 16 from shared memory takes 107, 128 x 64 x 16 75, with M in tensor memory 42) with the
-// exponentials and splits between them.  The mma.sync kernels of ssm.cu (64 tokens x 32 columns, 262 products of 16 cycles a warp) were bound by that unit and made
+// Bound by the chain of a block: products, exponentials and splits, products again, with a barrier of the block between them; the tensor pipe is busy for 18 % of the
+// active cycles, the warps wait for barriers and shared memory most (ncu).  The mma.sync kernels of ssm.cu (64 tokens x 32 columns, 262 products of 16 cycles a warp) were bound by that unit and made
 // C B^T twice.  Vobunex prompts, us, before -> after: 4001 tokens 5126 -> 4790, 1500 behind 300 2236 -> 2064, 600 1398 -> 1284, 100 behind 2000 916 -> 904.
 #include "tcgen05.cuh"
 #include "mma_sync.cuh"
