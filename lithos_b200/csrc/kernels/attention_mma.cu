@@ -232,6 +232,13 @@ __device__ __forceinline__ void am_finish(const lb_attn_params& p, int kv, int s
     }
 }
 
+// puts a flag on the CTA's share and says so in the word: AM_LEFT, or the word where everybody had arrived and nobody else has taken the share
+#define AM_LEFT 0xffffu
+__device__ __noinline__ uint32_t am_leave(uint32_t* word, uint32_t* flag, uint32_t all) {
+    atomicExch(flag, 1u);
+    const uint32_t v = am_add(word, 0x10000u);
+    return (v & 0xffffu) != all || atomicExch(flag, 0u) == 0u ? AM_LEFT : v;
+}
 // the shares that other CTAs have left; apart, so that the ordinary way does not carry its registers
 template <int G>
 __device__ __noinline__ void am_take_over(const lb_attn_params& p, int kv, uint32_t* flags, float* red) {
@@ -463,19 +470,14 @@ __device__ __forceinline__ void attn_mma_body(const lb_attn_params& p, unsigned 
             if ((v & 0xffffu) == (uint32_t)p.splits) { ok = true; break; }
             if ((it & mask) == mask && globaltimer_ns() - w0 >= 200ull * mask) break;
         }
-        if (!ok) {
-            atomicExch(flags + split, 1u);
-            v = am_add(word, 0x10000u);
-            if ((v & 0xffffu) != (uint32_t)p.splits || atomicExch(flags + split, 0u) == 0u) leave = 1;
-        }
+        if (!ok) v = am_leave(word, flags + split, (uint32_t)p.splits);
+        leave = v == AM_LEFT;
         left = v >> 16;
     }
-    if (__syncthreads_or(leave)) {
-        if (t == 0) am_done(p, word, finished);
-        return;
+    if (!__syncthreads_or(leave)) {
+        if (groups) am_finish<G, 4>(p, kv, split, gate0, part);
+        else am_finish<G, 1>(p, kv, split, gate0, part);
     }
-    if (groups) am_finish<G, 4>(p, kv, split, gate0, part);
-    else am_finish<G, 1>(p, kv, split, gate0, part);
     if (__syncthreads_or(left)) am_take_over<G>(p, kv, flags, part);
     if (t == 0) am_done(p, word, finished);
 }
