@@ -19,8 +19,8 @@
 // mma.sync rather than tcgen05: M is the 1..6 query heads of a KV head.
 // HBM-bound at long contexts (K and V rows once), a chain of latencies at short ones.  24 / 4 heads, us a call, before -> after (before: rows staged in
 // shared memory by 512-byte bulk copies, one block per warp in flight, up to 64 slices per KV head = two waves beyond 4736 rows, and there a single CTA
-// merging all of them): 500 rows 16.2 -> 10.6, 4096 14.4 -> 10.4, 8000 30.9 -> 14.0, 20 000 42.2 -> 22.0, 100 000 101.7 -> 69.1 (5.9 TB/s);
-// 12 / 2 heads, 100 000 rows 51.7 -> 40.3.
+// merging all of them): 300 rows 18.4 -> 9.5, 4096 14.4 -> 10.6, 8192 31.0 -> 14.3, 20 000 42.2 -> 22.0, 100 000 101.7 -> 69.1 (5.9 TB/s);
+// 12 / 2 heads, 100 000 rows 51.7 -> 40.7; 48 / 8 heads, 8192 rows 54.5 -> 20.9.
 #include "attention_core.cuh"
 
 #define AM_ROWS 16
